@@ -217,7 +217,8 @@ struct g4s_net {
   bool team_batch = false;  // geometry planned for a multi-network batch
   int64_t team_slice = 0;   // ... with this many neurons per CTA
   bool team_ok = true;
-  bool pair_ready = false;  // the interleaved rows match the tables
+  bool pair_ready = false;  // the packed rows match the tables
+  bool pair_fits = false;   // every weight fits a packed word beside its target
   unsigned long long *list = nullptr;
   uint16_t *seg = nullptr;
   size_t seg_bytes = 0;
@@ -265,7 +266,7 @@ static void free_net(g4s_net *n) {
   n->step_graphs.clear();
   net_free(n, n->d_t0);
   cudaFreeHost(n->h_t0);
-  net_free(n, const_cast<int2 *>(v.pair));
+  net_free(n, const_cast<unsigned long long *>(v.pair));
   net_free(n, v.vu);
   net_free(n, v.abcd);
   net_free(n, v.rpar);
@@ -345,6 +346,7 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
   v.nexc = (d->n * (int64_t)d->exc_permille) / 1000;
   v.nsyn = d->nsyn;
   v.stride = (int32_t)row_stride(d->nsyn);
+  v.pair_bits = pair_target_bits(d->n);
   v.seed = d->seed;
   set_drive(n);
   const size_t N = (size_t)d->n, S = (size_t)v.stride;
@@ -627,13 +629,13 @@ static bool plan_team(g4s_net *n, int want, bool batch, int64_t slice, int *p_ou
   return true;
 }
 
-// The team kernel's buffers that do not depend on the team: the interleaved rows of its
-// segment reads (optional: without them, as when the device has no room left for them, the
-// kernel reads the separate arrays) and the tagged spike lists.  Both are ready on return
+// The team kernel's buffers that do not depend on the team: the packed rows of its reads
+// (optional: without them, as when the device has no room left for them or a weight is too
+// large to be packed beside its target, the kernel reads the separate arrays) and the tagged spike lists.  Both are ready on return
 // (a batch may launch on another handle's stream).
 static int prepare_rows(g4s_net *n) {
-  if (!n->v.pair) {
-    const size_t bytes = (size_t)n->v.n * (size_t)n->v.stride * sizeof(int2);
+  if (!n->v.pair && n->pair_fits) {
+    const size_t bytes = (size_t)n->v.n * (size_t)n->v.stride * sizeof(unsigned long long);
     if (!g_fail_next_alloc.exchange(0) && net_malloc(n, (void **)&n->v.pair, bytes) == cudaSuccess) {
       n->device_bytes += bytes;
       n->pair_ready = false;
@@ -648,12 +650,12 @@ static int prepare_rows(g4s_net *n) {
     n->pair_ready = true;
   }
   if (!n->list) {
-    cudaError_t e = net_malloc(n, (void **)&n->list, (size_t)n->v.n * 4 * sizeof(unsigned long long));
+    cudaError_t e = net_malloc(n, (void **)&n->list, (size_t)n->v.n * 2 * sizeof(unsigned long long));
     if (e != cudaSuccess) return cuda_error(e, "spike lists");
-    G4S_CUDA(cudaMemsetAsync(n->list, 0, (size_t)n->v.n * 4 * sizeof(unsigned long long), n->stream));
+    G4S_CUDA(cudaMemsetAsync(n->list, 0, (size_t)n->v.n * 2 * sizeof(unsigned long long), n->stream));
     G4S_CUDA(cudaStreamSynchronize(n->stream));
     n->tag_next = 0;
-    n->device_bytes += (size_t)n->v.n * 4 * sizeof(unsigned long long);
+    n->device_bytes += (size_t)n->v.n * 2 * sizeof(unsigned long long);
   }
   return G4S_OK;
 }
@@ -751,6 +753,13 @@ static int finish_tables(g4s_net *n, bool may_be_sorted) {
   unsigned long long h[3] = {~0ull, ~0ull, ~0ull};
   int rc = bound_pass(n, false, h);
   if (rc) return rc;
+  // Packed rows hold a weight in the bits that the target leaves, with its sign.
+  n->pair_fits = h[2] <= 1ull << (47 - n->v.pair_bits);
+  if (!n->pair_fits && n->v.pair) {  // (no launch that reads them is in flight)
+    net_free(n, n->v.pair);
+    n->v.pair = nullptr;
+    n->device_bytes -= (size_t)n->v.n * (size_t)n->v.stride * sizeof(unsigned long long);
+  }
   const unsigned long long limit = (1ull << 31) - (1ull << 20);
   if (h[0] < 65536ull && h[2] < limit && h[0] * h[2] < limit)
     h[1] = h[0] * h[2];  // (an upper bound of the sum)
@@ -920,11 +929,19 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
   });
   int rc = L.reserve(count, nslots);
   if (rc) return rc;
-  bool pair = true;  // every network of the round has its interleaved rows
+  bool pair = true;  // every network of the round has its packed rows
   for (int i : order) pair = pair && nets[i]->v.pair != nullptr;
   int nt = nets[order[0]]->team_nt_eff;  // threads per CTA: the networks' own when they agree
-  for (int i : order)
-    if (nets[i]->team_nt_eff != nt) nt = kTeamNT;
+  // delivery mapping of the launch's multi-CTA teams: the one that most of their work asks for
+  double group_work = 0.0, run_work = 0.0;
+  bool solo = false;  // one-CTA teams in the round
+  for (int i : order) {
+    const g4s_net *n = nets[i];
+    if (n->team_nt_eff != nt) nt = kTeamNT;
+    solo = solo || n->team_p == 1;
+    if (n->team_p > 1) (deliver_mode_of(n) == kDeliverGroup ? group_work : run_work) += (double)n->v.n * n->v.nsyn * steps[i];
+  }
+  const int mode = group_work > run_work ? kDeliverGroup : kDeliverRun;
   int gmax = 0;
   G4S_CUDA(team_max_blocks(smem, &gmax, nt));  // also raises the kernel's shared-memory ceiling
   if (gmax < maxteam) return set_error(G4S_ERR_CUDA, "team larger than the co-resident grid");
@@ -944,10 +961,8 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
     it.team = n->team_p;
     it.rc = (int)n->team_rc;
     it.sync = n->gs;
-    it.mode = deliver_mode_of(n);
-    it.cap = team_window(n->team_rc, n->team_p);
     if ((uint64_t)n->tag_next + (uint64_t)steps[i] + 2 >= 0xFFFFFFFFull) {  // tags would wrap: start over
-      G4S_CUDA(cudaMemsetAsync(n->list, 0, (size_t)n->v.n * 4 * sizeof(unsigned long long), s));
+      G4S_CUDA(cudaMemsetAsync(n->list, 0, (size_t)n->v.n * 2 * sizeof(unsigned long long), s));
       n->tag_next = 0;
     }
     it.tag0 = n->tag_next;
@@ -979,7 +994,7 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
     G4S_CUDA(cudaMemcpyAsync(L.d_off, L.h_off, sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
     G4S_CUDA(launch_round_clear(L.d_items, count, s));
     G4S_CUDA(cudaEventRecord(L.e0, s));
-    G4S_CUDA(launch_team(L.d_items, L.d_slots, L.d_ctl, L.d_ctl + 1, grid, smem, limit_ns, stall, s, pair, nt));
+    G4S_CUDA(launch_team(L.d_items, L.d_slots, L.d_ctl, L.d_ctl + 1, grid, smem, limit_ns, stall, s, pair, mode, solo, nt));
     G4S_CUDA(cudaEventRecord(L.e1, s));
     G4S_CUDA(launch_round_gather(L.d_items, L.d_off, count, L.d_pack, s));
     G4S_CUDA(cudaMemcpyAsync(L.h_pack, L.d_pack, total, cudaMemcpyDeviceToHost, s));
@@ -996,7 +1011,7 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
   // graph, so the key holds each network's creation number as well as its addresses.
   auto u = [](const void *p) { return (uint64_t)(uintptr_t)p; };
   std::vector<uint64_t> sig = {(uint64_t)count, (uint64_t)nslots, (uint64_t)grid, (uint64_t)smem, limit_ns,
-                               (uint64_t)stall, (uint64_t)pair, (uint64_t)nt, u(L.d_items), u(L.d_slots), u(L.d_ctl), u(L.h_items),
+                               (uint64_t)stall, (uint64_t)pair, (uint64_t)mode, (uint64_t)nt, u(L.d_items), u(L.d_slots), u(L.d_ctl), u(L.h_items),
                                u(L.h_slots), u(L.h_ctl), u(L.h_status), u(L.e0), u(L.e1)};
   for (int i : order) {
     const g4s_net *n = nets[i];
@@ -1022,7 +1037,7 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
     if (e == cudaSuccess) e = cudaMemcpyAsync(L.d_ctl, L.h_ctl, 8, cudaMemcpyHostToDevice, s);
     // (external records: the graph records the events at every replay)
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(L.e0, s, cudaEventRecordExternal);
-    if (e == cudaSuccess) e = launch_team(L.d_items, L.d_slots, L.d_ctl, L.d_ctl + 1, grid, smem, limit_ns, stall, s, pair, nt);
+    if (e == cudaSuccess) e = launch_team(L.d_items, L.d_slots, L.d_ctl, L.d_ctl + 1, grid, smem, limit_ns, stall, s, pair, mode, solo, nt);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(L.e1, s, cudaEventRecordExternal);
     for (int i : order) {
       const g4s_net *n = nets[i];

@@ -54,35 +54,37 @@ constexpr int64_t kBatchSlice = 8192;          // neurons per CTA of a batched n
                                                // 824 at 16384; served requests 41.9/s, 40.1, 32.7)
 constexpr int kStepGraphSteps = 512;          // longest chunk of the host-driven schemes (one CUDA graph)
 constexpr int kStepGraphs = 4;                 // captured chunks kept per network
-constexpr int kMaxTeam = 192;                  // CTAs of one team (three record slots per thread)
-constexpr int kMinWindow = 1024;               // spike ids a multi-CTA rank can stage per delivery window
-constexpr int kMaxWindow = 4096;
-constexpr int kFlatMax = 8192;                 // synapses of a step a rank delivers flat (else by runs)
-constexpr int64_t kFlatSlice = 4096;           // ... on slices up to this size
+constexpr int kMaxTeam = 176;                  // CTAs of one team (eight source ranks a warp, 22 such warps)
 // Spike records of a multi-CTA team: per rank and step parity kRecLines lines of 16
 // tagged 64-bit words (count, then up to 16 kRecLines - 1 ids); readers fetch the second
 // line of a rank only if it had enough spikes in the previous step (g4s_team.cu).
 constexpr int kRecLines = 2;
 constexpr int kRecWords = 16;
 
+// Ranks of a team from which every warp polls source ranks of its own; in smaller teams, where
+// that would leave most warps idle, every warp reads every rank's count and takes its share
+// of the step's spikes (from 6 ranks on instead: 64 networks in one launch, teams of up to 7
+// CTAs, 118 ms against 45).
+constexpr int kOwnSources = 12;
+
 // Shared-memory layout of one team rank (byte offsets; the optional arrays are present
-// when their flag is set).  `cap` is the delivery window of a multi-CTA team (0 for one CTA).
+// when their flag is set).
 struct TeamLayout {
-  unsigned abcd, vu, a, b, own, z, cnt, off, xoff, inl, pay, spk, sb, pre, ex, wsum, bytes;
-  bool abcd_sm, vu_sm, prez, flat;
+  unsigned abcd, vu, a, b, own, z, pay, bytes;
+  bool abcd_sm, vu_sm, prez, pay_sm;
 };
 __host__ __device__ inline unsigned team_align16(size_t x) { return (unsigned)((x + 15) & ~(size_t)15); }
-__host__ __device__ inline TeamLayout team_layout(int64_t rc, int team, int cap) {
+__host__ __device__ inline TeamLayout team_layout(int64_t rc, int team) {
   TeamLayout L{};
   L.abcd_sm = rc <= kAbcdSlice;
   L.vu_sm = rc <= kVuSlice;
   L.prez = rc <= kPrezSlice;
-  L.flat = team > 1 && rc <= kFlatSlice;
+  L.pay_sm = team >= kOwnSources;
   size_t o = 0;
   L.abcd = (unsigned)o;
   if (L.abcd_sm) o += (size_t)rc * 16;
   L.vu = (unsigned)o;
-  if (L.vu_sm) o += (size_t)rc * 8;
+  if (L.vu_sm) o = team_align16(o + (size_t)rc * 8);
   L.a = (unsigned)o;
   o = team_align16(o + (size_t)rc * 4);
   L.b = (unsigned)o;
@@ -91,44 +93,10 @@ __host__ __device__ inline TeamLayout team_layout(int64_t rc, int team, int cap)
   o = team_align16(o + (size_t)rc * 4);
   L.z = (unsigned)o;
   if (L.prez) o = team_align16(o + (size_t)rc * 4);
-  L.cnt = L.off = L.xoff = L.inl = L.pay = L.spk = L.sb = L.pre = L.ex = L.wsum = (unsigned)o;
-  if (team > 1) {
-    L.cnt = (unsigned)o;  // spikes per rank
-    o = team_align16(o + (size_t)(team + 1) * 4);
-    L.off = (unsigned)o;  // their offsets in the step's list
-    o = team_align16(o + (size_t)(team + 1) * 4);
-    L.xoff = (unsigned)o;  // offsets of the ids not in the lines read by the first pass
-    o = team_align16(o + (size_t)(team + 1) * 4);
-    L.inl = (unsigned)o;  // ids of each rank in the lines read by the first pass
-    o = team_align16(o + (size_t)(team + 1) * 4);
-    L.pay = (unsigned)o;  // payloads of the record lines
-    o = team_align16(o + (size_t)team * kRecLines * kRecWords * 4);
-    L.spk = (unsigned)o;  // the delivery window: spike ids of the step
-    o = team_align16(o + (size_t)cap * 4);
-    L.sb = L.pre = L.ex = L.wsum = (unsigned)o;
-  }
-  if (L.flat) {
-    L.sb = (unsigned)o;  // flat delivery: first slot of each spike's segment
-    o = team_align16(o + (size_t)cap * 2);
-    L.pre = (unsigned)o;  // ... offset of each spike's segment in the concatenation
-    o = team_align16(o + (size_t)(cap + 1) * 4);
-    L.ex = (unsigned)o;  // ... spike of every synapse of the concatenation
-    o = team_align16(o + (size_t)kFlatMax * 2);
-    L.wsum = (unsigned)o;  // ... per-warp sums of the scan
-    o = team_align16(o + 33 * 4);
-  }
+  L.pay = (unsigned)o;  // payloads of the record lines
+  if (L.pay_sm) o = team_align16(o + (size_t)team * kRecLines * kRecWords * 4);
   L.bytes = (unsigned)o;
   return L;
-}
-// Delivery window of a multi-CTA rank: what is left of the shared-memory limit, at most
-// kMaxWindow ids; 0 if less than kMinWindow is left (the geometry does not fit).
-inline int team_window(int64_t rc, int team) {
-  if (team <= 1) return 0;
-  const size_t kPerId = rc <= kFlatSlice ? 4 + 2 + 4 : 4;  // id (segment start, segment offset)
-  const size_t base = team_layout(rc, team, 0).bytes + 64;  // + alignment of the arrays
-  if (base + (size_t)kMinWindow * kPerId > kTeamSmemLimit) return 0;
-  const size_t cap = (kTeamSmemLimit - base) / kPerId;
-  return (int)(cap > (size_t)kMaxWindow ? kMaxWindow : cap & ~(size_t)7);
 }
 // Rows sorted by target (unsigned, so unused slots last), equal targets by weight bits;
 // generated = rows as the connectivity kernel writes them (distinct targets, unused slots
@@ -154,17 +122,25 @@ cudaError_t launch_inbound(const NetView &v, unsigned *cnt, unsigned long long *
 // (80 registers a thread instead of 64: no spills, faster when a step's work is small).
 constexpr int kTeamNT = 1024;
 constexpr int kTeamNTSmall = 768;
-// pair: the tables are read from v.pair (interleaved rows) instead of v.idx and v.w;
-// nt: kTeamNT or kTeamNTSmall threads per CTA
+// pair: the tables are read from v.pair (packed words) instead of v.idx and v.w;
+// mode: delivery mapping of the launch's multi-CTA teams (kDeliverRun or kDeliverGroup);
+// solo: the launch has one-CTA teams; nt: kTeamNT or kTeamNTSmall threads per CTA
 cudaError_t launch_team(const TeamItem *items, const int2 *slots, const int *nslots, int *slot_head, int grid,
-                        size_t smem, unsigned long long limit_ns, int stall, cudaStream_t s, bool pair,
-                        int nt = kTeamNT);
-// v.pair <- the rows of v.idx and v.w interleaved (after every change of the tables)
+                        size_t smem, unsigned long long limit_ns, int stall, cudaStream_t s, bool pair, int mode,
+                        bool solo, int nt = kTeamNT);
+// v.pair <- the rows of v.idx and v.w as packed words (after every change of the tables)
 cudaError_t launch_pairs(const NetView &v, cudaStream_t s);
+// Bits of a packed word's target field: what n needs, at least 16 (so that the decoding
+// shifts stay within a word).
+inline int pair_target_bits(int64_t n) {
+  int b = 16;
+  while (b < 31 && ((int64_t)1 << b) < n) ++b;
+  return b;
+}
 cudaError_t team_max_blocks(size_t smem, int *out, int nt = kTeamNT);
 // mean duration in ms of the last k simulated steps of a handle with a step time (0: none)
 double net_recent_step_ms(const g4s_net *n, int64_t k);
-// the team kernel's team-independent buffers of a handle (its interleaved rows and spike
+// the team kernel's team-independent buffers of a handle (its packed rows and spike
 // lists), made ready ahead of its first team run; nothing for tables the kernel cannot run
 int net_prepare_rows(g4s_net *n);
 // g4s_net_create with the handle's device memory from a stream-ordered pool (a server's)

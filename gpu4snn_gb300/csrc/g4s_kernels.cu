@@ -142,7 +142,7 @@ __device__ __forceinline__ bool update_one(const NetView &v, int64_t i, int64_t 
   const float g = i < v.nexc ? v.ge : v.gi;
   const float z = normal(v.seed, (uint64_t)i, (uint64_t)t_abs);
   float I;
-  const bool spk = izh_step(s.x, s.y, I, p, g, z, a);
+  const bool spk = izh_step(s.x, s.y, I, p, g, z, q32_current(a));
   v.vu[i] = s;
   if (a != 0) v.acc[i] = 0;
   if (last) v.ilast[i] = I;

@@ -157,7 +157,6 @@ extern "C" int g4s_run_noalloc(const g4s_dev_net *d, int64_t t_abs0, int32_t ste
   h.seg = seg;
   h.list = list;
   h.rec = reinterpret_cast<unsigned long long *>(scr + kOffRec);
-  h.cap = team_window(rc, team);
   h.tag0 = 0;
   h.t_abs0 = t_abs0;
   h.steps = steps;
@@ -168,7 +167,7 @@ extern "C" int g4s_run_noalloc(const g4s_dev_net *d, int64_t t_abs0, int32_t ste
   // Everything that must start at zero: error word, spike records and overflow ids (their
   // tags restart with every call), step counts; then the queue words and the descriptor.
   cudaError_t e = cudaMemsetAsync(scr, 0, kOffSlots, s);
-  if (e == cudaSuccess && team > 1) e = cudaMemsetAsync(list, 0, (size_t)d->n * 4 * sizeof(unsigned long long), s);
+  if (e == cudaSuccess && team > 1) e = cudaMemsetAsync(list, 0, (size_t)d->n * 2 * sizeof(unsigned long long), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_counts, 0, (size_t)steps * sizeof(int32_t), s);
   if (e == cudaSuccess) {
     k_noalloc_setup<<<1, 32, 0, s>>>(h, ctl, slots, item);
@@ -176,7 +175,7 @@ extern "C" int g4s_run_noalloc(const g4s_dev_net *d, int64_t t_abs0, int32_t ste
   }
   if (e == cudaSuccess && team > 1) e = launch_segoff(v, team, rc, seg, s);
   if (e == cudaSuccess)
-    e = launch_team(item, slots, ctl, ctl + 1, team, team_smem(rc, team), 2000000000ull, 0, s, false);
+    e = launch_team(item, slots, ctl, ctl + 1, team, team_smem(rc, team), 2000000000ull, 0, s, false, kDeliverRun, team == 1);
   if (e == cudaSuccess && d_status) e = cudaMemcpyAsync(d_status, &sync->error, sizeof(int32_t), cudaMemcpyDeviceToDevice, s);
   if (e != cudaSuccess) return cuda_error(e, "g4s_run_noalloc launch");
   return G4S_OK;

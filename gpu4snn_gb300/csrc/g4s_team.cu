@@ -28,41 +28,39 @@
 //             with a step number that never repeats for the network's buffers, so a
 //             reader that sees the tag it expects needs no fence to trust the payload:
 //             two 128-byte record lines (count and 31 ids), further ids in a per-rank
-//             overflow list.  Every rank reads, in one pass, line 0 of every rank and
-//             line 1 of the ranks that had more than kLine1After spikes in the previous
-//             step (16-byte slots, polled until their tags are current, with a time
-//             limit), so the records double as the team barrier; ids beyond the lines
-//             read are polled word by word.  The step's ids are staged in shared memory;
-//             a step with more ids than the window writes a dense tagged list in global
-//             memory instead, read directly by the delivery.  Records are cleared before
-//             each launch.  Two record sets (by step parity) suffice: a rank writes step
-//             t+2's words only after every rank has published step t+1, i.e. finished
-//             reading step t.
-//   delivery  one-CTA team: whole spiking rows, 128-bit loads, flat over all threads.
-//             Larger team: every rank reads, for every spike, the segment of the spiking
-//             row whose targets fall in its slice (rows are sorted by target and a per-row
-//             offset table gives the segment).  The run and group mappings read the rows
-//             interleaved as (target, weight bits) pairs, so a segment of ~7 synapses is one
-//             contiguous run of sectors instead of two half-used ones: at 7,000 spikes per
-//             step this cut the delivery by a third.  Flat mapping (at least kFlatMinSpikes
-//             staged spikes, at most kFlatMax synapses for the rank, and, in a 768-thread
-//             CTA, fewer than NT/2 spikes): the segment bounds
-//             of all spikes at once, a block scan, every synapse of the concatenation
-//             mapped to its spike in shared memory, and thread i walks synapses i, i+NT,
-//             ... with eight reads in flight.  Run mapping (otherwise): a warp takes 32
-//             spikes, scans their segment lengths and walks the concatenated segments,
-//             eight synapses per lane in flight, each lane finding its synapse's spike by
-//             a shuffle search.  Group mapping (the team's choice for long segments): the
-//             warp's 32 spikes in 8 rounds of 4, eight lanes walking each spike's segment,
-//             no search.  Each weight goes into the rank's own shared memory.
+//             overflow list.  In teams of kOwnSources CTAs and more every warp polls the
+//             records of a few source ranks of its own (line 0, and line 1 of the ranks that
+//             had more than kLine1After spikes in the previous step, with a time limit) and
+//             goes on to deliver those ranks' spikes at once: no warp waits for another
+//             one's sources, and the step has two block barriers (after the update, at its
+//             end).  In smaller teams every warp reads every rank's count and takes its share
+//             of the step's spikes.  Records are cleared before each launch.  Two record sets
+//             (by step parity) suffice: a rank writes step t+2's words only after every rank
+//             has published step t+1, i.e. finished reading step t.
+//   delivery  one-CTA team: whole spiking rows.  Larger team: every rank reads, for every
+//             spike, the segment of the spiking row whose targets fall in its slice (rows
+//             are sorted by target and a per-row offset table gives the segment).  The rows
+//             are read as packed words, the weight already in fixed point beside its target,
+//             so that a segment of ~7 synapses is one contiguous run of sectors and needs no
+//             float conversion.  Run mapping: a warp walks the concatenated segments of 32
+//             spikes.  Group mapping (the team's choice for long segments): eight lanes walk
+//             one spike's segment each.  Each weight goes into the rank's own shared memory.
 //   tail      the raster and the spike statistics of this rank's spikes, and the next
 //             step's drive, handed out in chunks of 32 neurons to warps as they finish
-//             delivering (the flat mapping computes each thread's own neuron's drive
-//             while its reads are in flight).
+//             delivering.
+//   What bounds a step: with few spikes the chain update -> publish -> poll -> bounds ->
+//   rows; with many, instruction issue and the shared-memory additions together (ncu: issue
+//   50-75%, LSU data pipe 58%; DRAM 18% at N=300,000).  us per step of this kernel and of
+//   the one before it (block-wide scan and staging of the step's ids, a search per synapse,
+//   a conversion per synapse; all mappings in one kernel): N=2,500 x 1000 3.85 / 4.55,
+//   33,333 x 777 at drive 1.5 5.40 / 7.10, 100,000 x 1000 7.32 / 8.77, 10^6 x 1000 40.6 /
+//   43.4 (drive 0.5 14.5 / 17.6, drive 2 106.7 / 112.4), 250,000 x 10,000 40.0 / 54.8; 64
+//   networks in one launch 45.4 / 60.7 ms.
 //   The raster records the spike ids of every step while its buffer has room.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstdint>
 
 #include "g4s_device.cuh"
@@ -277,11 +275,26 @@ __global__ void k_segoff(NetView v, int T, int64_t Rc, uint16_t *seg) {
   }
 }
 
-// Interleaved rows for the team kernel: pair[g] = (target, weight bits) of slot g.
-__global__ void k_pairs(NetView v, int2 *pair) {
-  const int64_t total = v.n * (int64_t)v.stride;
-  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x)
-    pair[g] = make_int2(v.idx[g], __float_as_int(v.w[g]));
+// Packed rows for the team kernel: pair[g] = Q32.32 weight of slot g << pair_bits | its
+// target; an unused slot is weight 0 into neuron 0, which adds nothing.  The conversion of
+// every weight to fixed point happens here, once per table change, instead of at every
+// delivery: F2I.S64 runs on the FP64 pipe, about 16 cycles a warp instruction per SM on this
+// part (N=250,000 x 10,000: 4,200 of them a step and SM, 33 of the step's 55 us).
+// Four slots a thread (rows are multiples of four slots): bound by memory, 16 bytes a slot.
+__global__ void k_pairs(NetView v, ulonglong2 *pair) {
+  const int64_t quads = v.n * (int64_t)(v.stride >> 2);
+  const int4 *idx = reinterpret_cast<const int4 *>(v.idx);
+  const float4 *w = reinterpret_cast<const float4 *>(v.w);
+  const int bits = v.pair_bits;
+  auto word = [&](int t, float x) {
+    return t < 0 ? 0ull : ((unsigned long long)wfix(x) << bits) | (unsigned long long)(unsigned)t;
+  };
+  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < quads; g += (int64_t)gridDim.x * blockDim.x) {
+    const int4 t = __ldcs(idx + g);
+    const float4 x = __ldcs(w + g);
+    pair[2 * g] = make_ulonglong2(word(t.x, x.x), word(t.y, x.y));
+    pair[2 * g + 1] = make_ulonglong2(word(t.z, x.z), word(t.w, x.w));
+  }
 }
 
 // Exactness bound of the split accumulation: per target, the number of incoming synapses
@@ -333,36 +346,102 @@ __device__ __forceinline__ void acc_add4(unsigned base_a, unsigned base_b, int l
   if (t.w >= 0) acc_add(base_a, base_b, (unsigned)(t.w - lo), wfix(w.w));
 }
 
-// Last index r in [0, n) with a[r] <= x, for a non-decreasing a[0..n] with a[0] <= x < a[n].
-__device__ __forceinline__ int find_run(const int *a, int n, int x) {
-  int lo = 0, hi = n;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (a[mid] <= x)
-      lo = mid;
-    else
-      hi = mid;
+// A synapse as the delivery loads it: a packed word (kPair), or target and weight bits.
+struct Syn {
+  unsigned x, y;
+};
+
+// The synapse `at` slots after a place of the tables, where `rem` > `at`; `row` is the
+// place: an address in the packed rows (kPair), or a slot of the separate arrays.
+template <bool kPair>
+__device__ __forceinline__ Syn load_syn(const NetView &v, long long row, int rem, int at) {
+  Syn s;
+  if constexpr (kPair) {
+    asm("{.reg .pred p;\n\tsetp.gt.s32 p, %3, %4;\n\t@p ld.global.nc.v2.u32 {%0, %1}, [%2];}"
+        : "=r"(s.x), "=r"(s.y)
+        : "l"(row + at * 8), "r"(rem), "r"(at));
+  } else {
+    asm("{.reg .pred p;\n\tsetp.gt.s32 p, %4, %5;\n\t@p ld.global.nc.u32 %0, [%2];\n\t@p ld.global.nc.u32 %1, [%3];}"
+        : "=r"(s.x), "=r"(s.y)
+        : "l"(v.idx + row + at), "l"(v.w + row + at), "r"(rem), "r"(at));
   }
-  return lo;
+  return s;
 }
+template <bool kPair>
+__device__ __forceinline__ long long syn_row(const NetView &v, long long slot) {
+  return kPair ? (long long)reinterpret_cast<uintptr_t>(v.pair + slot) : slot;
+}
+template <bool kPair>
+__device__ __forceinline__ long long syn_after(long long row, int slots) {
+  return row + (kPair ? slots * 8 : slots);
+}
+
+// Adds a synapse to the split accumulators, where `rem` > `at` (red.shared of random words:
+// 3.9 cycles a warp instruction per SM, 1.2 without bank conflicts); base_a and base_b are the
+// shared addresses that neuron 0's words would have.  The packed word's high part shifted
+// right is q >> 16.
+template <bool kPair, bool kSink>
+__device__ __forceinline__ void acc_syn(unsigned base_a, unsigned base_b, int bits, unsigned tmask, const Syn s,
+                                        int rem, int at) {
+  int a;
+  unsigned b, t;
+  if constexpr (kPair) {
+    t = s.x & tmask;
+    a = (int)s.y >> (bits - 16);
+    b = __funnelshift_r(s.x, s.y, bits) & 0xFFFFu;
+  } else {
+    const long long q = wfix(__uint_as_float(s.y));
+    t = s.x;
+    a = (int)(q >> 16);
+    b = (unsigned)(q & 0xFFFF);
+  }
+  const bool on = rem > at;
+  if constexpr (kSink) {
+    // lanes past the end add to a word of their own that is never read (whole rows: few such
+    // lanes, and no divergence region per synapse, 70.4 against 79.0 us a step for a lone CTA)
+    __shared__ int s_sink[32];
+    const unsigned sink = (unsigned)__cvta_generic_to_shared(&s_sink[threadIdx.x & 31]);
+    asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(on ? base_a + t * 4u : sink), "r"(a));
+    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(on ? base_b + t * 4u : sink), "r"(b));
+  } else if (on) {
+    asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(base_a + t * 4u), "r"(a));
+    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(base_b + t * 4u), "r"(b));
+  }
+}
+
+// Scratch of one warp: the delivery's segment runs, then the drive's repeated draws.
+struct WarpScratch {
+  union {
+    struct {
+      long long row[32];  // place of every segment of a batch, less its position in the run
+      unsigned head[8];   // segment heads of 256 synapses
+    };
+    int retry[64];  // neurons whose first draw was rejected
+  };
+};
+
+__device__ __forceinline__ unsigned lanemask_le() { return 0xFFFFFFFFu >> (31u - (threadIdx.x & 31u)); }
 
 // Scalars of one CTA shared by the phases of a step; the per-step counters come in pairs
 // (by step parity) so that one is cleared while the other is in use.
 struct TeamShared {
-  int nown[2];  // spikes of this rank in the step
-  int work[2];  // next chunk of the next step's drive
-  int fail;     // the exchange gave up (time limit, or the team's error word was set)
-  int slot;     // queue slot taken by this CTA
+  int nown[2];    // spikes of this rank in the step
+  int work[2];    // next chunk of the next step's drive
+  int k[2];       // spikes of the team in the step ...
+  int off[2];     // ... of the ranks before this one
+  int polled[2];  // warps that have added their source ranks to k and off
+  long long base; // raster offset of the step
+  int fail;       // the exchange gave up (time limit, or the team's error word was set)
+  int slot;       // queue slot taken by this CTA
+  int rank;       // rank and layout of the network's slice, read where they are needed (kept
+  TeamLayout L;   // in registers they would spill the delivery's reads in flight)
+  unsigned long long lim;  // time limit of the step's waits
 };
 
-// Record words of a rank per step: word 0 = spike count, words 1.. = ids (kInline inline);
-// a thread of an NT-thread CTA reads up to slots_per_thread(NT) 16-byte slots of a step's
-// records.
+// Record words of a rank per step: word 0 = spike count, words 1.. = ids (kInline inline).
 constexpr int kRankWords = kRecLines * kRecWords;
 constexpr int kInline = kRankWords - 1;
-__host__ __device__ constexpr int slots_per_thread(int nt) { return (kMaxTeam * kRankWords / 2 + nt - 1) / nt; }
-constexpr int kLine1After = 7;
-constexpr int kFlatMinSpikes = 128;  // fewer spikes: run delivery (the flat one's scan costs more)  // line 1 of a rank is read if it had more spikes in the previous step
+constexpr int kLine1After = 7;  // line 1 of a rank is polled if it had more spikes in the previous step
 
 // Gives up a wait: first error wins, every CTA of the team leaves at its next check.
 __device__ __forceinline__ void give_up(TeamShared &sh, GridSync *gs) {
@@ -386,127 +465,455 @@ __device__ __forceinline__ int tagged_id(const unsigned long long *p, unsigned t
   }
 }
 
+// One round of a poll's checks by a warp whose words are not all there yet (t0: the poll's
+// start, set in round 0): true when the wait is given up.
+__device__ __forceinline__ bool poll_check(TeamShared &sh, GridSync *gs, int iter, unsigned long long &t0,
+                                           unsigned long long lim) {
+  int f = 0;
+  if ((threadIdx.x & 31) == 0) {
+    const unsigned long long now = globaltimer();
+    if (iter == 0) t0 = now;
+    f = *(volatile int *)&sh.fail;
+    if (!f && threadIdx.x == 0 && ld_relaxed(&gs->error) != 0) f = 1;
+    if (!f && now - t0 > lim) {
+      give_up(sh, gs);
+      f = 1;
+    }
+    if (f) *(volatile int *)&sh.fail = 1;
+  }
+  return __shfl_sync(0xFFFFFFFFu, f, 0) != 0;
+}
+
+// Warps that poll source ranks and deliver their spikes; the others go straight to the next
+// step's drive, beside the first ones' waits.  Of the 768-thread CTA's 24 warps, 22 with
+// segment runs (us per step with 24, 22 and 20: N=33,333 x 777 5.65, 5.40, 5.75, N=100,000
+// 7.45, 7.34, 7.39); all of them for long segments and for 1024 threads, whose steps deliver
+// most of the time (N=10^6 at drive 2: 107 with 32 warps, 116 with 28).
+__host__ __device__ constexpr int source_warps(int nt, int mode) {
+  return nt == kTeamNTSmall && mode == kDeliverRun ? 22 : nt / 32;
+}
+
+static_assert(kMaxTeam <= 8 * source_warps(kTeamNT, kDeliverRun) && kMaxTeam <= 8 * source_warps(kTeamNTSmall, kDeliverRun),
+              "a warp polls two lines of at most eight source ranks, two slots of each line a lane");
+
+// The spikes a warp delivers in a step: a concatenation of source ranks' id lists.  Lane k
+// holds source k: its offset in the concatenation and how many of its ids are staged in
+// shared memory.  The source's rank is k, or warp + k x warps where warps have sources of
+// their own.
+struct Source {
+  int off;      // this lane's source: offset in the concatenation (large: no such source)
+  int inl;      // ... ids staged
+  int total;    // ids of the concatenation
+  int q0, dq;   // the warp's batches of 32: positions q0, q0 + dq, ...
+  int wi, wpb;  // ... and its share of each (share wi of wpb)
+  int lt;       // step of the launch
+};
+
+// This lane's spike of the batch at position q0 (whole warps call it): its row and the
+// bounds of this rank's segment in it; an empty segment past the end.
+template <int NT, int kMode>
+__device__ __forceinline__ void fetch_spike(const TeamItem &it, TeamShared &sh, const unsigned char *s_raw,
+                                            const Source &c, int q0, uint64_t pkeep, int &s, int &b, int &e) {
+  const int q = q0 + (threadIdx.x & 31);
+  s = b = e = 0;
+  if (q0 >= c.total) return;
+  int k = 0;  // the source holding position q: the last one that starts at or before it
+#pragma unroll
+  for (int step = 16; step; step >>= 1)
+    if (__shfl_sync(0xFFFFFFFFu, c.off, k + step) <= q) k += step;
+  const int j = q - __shfl_sync(0xFFFFFFFFu, c.off, k), staged = __shfl_sync(0xFFFFFFFFu, c.inl, k);
+  if (q < c.total) {
+    const int r = sh.L.pay_sm ? (int)(threadIdx.x >> 5) + k * source_warps(NT, kMode) : k;
+    if (j < staged) {
+      s = reinterpret_cast<const int *>(s_raw + sh.L.pay)[r * kRankWords + 1 + j];
+    } else {
+      const int par = c.lt & 1;
+      s = tagged_id(j < kInline ? it.rec + ((size_t)par * it.team + r) * kRankWords + 1 + j
+                                : it.list + (size_t)par * it.v.n + (size_t)r * it.rc + j,
+                    it.tag0 + (unsigned)c.lt + 1u, sh, it.sync, sh.lim);
+    }
+    const uint16_t *so = it.seg + (size_t)s * (unsigned)(it.team + 1) + sh.rank;
+    b = ld_keep_u16(so, pkeep);
+    e = ld_keep_u16(so + 1, pkeep);
+  }
+}
+
+// Delivery of a one-CTA team: K whole spiking rows.
+template <int NT, bool kPair>
+__device__ __forceinline__ void deliver_solo(const TeamItem &it, const int *list, int K, unsigned base_a,
+                                             unsigned base_b) {
+  const NetView &v = it.v;
+  if constexpr (kPair) {
+    // warps take the rows in pieces of 128 packed words, two 16-byte vectors a lane in flight
+    // (pieces of 256 words, four vectors, spill: 64 networks in one launch 52.6 ms against 45.5)
+    constexpr int kWarps = NT / 32;
+    const int lane = threadIdx.x & 31;
+    const int rv = v.stride >> 1, np = (rv + 63) >> 6, total = K * np;
+    const int dq = kWarps / np, dp = kWarps - dq * np;
+    const int bits = v.pair_bits;
+    const unsigned tmask = (1u << bits) - 1u;
+    int task = threadIdx.x >> 5, q = task / np, pc = task - q * np;
+    for (; task < total; task += kWarps) {
+      const int rem = rv - pc * 64 - lane;
+      const long long at = syn_row<true>(v, (long long)list[q] * v.stride) + (pc * 64 + lane) * 16;
+      int4 p[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        asm("{.reg .pred p;\n\tsetp.gt.s32 p, %5, %6;\n\t@p ld.global.nc.L1::no_allocate.v4.s32 {%0,%1,%2,%3}, [%4];}"
+            : "=r"(p[u].x), "=r"(p[u].y), "=r"(p[u].z), "=r"(p[u].w)
+            : "l"(at + u * 512), "r"(rem), "r"(u * 32));
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        acc_syn<true, true>(base_a, base_b, bits, tmask, Syn{(unsigned)p[u].x, (unsigned)p[u].y}, rem, u * 32);
+        acc_syn<true, true>(base_a, base_b, bits, tmask, Syn{(unsigned)p[u].z, (unsigned)p[u].w}, rem, u * 32);
+      }
+      q += dq;
+      pc += dp;
+      if (pc >= np) {
+        pc -= np;
+        q += 1;
+      }
+    }
+  } else {
+    const uint64_t pol = policy_evict_first();
+    const int rv = v.stride >> 2;
+    const int total = K * rv;
+    const int dq = NT / rv, dj = NT - dq * rv;
+    int q = threadIdx.x / rv, j = threadIdx.x - q * rv;
+    const int4 *ti = reinterpret_cast<const int4 *>(v.idx);
+    const float4 *wi = reinterpret_cast<const float4 *>(v.w);
+    for (int g = threadIdx.x; g < total; g += 2 * NT) {
+      const size_t o0 = (size_t)list[q] * rv + j;
+      int q1 = q + dq, j1 = j + dj;
+      if (j1 >= rv) {
+        j1 -= rv;
+        q1 += 1;
+      }
+      const bool h1 = g + NT < total;
+      const size_t o1 = h1 ? (size_t)list[q1] * rv + j1 : o0;
+      const int4 t0 = ld_stream_i4(ti + o0, pol), t1 = ld_stream_i4(ti + o1, pol);
+      const float4 w0 = ld_stream_f4(wi + o0, pol), w1 = ld_stream_f4(wi + o1, pol);
+      acc_add4(base_a, base_b, 0, t0, w0);
+      if (h1) acc_add4(base_a, base_b, 0, t1, w1);
+      q = q1 + dq;
+      j = j1 + dj;
+      if (j >= rv) {
+        j -= rv;
+        q += 1;
+      }
+    }
+  }
+}
+
+// Delivery of a larger team, eight lanes a spike (long segments): a batch of 32 spikes is
+// walked in 8 rounds of 4, lane group g (lanes 8g .. 8g+7) reading spike 4r+g's segment in
+// contiguous 64-synapse steps, eight reads a lane in flight; warps sharing a batch take its
+// rounds in turn.  The next batch's ids and bounds are loaded while the current one is
+// walked.  rel_a, rel_b: the shared addresses that neuron 0's accumulator words would have.
+template <int NT, bool kPair>
+__device__ __forceinline__ void deliver_group(const TeamItem &it, TeamShared &sh, const unsigned char *s_raw,
+                                              const Source &c, unsigned rel_a, unsigned rel_b) {
+  const NetView &v = it.v;
+  const int lane = threadIdx.x & 31;
+  const int bits = v.pair_bits;
+  const unsigned tmask = (1u << (bits & 31)) - 1u;
+  const uint64_t pkeep = policy_evict_last();
+  const int sub = lane & 7, grp = lane >> 3;
+  int s, b, e;
+  fetch_spike<NT, kDeliverGroup>(it, sh, s_raw, c, c.q0, pkeep, s, b, e);
+  for (int q0 = c.q0; q0 < c.total; q0 += c.dq) {
+    const long long rowb = syn_row<kPair>(v, (long long)s * v.stride + b);  // segment start of this lane's spike
+    const int len = e - b;
+    fetch_spike<NT, kDeliverGroup>(it, sh, s_raw, c, q0 + c.dq, pkeep, s, b, e);  // next batch, in flight meanwhile
+    for (int r = c.wi; r < 8; r += c.wpb) {
+      long long at = syn_after<kPair>(__shfl_sync(0xFFFFFFFFu, rowb, r * 4 + grp), sub);
+      for (int rem = __shfl_sync(0xFFFFFFFFu, len, r * 4 + grp) - sub; rem > 0; rem -= 64) {
+        Syn x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = load_syn<kPair>(v, at, rem, u * 8);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc_syn<kPair, false>(rel_a, rel_b, bits, tmask, x[u], rem, u * 8);
+        at = syn_after<kPair>(at, 64);
+      }
+    }
+  }
+}
+
+// Delivery of a larger team, segment runs: the segments of a batch of 32 spikes as one run,
+// walked 256 synapses at a time with eight reads a lane in flight; warps sharing a batch
+// take its 256-synapse pieces in turn.  A synapse finds its segment without a search: the
+// heads of the batch's segments are set as bits in shared memory, and the segment's number
+// is the count of heads up to the synapse (the binary search by shuffles that this replaces
+// took about 25 of 93 instructions per 32 synapses; now 32 in all).
+template <int NT, bool kPair>
+__device__ __forceinline__ void deliver_run(const TeamItem &it, TeamShared &sh, const unsigned char *s_raw,
+                                            const Source &c, unsigned rel_a, unsigned rel_b, WarpScratch &ws) {
+  const NetView &v = it.v;
+  const int lane = threadIdx.x & 31;
+  const unsigned lane_le = lanemask_le();
+  const int bits = v.pair_bits;
+  const unsigned tmask = (1u << (bits & 31)) - 1u;
+  const uint64_t pkeep = policy_evict_last();
+  int s, b, e;
+  fetch_spike<NT, kDeliverRun>(it, sh, s_raw, c, c.q0, pkeep, s, b, e);
+  for (int q0 = c.q0; q0 < c.total; q0 += c.dq) {
+    const int len = e - b;
+    int excl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, excl, o);
+      if (lane >= o) excl += y;
+    }
+    const int total = __shfl_sync(0xFFFFFFFFu, excl, 31);
+    excl -= len;
+    const bool has = len > 0;
+    // the batch's segments that are not empty, in order: synapse f of the run that lies in
+    // the k-th of them is f slots after row[k]
+    const unsigned some = __ballot_sync(0xFFFFFFFFu, has);
+    if (has) ws.row[__popc(some & (lane_le >> 1))] = syn_row<kPair>(v, (long long)s * v.stride + b - excl);
+    fetch_spike<NT, kDeliverRun>(it, sh, s_raw, c, q0 + c.dq, pkeep, s, b, e);  // next batch, in flight meanwhile
+    for (int f0 = c.wi * 256; f0 < total; f0 += c.wpb * 256) {
+      const unsigned at = (unsigned)(excl - f0);
+      int k = __popc(__ballot_sync(0xFFFFFFFFu, has && excl < f0)) - 1;
+      if (lane < 8) ws.head[lane] = 0u;
+      __syncwarp();
+      if (has && at < 256u) atomicOr(&ws.head[at >> 5], 1u << (at & 31u));
+      __syncwarp();
+      const int rem = total - f0 - lane;
+      Syn x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const unsigned h = ws.head[u];
+        x[u] = load_syn<kPair>(v, syn_after<kPair>(ws.row[k + __popc(h & lane_le)], f0 + lane), rem, u * 32);
+        k += __popc(h);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc_syn<kPair, false>(rel_a, rel_b, bits, tmask, x[u], rem, u * 32);
+      __syncwarp();  // (the bits are read before they are cleared again)
+    }
+    __syncwarp();
+  }
+}
+
+// The update of a rank's neurons (their arrays, at the slice's first neuron).
+struct Update {
+  float2 *vu;
+  const float4 *abcd;
+  const float *rpar;
+  const float *z;  // the step's drive
+  int *a;
+  unsigned *b;
+  float *ilast;  // input current, on the run's last step (else null)
+  int *own;      // spikes: global ids ...
+  int *nown;     // ... and their count
+  int cnt, nexc; // neurons of the slice; the first nexc are excitatory
+  int lo;        // first neuron
+  float ge, gi;
+};
+
+// kUpd neurons a thread per round, the state loads of all of them first (a slice whose state
+// lives in global memory takes one memory round trip per round), then each in turn; kFromR:
+// a, b, c, d recomputed from the parameter r.  Two rather than four: the registers that
+// leaves are worth more than the round trips (N=2,500 3.69 us a step against 3.84, N=10^6
+// equal, 64 networks in one launch 52.9 ms against 58.3).
+constexpr int kUpd = 2;
+template <int NT, bool kFromR>
+__device__ __forceinline__ void update_slice(const Update &w) {
+  for (int i0 = threadIdx.x; i0 < w.cnt; i0 += kUpd * NT) {
+    float2 sv[kUpd];
+    float rr[kUpd];
+#pragma unroll
+    for (int u = 0; u < kUpd; ++u) {
+      const int i = i0 + u * NT, j = i < w.cnt ? i : i0;
+      sv[u] = w.vu[j];
+      if (kFromR) rr[u] = w.rpar[j];
+    }
+    unsigned spk = 0;
+#pragma unroll
+    for (int u = 0; u < kUpd; ++u) {
+      const int i = i0 + u * NT;
+      if (i < w.cnt) {
+        const float4 p = kFromR ? izh_abcd(rr[u], i < w.nexc) : w.abcd[i];
+        const float isyn = split_current(w.a[i], w.b[i]);
+        float I;
+        const bool k = izh_step(sv[u].x, sv[u].y, I, p, i < w.nexc ? w.ge : w.gi, w.z[i], isyn);
+        w.a[i] = 0;
+        w.b[i] = 0;
+        w.vu[i] = sv[u];
+        if (w.ilast) w.ilast[i] = I;
+        if (k) spk |= 1u << u;
+      }
+    }
+    for (; spk; spk &= spk - 1) w.own[atomicAdd(w.nown, 1)] = w.lo + i0 + (__ffs(spk) - 1) * NT;
+  }
+}
+
+// The drive of step `step` for the slice's neurons, in chunks of 32 handed to warps as they
+// come.  Bound by instruction issue: the generator and the transform take 47 SM cycles per 32
+// normals.  A neuron's first Philox call holds an accepted pair 95% of the time; in slices
+// of more than kListDraws neurons the other draws are repeated in full warps (retried in
+// place, four chunks out of five go through the generator again for one or two lanes: N=10^6
+// at drive 0.5 14.5 us a step against 16.1).  Smaller slices, a chunk or two a warp, retry in
+// place: a second pass by each warp costs them 0.1 us a step more.
+constexpr int kListDraws = 1024;
+__device__ __forceinline__ void drive_chunks(uint64_t seed, int lo, int cnt, int step, float *z, int *next,
+                                             int *retry) {
+  const int lane = threadIdx.x & 31;
+  const unsigned below = lanemask_le() >> 1;
+  const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
+  if (cnt <= kListDraws) {
+    for (;;) {
+      int c = 0;
+      if (lane == 0) c = atomicAdd(next, 1);
+      c = __shfl_sync(0xFFFFFFFFu, c, 0) * 32;
+      if (c >= cnt) return;
+      if (c + lane < cnt) z[c + lane] = normal(seed, (uint64_t)(lo + c + lane), (uint64_t)step);
+    }
+  }
+  int pend = 0;  // neurons in `retry`
+  auto again = [&](int from, int count) {
+    __syncwarp();
+    if (lane < count) {
+      const int i = retry[from + lane];
+      float x = 0.0f, s = 0.0f;
+      bool ok = false;
+      for (uint32_t attempt = 1; attempt < 16 && !ok; ++attempt)
+        ok = normal_try(k0, k1, (uint32_t)(lo + i), (uint32_t)step, attempt, x, s);
+      z[i] = ok ? normal_value(x, s) : 0.0f;
+    }
+    __syncwarp();
+  };
+  for (;;) {
+    int c = 0;
+    if (lane == 0) c = atomicAdd(next, 1);
+    c = __shfl_sync(0xFFFFFFFFu, c, 0) * 32;
+    if (c >= cnt) break;
+    const int i = c + lane;
+    float x = 0.0f, s = 0.0f;
+    bool ok = false;
+    ok = normal_try(k0, k1, (uint32_t)(lo + i), (uint32_t)step, 0, x, s);
+    if (i < cnt && ok) z[i] = normal_value(x, s);
+    const unsigned bad = __ballot_sync(0xFFFFFFFFu, !ok && i < cnt);
+    if (bad) {
+      if (bad >> lane & 1u) retry[pend + __popc(bad & below)] = i;
+      pend += __popc(bad);
+      if (pend >= 32) {
+        pend -= 32;
+        again(pend, 32);
+      }
+    }
+  }
+  if (pend) again(0, pend);
+}
+
 // ---------------------------------------------------------------------------------------
 // One team member's share of one network for the steps of this launch.
 // ---------------------------------------------------------------------------------------
-constexpr int kUpd = 4;  // neurons a thread updates per round of the team kernel's update
 
-template <int NT, bool kPair>
+template <int NT, bool kPair, int kMode, bool kSolo>
 __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, TeamShared &sh,
                          unsigned long long limit_ns, int stall) {
   const NetView &v = it.v;
-  const int T = it.team, rc = it.rc;
-  const TeamLayout L = team_layout(rc, T, it.cap);
-  float4 *s_abcd = reinterpret_cast<float4 *>(s_raw + L.abcd);
-  float2 *s_vu = reinterpret_cast<float2 *>(s_raw + L.vu);
-  int *s_a = reinterpret_cast<int *>(s_raw + L.a);
-  unsigned *s_b = reinterpret_cast<unsigned *>(s_raw + L.b);
-  int *s_own = reinterpret_cast<int *>(s_raw + L.own);
-  float *s_z = reinterpret_cast<float *>(s_raw + L.z);
-  int *s_cnt = reinterpret_cast<int *>(s_raw + L.cnt);
-  int *s_off = reinterpret_cast<int *>(s_raw + L.off);
-  int *s_xoff = reinterpret_cast<int *>(s_raw + L.xoff);
-  int *s_inl = reinterpret_cast<int *>(s_raw + L.inl);
-  unsigned *s_pay = reinterpret_cast<unsigned *>(s_raw + L.pay);
-  uint16_t *s_sb = reinterpret_cast<uint16_t *>(s_raw + L.sb);
-  int *s_pre = reinterpret_cast<int *>(s_raw + L.pre);
-  uint16_t *s_ex = reinterpret_cast<uint16_t *>(s_raw + L.ex);
-  int *s_wsum = reinterpret_cast<int *>(s_raw + L.wsum);
-  int *s_spk = reinterpret_cast<int *>(s_raw + L.spk);
-  const int64_t lo = min((int64_t)rank * rc, v.n);
-  const int64_t hi = min(lo + rc, v.n);
-  const int cnt = (int)(hi - lo);
-  const unsigned base_a = (unsigned)__cvta_generic_to_shared(s_a);
-  const unsigned base_b = (unsigned)__cvta_generic_to_shared(s_b);
-  const unsigned segw = (unsigned)T + 1;
+  const int lo = (int)min((int64_t)rank * it.rc, v.n);
+  const int cnt = (int)min((int64_t)it.rc, v.n - lo);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kWarps = NT / 32;
-  constexpr int kSlots = slots_per_thread(NT);
-  const bool solo = T == 1;   // the whole network in this CTA: no exchange
+  constexpr int kWarps = NT / 32, kSrc = source_warps(NT, kMode);
+  const bool solo = kSolo && it.team == 1;  // the whole network in this CTA: no exchange
   const bool lead = rank == 0 && threadIdx.x == 0;
-  // synapse `off` of the tables: one 8-byte load from the interleaved rows, or two loads
-  auto synapse = [&](long long off, int &t, float &w) {
-    if constexpr (kPair) {
-      const int2 p = __ldg(v.pair + off);
-      t = p.x;
-      w = __int_as_float(p.y);
-    } else {
-      t = __ldg(v.idx + off);
-      w = __ldg(v.w + off);
-    }
-  };
-  // neuron state of the slice: shared memory for the launch when it fits, else global
-  float2 *vu = L.vu_sm ? s_vu : v.vu + lo;
-  const float4 *abcd = L.abcd_sm ? s_abcd : v.abcd + lo;
-  const float *rp = L.abcd_sm ? nullptr : (v.rpar ? v.rpar + lo : nullptr);  // a,b,c,d recomputed from r
+  if (threadIdx.x == 0) {
+    sh.L = team_layout(it.rc, it.team);
+    sh.rank = rank;
+    sh.nown[0] = sh.nown[1] = 0;
+    sh.work[0] = sh.work[1] = 0;
+    sh.k[0] = sh.k[1] = 0;
+    sh.off[0] = sh.off[1] = 0;
+    sh.polled[0] = sh.polled[1] = 0;
+    sh.base = 0;
+    sh.fail = 0;
+  }
+  __shared__ __align__(16) WarpScratch s_ws[kWarps];
+  __syncthreads();
+  const TeamLayout &L = sh.L;
+  // arrays of the slice in shared memory, by their offsets
+  auto s_abcd = [&] { return reinterpret_cast<float4 *>(s_raw + L.abcd); };
+  auto s_vu = [&] { return reinterpret_cast<float2 *>(s_raw + L.vu); };
+  auto s_a = [&] { return reinterpret_cast<int *>(s_raw + L.a); };
+  auto s_b = [&] { return reinterpret_cast<unsigned *>(s_raw + L.b); };
+  auto s_own = [&] { return reinterpret_cast<int *>(s_raw + L.own); };
+  auto s_z = [&] { return reinterpret_cast<float *>(s_raw + L.z); };
+  auto s_pay = [&] { return reinterpret_cast<unsigned *>(s_raw + L.pay); };
 
   for (int i = threadIdx.x; i < cnt; i += NT) {
     const long long q = __ldcg(v.acc + lo + i);
-    s_a[i] = (int)(q >> 16);
-    s_b[i] = (unsigned)(q & 0xFFFF);
-    if (L.vu_sm) s_vu[i] = v.vu[lo + i];
-    if (L.abcd_sm) s_abcd[i] = v.abcd[lo + i];
+    s_a()[i] = (int)(q >> 16);
+    s_b()[i] = (unsigned)(q & 0xFFFF);
+    if (L.vu_sm) s_vu()[i] = v.vu[lo + i];
+    if (L.abcd_sm) s_abcd()[i] = v.abcd[lo + i];
   }
-  if (!solo)  // the first step reads one record line per rank
-    for (int r = threadIdx.x; r <= T; r += NT) s_cnt[r] = 0;
-  if (threadIdx.x == 0) {
-    sh.nown[0] = sh.nown[1] = 0;
-    sh.work[0] = sh.work[1] = 0;
-    sh.fail = 0;
-  }
+  if (L.pay_sm)  // the first step polls one record line per rank
+    for (int r = threadIdx.x; r < it.team; r += NT) s_pay()[r * kRankWords] = 0;
+  if (L.prez) drive_chunks(v.seed, lo, cnt, (int)it.t_abs0, s_z(), &sh.work[1], s_ws[warp].retry);
   __syncthreads();
 
-  long long base = 0;
-  for (int lt = 0; lt < it.steps; ++lt) {
-    const int64_t t_abs = it.t_abs0 + lt;
-    const bool last = it.last && lt == it.steps - 1;
+  const int steps = it.steps;
+  for (int lt = 0; lt < steps; ++lt) {
+    const int t_abs = (int)it.t_abs0 + lt;
+    const bool last = it.last && lt == steps - 1;
     const int par = lt & 1;
     if (threadIdx.x == 0) {
-      sh.nown[par ^ 1] = 0;  // last used by the previous step, next by the following one
+      // the previous step's counters are final: its team count, then cleared for the next step
+      if (lead && lt > 0) v.counts[lt - 1] = sh.k[par ^ 1];
+      sh.base += sh.k[par ^ 1];
+      sh.lim = lt == 0 ? limit_ns * 16 : limit_ns;  // (members may start late)
+      sh.nown[par ^ 1] = 0;
       sh.work[par ^ 1] = 0;
-    }
-    if (lead) {
-      v.base[lt] = base;
-      if (v.stamps) v.stamps[2 * lt] = globaltimer();
-    }
-    // ---- update of the owned neurons, four per thread per round: the state loads of all
-    // four first (a slice whose state lives in global memory takes one memory round trip
-    // per round), then each neuron in turn
-    const bool use_z = L.prez && lt > 0;
-    for (int i0 = threadIdx.x; i0 < cnt; i0 += kUpd * NT) {
-      float2 sv[kUpd];
-      float rr[kUpd];
-#pragma unroll
-      for (int u = 0; u < kUpd; ++u) {
-        const int i = i0 + u * NT, j = i < cnt ? i : i0;
-        sv[u] = vu[j];
-        rr[u] = rp ? rp[j] : 0.0f;
+      sh.k[par ^ 1] = 0;
+      sh.off[par ^ 1] = 0;
+      sh.polled[par ^ 1] = 0;
+      if (lead) {
+        v.base[lt] = sh.base;
+        if (v.stamps) v.stamps[2 * lt] = globaltimer();
       }
-#pragma unroll
-      for (int u = 0; u < kUpd; ++u) {
-        const int i = i0 + u * NT;
-        if (i < cnt) {
-          const int64_t nn = lo + i;
-          const float4 p = rp ? izh_abcd(rr[u], nn < v.nexc) : abcd[i];
-          const long long a = (long long)s_a[i] * 65536 + s_b[i];
-          s_a[i] = 0;
-          s_b[i] = 0;
-          const float z = use_z ? s_z[i] : normal(v.seed, (uint64_t)nn, (uint64_t)t_abs);
-          float I;
-          const bool k = izh_step(sv[u].x, sv[u].y, I, p, nn < v.nexc ? v.ge : v.gi, z, a);
-          vu[i] = sv[u];
-          if (last) v.ilast[nn] = I;
-          if (k) s_own[atomicAdd(&sh.nown[par], 1)] = (int)nn;
-        }
+    }
+    // ---- update of the owned neurons, their state in shared memory for the launch when it
+    // fits, else in global memory (a, b, c, d then recomputed from the parameter r)
+    if (L.prez) {
+      const Update w{L.vu_sm ? s_vu() : v.vu + lo, L.abcd_sm ? s_abcd() : v.abcd + lo, v.rpar + lo, s_z(), s_a(), s_b(),
+                     last ? v.ilast + lo : nullptr, s_own(), &sh.nown[par], cnt, (int)min(v.nexc - lo, (int64_t)cnt),
+                     lo, v.ge, v.gi};
+      if (L.abcd_sm || !v.rpar)
+        update_slice<NT, false>(w);
+      else
+        update_slice<NT, true>(w);
+    } else {
+      // no room for the next step's drive: computed here, one neuron at a time with the next
+      // one's state in flight
+      float2 *vu = v.vu + lo;
+      int *sa = s_a();
+      unsigned *sb = s_b();
+      float2 sn = threadIdx.x < cnt ? vu[threadIdx.x] : make_float2(0.0f, 0.0f);
+      for (int i = threadIdx.x; i < cnt; i += NT) {
+        float2 s = sn;
+        if (i + NT < cnt) sn = vu[i + NT];
+        const int nn = lo + i;
+        const float4 p = v.rpar ? izh_abcd(v.rpar[nn], nn < v.nexc) : v.abcd[nn];
+        const float z = normal(v.seed, (uint64_t)nn, (uint64_t)t_abs);
+        const float isyn = split_current(sa[i], sb[i]);
+        sa[i] = 0;
+        sb[i] = 0;
+        float I;
+        const bool k = izh_step(s.x, s.y, I, p, nn < v.nexc ? v.ge : v.gi, z, isyn);
+        vu[i] = s;
+        if (last) v.ilast[nn] = I;
+        if (k) s_own()[atomicAdd(&sh.nown[par], 1)] = nn;
       }
     }
     __syncthreads();
     const int nown = sh.nown[par];
-    const unsigned long long lim = lt == 0 ? limit_ns * 16 : limit_ns;  // members may start late
     if (stall != 0 && solo) {
       // injected fault of a one-CTA team: wait for a member that does not exist
       if (threadIdx.x == 0) {
-        const unsigned long long t0 = globaltimer();
+        const unsigned long long lim = sh.lim, t0 = globaltimer();
         while (ld_relaxed(&it.sync->error) == 0 && globaltimer() - t0 <= lim) {
         }
         give_up(sh, it.sync);
@@ -514,420 +921,166 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
       __syncthreads();
       return;
     }
-    int K = nown, my_off = 0;
-    const int *list = s_own;
-    const unsigned tag = it.tag0 + (unsigned)lt + 1u;
-    const unsigned long long *recs = it.rec + (size_t)par * T * kRankWords;
-    const unsigned long long *ovf_all = it.list + (size_t)par * v.n;
-    unsigned long long *dense = it.list + (size_t)(2 + par) * v.n;
-    bool gl = false;    // the step's ids are read from the dense list in global memory
-    bool flat = false;  // flat delivery from shared memory
-    int F = 0;          // ... synapses of the concatenated segments
-    const bool zwant = L.prez && lt + 1 < it.steps;  // the next step's drive is precomputed
-    int zdone = 0;      // ... for neurons [0, zdone) already
-    if (!solo) {
-      // ---- publish: both record lines of this rank (count, ids, padding), ids beyond
-      // them in the overflow list; every word tagged with the step, so no fence is needed
+    const unsigned rel_a = (unsigned)__cvta_generic_to_shared(s_a()) - (unsigned)lo * 4u;
+    const unsigned rel_b = (unsigned)__cvta_generic_to_shared(s_b()) - (unsigned)lo * 4u;
+    if (solo) {
+      if (threadIdx.x == 0) {
+        sh.k[par] = nown;
+        if (lead && v.stamps) v.stamps[2 * lt + 1] = globaltimer();
+      }
+      deliver_solo<NT, kPair>(it, s_own(), nown, rel_a, rel_b);
+    } else {
+      Source c;
+      c.lt = lt;
+      const bool own_sources = L.pay_sm;  // every warp polls source ranks of its own
+      const unsigned tag = it.tag0 + (unsigned)lt + 1u;
+      const unsigned long long *recs = it.rec + (size_t)par * it.team * kRankWords;
+      // ---- publish: both record lines of this rank (count, ids, padding), ids beyond them
+      // in the overflow list; every word tagged with the step, so no fence is needed
       {
         const unsigned long long tg = (unsigned long long)tag << 32;
-        unsigned long long *ovf = it.list + (size_t)par * v.n + lo;
-        for (int j = kInline + threadIdx.x; j < nown; j += NT) st_relaxed_u64(ovf + j, tg | (unsigned)s_own[j]);
         if (threadIdx.x < kRankWords) {
           const int j = threadIdx.x;
-          const unsigned pay = j == 0 ? (unsigned)nown : (j - 1 < nown ? (unsigned)s_own[j - 1] : 0xFFFFFFFFu);
-          st_relaxed_u64(it.rec + ((size_t)par * T + rank) * kRankWords + j, tg | pay);
+          const unsigned pay = j == 0 ? (unsigned)nown : (j - 1 < nown ? (unsigned)s_own()[j - 1] : 0xFFFFFFFFu);
+          st_relaxed_u64(it.rec + ((size_t)par * it.team + rank) * kRankWords + j, tg | pay);
         }
+        unsigned long long *ovf = it.list + (size_t)par * v.n + lo;
+        for (int j = kInline + threadIdx.x; j < nown; j += NT) st_relaxed_u64(ovf + j, tg | (unsigned)s_own()[j]);
       }
-      // ---- first pass: line 0 of every rank and line 1 of the ranks that had more than
-      // kLine1After spikes in the previous step, as 16-byte slots (slot x = words 2x, 2x+1 of the
-      // step's records, rank x / 16), up to three per thread; each warp polls its slots
-      // until all carry the step's tag, then the payloads go to shared memory
-      unsigned need = 0;
-#pragma unroll
-      for (int k = 0; k < kSlots; ++k) {
-        const int x = threadIdx.x + k * NT;
-        if (x < T * 16 && ((x & 15) < 8 || s_cnt[x >> 4] > kLine1After)) need |= 1u << k;
-      }
+      // ---- the other ranks' spikes, polled until the words carry the step's tag
+      int n_src, cl = 0;  // sources of this warp; this lane's source's spikes
       unsigned long long t0 = 0;
-      for (int iter = 0;; ++iter) {
-        ulonglong2 a[kSlots];
+      c.inl = 0;
+      if (own_sources) {
+        // every warp its own source ranks warp, warp + kSrc, ...: line 0 of each, and line 1
+        // of those that had more than kLine1After spikes in the previous step, as 16-byte
+        // slots, eight a line, up to two lines' slots per lane.  No warp waits for another
+        // one's sources: it delivers as soon as its own have arrived.
+        n_src = warp < min(kSrc, it.team) ? (it.team - 1 - warp) / kSrc + 1 : 0;
+        if (lane < n_src) c.inl = (int)s_pay()[(warp + lane * kSrc) * kRankWords] > kLine1After ? kInline : kRecWords - 1;
+        unsigned need = 0;
 #pragma unroll
-        for (int k = 0; k < kSlots; ++k)
-          if (need & (1u << k)) a[k] = ld_relaxed_u64x2(recs + 2 * (threadIdx.x + k * NT));
-#pragma unroll
-        for (int k = 0; k < kSlots; ++k)
-          if ((need & (1u << k)) && (unsigned)(a[k].x >> 32) == tag && (unsigned)(a[k].y >> 32) == tag) {
-            const int x = threadIdx.x + k * NT;
-            s_pay[2 * x] = (unsigned)a[k].x;
-            s_pay[2 * x + 1] = (unsigned)a[k].y;
-            need &= ~(1u << k);
-          }
-        if (__all_sync(0xFFFFFFFFu, need == 0) && stall == 0) break;
-        int f = 0;
-        if (lane == 0) {
-          const unsigned long long now = globaltimer();
-          if (iter == 0) t0 = now;
-          f = *(volatile int *)&sh.fail;
-          if (!f && warp == 0 && ld_relaxed(&it.sync->error) != 0) f = 1;
-          if (!f && now - t0 > lim) {
-            give_up(sh, it.sync);
-            f = 1;
-          }
-          if (f) *(volatile int *)&sh.fail = 1;
+        for (int k = 0; k < 4; ++k) {
+          const int x = lane + 32 * (k & 1), src = x >> 3;
+          if (src < n_src && (k < 2 || (int)s_pay()[(warp + src * kSrc) * kRankWords] > kLine1After)) need |= 1u << k;
         }
-        if (__shfl_sync(0xFFFFFFFFu, f, 0)) break;
-      }
-      __syncthreads();
-      if (sh.fail) return;
-      if (warp == 0) {
-        // per rank: count, ids in the lines read (15 or 31), offsets of all ids and of
-        // those beyond the lines read
-        constexpr int kPer = kMaxTeam / 32;
-        int c[kPer], xr[kPer], sc = 0, sx = 0;
+        __syncwarp();
+        for (int iter = 0;; ++iter) {
+          ulonglong2 a[4];
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-          const int r = lane * kPer + k;
-          c[k] = 0;
-          xr[k] = 0;
-          if (r < T) {
-            const int inl = s_cnt[r] > kLine1After ? kInline : kRecWords - 1;
-            c[k] = (int)s_pay[r * kRankWords];
-            xr[k] = max(0, c[k] - inl);
-            s_inl[r] = inl;
+          for (int k = 0; k < 4; ++k) {
+            const int x = lane + 32 * (k & 1);
+            if (need & (1u << k))
+              a[k] = ld_relaxed_u64x2(recs + (warp + (x >> 3) * kSrc) * kRankWords + (k >> 1) * kRecWords + 2 * (x & 7));
           }
-          sc += c[k];
-          sx += xr[k];
-        }
-        int ic = sc, ix = sx;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int yc = __shfl_up_sync(0xFFFFFFFFu, ic, o), yx = __shfl_up_sync(0xFFFFFFFFu, ix, o);
-          if (lane >= o) {
-            ic += yc;
-            ix += yx;
-          }
-        }
-        int ec = ic - sc, ex = ix - sx;
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-          const int r = lane * kPer + k;
-          if (r < T) {
-            s_cnt[r] = c[k];
-            s_off[r] = ec;
-            s_xoff[r] = ex;
-          }
-          ec += c[k];
-          ex += xr[k];
-        }
-        if (lane == 31) {
-          s_off[T] = ec;
-          s_xoff[T] = ex;
-        }
-      }
-      __syncthreads();
-      K = s_off[T];
-      my_off = s_off[rank];
-      list = s_spk;
-      if (K > it.cap) {
-        // many spikes: instead of staging windows, every rank writes its ids (tagged) at
-        // its offset in the step's dense list, which the delivery reads directly
-        gl = true;
-        const unsigned long long tg = (unsigned long long)tag << 32;
-        for (int j = threadIdx.x; j < nown; j += NT) st_relaxed_u64(dense + my_off + j, tg | (unsigned)s_own[j]);
-      }
-    }
-    if (lead && v.stamps) v.stamps[2 * lt + 1] = globaltimer();
-    if (lead) v.counts[lt] = K;
-
-    {
-      const int Kw = K;
-      if (!solo && !gl && K > 0) {
-        // ---- stage the step's spike ids in shared memory: the first pass's payloads,
-        // then ids beyond the lines read, polled from the records or the overflow list
-        {
-#pragma unroll
-          for (int k = 0; k < kSlots; ++k) {
-            const int x = threadIdx.x + k * NT;
-            if (x < T * 16) {
-              const int r = x >> 4, w0 = 2 * (x & 15), c = min(s_cnt[r], s_inl[r]), o = s_off[r] - 1;
-              if (w0 >= 1 && w0 - 1 < c) s_spk[o + w0] = (int)s_pay[2 * x];
-              if (w0 < c) s_spk[o + w0 + 1] = (int)s_pay[2 * x + 1];
+          for (int k = 0; k < 4; ++k) {
+            const int x = lane + 32 * (k & 1);
+            if ((need & (1u << k)) && (unsigned)(a[k].x >> 32) == tag && (unsigned)(a[k].y >> 32) == tag) {
+              *reinterpret_cast<uint2 *>(s_pay() + (warp + (x >> 3) * kSrc) * kRankWords + (k >> 1) * kRecWords + 2 * (x & 7)) =
+                  make_uint2((unsigned)a[k].x, (unsigned)a[k].y);
+              need &= ~(1u << k);
             }
           }
-          const int X = s_xoff[T];
-          for (int e = threadIdx.x; e < X; e += NT) {
-            const int r = find_run(s_xoff, T, e);
-            const int j = s_inl[r] + e - s_xoff[r];
-            s_spk[s_off[r] + j] = tagged_id(
-                j < kInline ? recs + (size_t)r * kRankWords + 1 + j : ovf_all + (size_t)r * rc + j, tag, sh, it.sync, lim);
-          }
+          if (__all_sync(0xFFFFFFFFu, need == 0) && stall == 0) break;
+          if (poll_check(sh, it.sync, iter, t0, sh.lim)) break;
         }
-        __syncthreads();
-        if (sh.fail) return;
+        __syncwarp();
+        if (lane < n_src) cl = (int)s_pay()[(warp + lane * kSrc) * kRankWords];
+      } else {
+        // few ranks: every warp reads every rank's count and takes its share of the batches
+        n_src = it.team;
+        for (int iter = 0;; ++iter) {
+          unsigned long long w = 0;
+          if (lane < n_src) w = ld_relaxed_u64(recs + lane * kRankWords);
+          if (__all_sync(0xFFFFFFFFu, lane >= n_src || (unsigned)(w >> 32) == tag) && stall == 0) {
+            cl = lane < n_src ? (int)(unsigned)w : 0;
+            break;
+          }
+          if (poll_check(sh, it.sync, iter, t0, sh.lim)) break;
+        }
       }
-      // (a smaller CTA takes the flat mapping only for steps too small to give most of its
-      // warps a 32-spike batch of the run mapping, which measured faster above that)
-      if (!solo && !gl && K >= kFlatMinSpikes && L.flat && K <= 4 * NT && (NT >= 1024 || K < NT / 2)) {
-        // segment bounds and their offsets in the concatenation (for the flat delivery):
-        // thread t takes spikes 4t .. 4t+3 (K <= 4 NT); a block scan of their
-        // lengths (every warp scans the warp sums itself), then each thread marks the
-        // synapses of its spikes with the spike's index
-        const uint64_t pkeep = policy_evict_last();
-        int len[4], b4[4], sum = 0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int q = threadIdx.x * 4 + u;
-          len[u] = 0;
-          b4[u] = 0;
-          if (q < K) {
-            const uint16_t *so = it.seg + (size_t)s_spk[q] * segw + rank;
-            b4[u] = ld_keep_u16(so, pkeep);
-            len[u] = ld_keep_u16(so + 1, pkeep) - b4[u];
-          }
-          sum += len[u];
-        }
-        int incl = sum;
+      {
+        int incl = cl, below = (own_sources ? warp + lane * kSrc : lane) < rank ? cl : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
           if (lane >= o) incl += y;
+          below += __shfl_xor_sync(0xFFFFFFFFu, below, o);
         }
-        if (lane == 31) s_wsum[warp] = incl;
-        __syncthreads();
-        const int ws = lane < kWarps ? s_wsum[lane] : 0;
-        int wi = ws;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xFFFFFFFFu, wi, o);
-          if (lane >= o) wi += y;
-        }
-        F = __shfl_sync(0xFFFFFFFFu, wi, 31);
-        flat = F <= kFlatMax;
-        if (flat) {
-          int pre = __shfl_sync(0xFFFFFFFFu, wi - ws, warp) + incl - sum;
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int q = threadIdx.x * 4 + u;
-            if (q < K) {
-              s_pre[q] = pre;
-              s_sb[q] = (uint16_t)b4[u];
-              for (int f = pre; f < pre + len[u]; ++f) s_ex[f] = (uint16_t)q;
-            }
-            pre += len[u];
-          }
-        }
-        __syncthreads();
-      }
-      if (solo) {
-        // ---- delivery, one-CTA team: flat over K whole rows of stride/4 vectors
-        const int rv = v.stride >> 2;
-        const int total = Kw * rv;
-        const int dq = NT / rv, dj = NT - dq * rv;
-        int q = threadIdx.x / rv, j = threadIdx.x - q * rv;
-        const int4 *ti = reinterpret_cast<const int4 *>(v.idx);
-        const float4 *wi = reinterpret_cast<const float4 *>(v.w);
-        const uint64_t pol = policy_evict_first();
-        for (int g = threadIdx.x; g < total; g += 2 * NT) {
-          const size_t o0 = (size_t)list[q] * rv + j;
-          int q1 = q + dq, j1 = j + dj;
-          if (j1 >= rv) {
-            j1 -= rv;
-            q1 += 1;
-          }
-          const bool h1 = g + NT < total;
-          const size_t o1 = h1 ? (size_t)list[q1] * rv + j1 : o0;
-          const int4 t0 = ld_stream_i4(ti + o0, pol), t1 = ld_stream_i4(ti + o1, pol);
-          const float4 w0 = ld_stream_f4(wi + o0, pol), w1 = ld_stream_f4(wi + o1, pol);
-          acc_add4(base_a, base_b, 0, t0, w0);
-          if (h1) acc_add4(base_a, base_b, 0, t1, w1);
-          q = q1 + dq;
-          j = j1 + dj;
-          if (j >= rv) {
-            j -= rv;
-            q += 1;
-          }
-        }
-      } else if (flat) {
-        // ---- delivery, larger team, flat: each thread walks synapses f = tid, tid + NT,
-        // ... of the concatenated segments (consecutive lanes, consecutive synapses),
-        // eight table reads in flight, no shuffles; its next-step drive is computed
-        // while the reads are in flight
-        for (int f0 = threadIdx.x, pass = 0; pass == 0 || f0 < F; f0 += 8 * NT, ++pass) {
-          int t[8];
-          float w[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int f = f0 + u * NT;
-            t[u] = -1;
-            w[u] = 0.0f;
-            if (f < F) {
-              const int q = s_ex[f];
-              const long long off = (long long)s_spk[q] * v.stride + s_sb[q] + (f - s_pre[q]);
-              // (the separate arrays: consecutive lanes read consecutive synapses here, and
-              // two 4-byte loads measured faster than one 8-byte load of the interleaved rows)
-              t[u] = __ldg(v.idx + off);
-              w[u] = __ldg(v.w + off);
-            }
-          }
-          if (pass == 0 && zwant && threadIdx.x < cnt)
-            s_z[threadIdx.x] = normal(v.seed, (uint64_t)(lo + threadIdx.x), (uint64_t)(t_abs + 1));
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (t[u] >= 0) acc_add(base_a, base_b, (unsigned)(t[u] - (int)lo), wfix(w[u]));
-        }
-        zdone = zwant ? min(cnt, NT) : 0;
-      } else if (it.mode == kDeliverGroup) {
-        // ---- delivery, larger team, eight lanes a spike (long segments): warps take the
-        // step's spikes in batches of 32 as in the run mapping (`wpb` warps sharing a batch's
-        // rounds when there are fewer batches than warps); a batch is walked in 8 rounds of 4
-        // spikes, lane group g (lanes 8g .. 8g+7) reading spike 4r+g's segment in contiguous
-        // 64-synapse steps, eight reads a lane in flight.  No search: a segment's synapses
-        // need no shuffles to find their spike.  The next batch's ids and bounds are loaded
-        // while the current one is walked.
-        const uint64_t pkeep = policy_evict_last();
-        const int nbatch = (Kw + 31) >> 5;
-        const int wpb = nbatch >= kWarps ? 1 : min(8, kWarps / max(nbatch, 1));
-        const int groups = kWarps / wpb, gw = warp / wpb, wi = warp % wpb;
-        const int sub = lane & 7, grp = lane >> 3;
-        int s = 0, b = 0, e = 0;
-        auto fetch = [&](int batch) {
-          const int q = batch * 32 + lane;
-          s = 0;
-          b = 0;
-          e = 0;
-          if (gw < groups && batch < nbatch && q < Kw) {
-            s = gl ? tagged_id(dense + q, tag, sh, it.sync, lim) : list[q];
-            const uint16_t *so = it.seg + (size_t)s * segw + rank;
-            b = ld_keep_u16(so, pkeep);
-            e = ld_keep_u16(so + 1, pkeep);
-          }
-        };
-        fetch(gw);
-        for (int batch = gw; gw < groups && batch < nbatch; batch += groups) {
-          const long long rowb = (long long)s * v.stride + b;  // segment start of this lane's spike
-          const int len = e - b;
-          fetch(batch + groups);  // next batch, in flight meanwhile
-          for (int r = wi; r < 8; r += wpb) {
-            const long long rb = __shfl_sync(0xFFFFFFFFu, rowb, r * 4 + grp);
-            const int ln = __shfl_sync(0xFFFFFFFFu, len, r * 4 + grp);
-            for (int k0 = 0; k0 < ln; k0 += 64) {
-              int t[8];
-              float w[8];
-#pragma unroll
-              for (int u = 0; u < 8; ++u) {
-                const int k = k0 + u * 8 + sub;
-                t[u] = -1;
-                w[u] = 0.0f;
-                if (k < ln) synapse(rb + k, t[u], w[u]);
-              }
-#pragma unroll
-              for (int u = 0; u < 8; ++u)
-                if (t[u] >= 0) acc_add(base_a, base_b, (unsigned)(t[u] - (int)lo), wfix(w[u]));
-            }
-          }
-        }
-      } else {
-        // ---- delivery, larger team: this rank's segment of every spiking row.  Spikes go
-        // to warps in batches of 32; when there are fewer batches than warps, `wpb` warps
-        // share a batch and split its run.  The next batch's spike ids and segment bounds
-        // are loaded before the current run is walked.
-        const uint64_t pkeep = policy_evict_last();
-        const int nbatch = (Kw + 31) >> 5;
-        const int wpb = nbatch >= kWarps ? 1 : kWarps / max(nbatch, 1);
-        const int groups = kWarps / wpb, gw = warp / wpb, wi = warp % wpb;
-        int s = 0, b = 0, len = 0;
-        auto fetch = [&](int batch) {
-          const int q = batch * 32 + lane;
-          s = 0;
-          b = 0;
-          len = 0;
-          if (gw < groups && batch < nbatch && q < Kw) {
-            s = gl ? tagged_id(dense + q, tag, sh, it.sync, lim) : list[q];
-            const uint16_t *so = it.seg + (size_t)s * segw + rank;
-            b = ld_keep_u16(so, pkeep);
-            len = ld_keep_u16(so + 1, pkeep) - b;
-          }
-        };
-        fetch(gw);
-        for (int batch = gw; gw < groups && batch < nbatch; batch += groups) {
-          int incl = len;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += y;
-          }
-          const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-          const int excl = incl - len;
-          const long long rowoff = (long long)s * v.stride + b - excl;  // synapse f of the run: rowoff_j + f
-          fetch(batch + groups);                                        // next batch, in flight meanwhile
-          for (int f0 = wi * 256; f0 < total; f0 += wpb * 256) {
-            int t[8];
-            float w[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const int f = f0 + u * 32 + lane;
-              // spike j of the run holding f: last lane whose exclusive prefix is <= f
-              int jj = 0;
-#pragma unroll
-              for (int step = 16; step; step >>= 1) {
-                const int e = __shfl_sync(0xFFFFFFFFu, excl, jj + step);
-                if (e <= f) jj += step;
-              }
-              const long long off = __shfl_sync(0xFFFFFFFFu, rowoff, jj) + f;
-              t[u] = -1;
-              w[u] = 0.0f;
-              if (f < total) {
-                synapse(off, t[u], w[u]);
-              }
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (t[u] >= 0) acc_add(base_a, base_b, (unsigned)(t[u] - (int)lo), wfix(w[u]));
-          }
+        c.total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        c.off = lane < n_src ? incl - cl : INT_MAX;
+        if (lane == 0 && (own_sources || warp == 0)) {
+          // the step's team count and this rank's raster offset, for the tail
+          if (c.total) atomicAdd(&sh.k[par], c.total);
+          if (below) atomicAdd(&sh.off[par], below);
+          __threadfence_block();
+          atomicAdd(&sh.polled[par], 1);
         }
       }
+      if (lead && v.stamps) v.stamps[2 * lt + 1] = globaltimer();
+      if (*(volatile int *)&sh.fail) c.total = 0;  // (the words read may be old)
+      c.q0 = 0;
+      c.dq = 32;
+      c.wi = 0;
+      c.wpb = 1;
+      if (!own_sources) {
+        const int nbatch = (c.total + 31) >> 5;
+        int wpb = nbatch >= kWarps ? 1 : kWarps / max(nbatch, 1);
+        if (kMode == kDeliverGroup) wpb = min(8, wpb);
+        const int groups = kWarps / wpb;
+        c.q0 = warp / wpb < groups ? warp / wpb * 32 : c.total;
+        c.dq = groups * 32;
+        c.wi = warp % wpb;
+        c.wpb = wpb;
+      }
+      if constexpr (kMode == kDeliverGroup)
+        deliver_group<NT, kPair>(it, sh, s_raw, c, rel_a, rel_b);
+      else
+        deliver_run<NT, kPair>(it, sh, s_raw, c, rel_a, rel_b, s_ws[warp]);
     }
     // ---- tail, by warps as they finish delivering: the raster and the statistics of this
-    // rank's spikes (from the highest thread down, i.e. warps that had no delivery batch
-    // first), then the next step's drive in chunks of 32 neurons
-    for (int j = NT - 1 - threadIdx.x; j < nown; j += NT) {
-      const int n = s_own[j];
-      const long long pos = base + my_off + j;
-      if (pos < v.raster_cap) v.raster[pos] = n;
-      SpikeStat st = v.sstat[n];
-      st.nospks += 1;
-      if (st.last >= 0) {
-        const long long isi = t_abs - st.last;
-        st.nisi += 1;
-        st.s1 += isi;
-        st.s2 += isi * isi;
+    // rank's spikes (from the highest thread down), then the next step's drive in chunks of
+    // 32 neurons
+    if (NT - 32 - warp * 32 < nown) {
+      if (!solo) {  // (every warp's sources are counted, unless the exchange gave up)
+        const int all = L.pay_sm ? kWarps : 1;
+        while (*(volatile int *)&sh.polled[par] < all && !*(volatile int *)&sh.fail) {
+        }
+        __threadfence_block();
       }
-      st.last = (int)t_abs;
-      v.sstat[n] = st;
+      const long long pos0 = sh.base + *(volatile int *)&sh.off[par];
+      for (int j = NT - 1 - threadIdx.x; j < nown; j += NT) {
+        const int n = s_own()[j];
+        if (pos0 + j < v.raster_cap) v.raster[pos0 + j] = n;
+        SpikeStat st = v.sstat[n];
+        st.nospks += 1;
+        if (st.last >= 0) {
+          const long long isi = t_abs - st.last;
+          st.nisi += 1;
+          st.s1 += isi;
+          st.s2 += isi * isi;
+        }
+        st.last = t_abs;
+        v.sstat[n] = st;
+      }
     }
-    if (zwant)
-      for (;;) {
-        int c = 0;
-        if (lane == 0) c = atomicAdd(&sh.work[par], 1);
-        c = __shfl_sync(0xFFFFFFFFu, c, 0) * 32 + zdone;
-        if (c >= cnt) break;
-        const int i = c + lane;
-        if (i < cnt) s_z[i] = normal(v.seed, (uint64_t)(lo + i), (uint64_t)(t_abs + 1));
-      }
+    if (L.prez && lt + 1 < steps)
+      drive_chunks(v.seed, lo, cnt, t_abs + 1, s_z(), &sh.work[par], s_ws[warp].retry);
     __syncthreads();
-    if (gl && sh.fail) return;
-    base += K;
+    if (!solo && sh.fail) return;
   }
+  if (lead) v.counts[steps - 1] = sh.k[(steps - 1) & 1];
   // pending currents (from the last delivery) and the state back to global memory
   for (int i = threadIdx.x; i < cnt; i += NT) {
-    v.acc[lo + i] = (long long)s_a[i] * 65536 + s_b[i];
-    if (L.vu_sm) v.vu[lo + i] = s_vu[i];
+    v.acc[lo + i] = (long long)s_a()[i] * 65536 + s_b()[i];
+    if (L.vu_sm) v.vu[lo + i] = s_vu()[i];
   }
   __syncthreads();
 }
 
 // The persistent grid: CTAs take (network, rank) slots until the queue is empty.
-template <int NT, bool kPair>
+template <int NT, bool kPair, int kMode, bool kSolo>
 __global__ void __launch_bounds__(NT, 1) k_team(const TeamItem *__restrict__ items, const int2 *__restrict__ slots,
                                                 const int *nslots, int *slot_head, unsigned long long limit_ns,
                                                 int stall) {
@@ -945,7 +1098,7 @@ __global__ void __launch_bounds__(NT, 1) k_team(const TeamItem *__restrict__ ite
     __shared__ TeamItem s_it;
     if (threadIdx.x == 0) s_it = items[x.x];
     __syncthreads();
-    if (s_it.steps > 0) team_run<NT, kPair>(s_it, x.y, s_raw, sh, limit_ns, stall);
+    if (s_it.steps > 0) team_run<NT, kPair, kMode, kSolo>(s_it, x.y, s_raw, sh, limit_ns, stall);
     __syncthreads();
   }
 }
@@ -956,36 +1109,38 @@ __global__ void __launch_bounds__(NT, 1) k_team(const TeamItem *__restrict__ ite
 
 size_t team_smem(int64_t rc, int team) {
   if (rc < 1 || team < 1 || team > kMaxTeam) return 0;
-  const int cap = team_window(rc, team);
-  if (team > 1 && cap == 0) return 0;
-  const size_t bytes = team_layout(rc, team, cap).bytes;
+  const size_t bytes = team_layout(rc, team).bytes;
   return bytes > kTeamSmemLimit ? 0 : (bytes < 16 ? 16 : bytes);
+}
+
+// The instantiation of the team kernel for a CTA size, table layout and delivery mapping.
+using TeamKernel = void (*)(const TeamItem *, const int2 *, const int *, int *, unsigned long long, int);
+template <int NT, bool kPair, int kMode>
+static TeamKernel team_kernel_of(bool solo) {
+  return solo ? k_team<NT, kPair, kMode, true> : k_team<NT, kPair, kMode, false>;
+}
+template <int NT>
+static TeamKernel team_kernel_nt(bool pair, int mode, bool solo) {
+  if (mode == kDeliverGroup)
+    return pair ? team_kernel_of<NT, true, kDeliverGroup>(solo) : team_kernel_of<NT, false, kDeliverGroup>(solo);
+  return pair ? team_kernel_of<NT, true, kDeliverRun>(solo) : team_kernel_of<NT, false, kDeliverRun>(solo);
+}
+static TeamKernel team_kernel(int nt, bool pair, int mode, bool solo) {
+  return nt == kTeamNTSmall ? team_kernel_nt<kTeamNTSmall>(pair, mode, solo) : team_kernel_nt<kTeamNT>(pair, mode, solo);
+}
+constexpr int kTeamVariants = 8;  // of one CTA size
+static TeamKernel team_variant(int nt, int k) {
+  return team_kernel(nt, k & 1, k & 2 ? kDeliverGroup : kDeliverRun, k & 4);
 }
 
 // The kernel's shared-memory ceiling is always the largest layout's (every team layout
 // stays under it), so host threads that launch teams of different sizes never lower it
 // under one another, and a captured launch needs no attribute call.
-template <int NT>
-static cudaError_t team_ceiling_nt() {
-  cudaError_t e = cudaFuncSetAttribute(k_team<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTeamSmemLimit);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_team<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTeamSmemLimit);
-  return e;
-}
-
 cudaError_t team_smem_ceiling() {
-  cudaError_t e = team_ceiling_nt<kTeamNT>();
-  return e == cudaSuccess ? team_ceiling_nt<kTeamNTSmall>() : e;
-}
-
-// CTAs of the team kernel with `smem` bytes of shared memory that fit an SM (both table
-// layouts' instantiations; they need the same resources)
-template <int NT>
-static cudaError_t team_occupancy(size_t smem, int *occ) {
-  int a = 0, b = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_team<NT, true>, NT, smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_team<NT, false>, NT, smem);
-  *occ = a < b ? a : b;
+  cudaError_t e = cudaSuccess;
+  for (int nt : {kTeamNT, kTeamNTSmall})
+    for (int k = 0; k < kTeamVariants && e == cudaSuccess; ++k)
+      e = cudaFuncSetAttribute(team_variant(nt, k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTeamSmemLimit);
   return e;
 }
 
@@ -993,18 +1148,23 @@ cudaError_t team_max_blocks(size_t smem, int *out, int nt) {
   if (smem > kTeamSmemLimit || (nt != kTeamNT && nt != kTeamNTSmall)) return cudaErrorInvalidValue;
   cudaError_t e = team_smem_ceiling();
   if (e != cudaSuccess) return e;
-  int occ = 0;
-  e = nt == kTeamNT ? team_occupancy<kTeamNT>(smem, &occ) : team_occupancy<kTeamNTSmall>(smem, &occ);
-  if (e != cudaSuccess) return e;
+  int least = INT_MAX;  // (of the instantiations, which need nearly the same resources)
+  for (int k = 0; k < kTeamVariants; ++k) {
+    int occ = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, team_variant(nt, k), nt, smem);
+    if (e != cudaSuccess) return e;
+    least = std::min(least, occ);
+  }
   int dev = 0, sms = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  *out = occ * sms;
+  *out = least * sms;
   return cudaSuccess;
 }
 
 cudaError_t launch_team(const TeamItem *items, const int2 *slots, const int *nslots, int *slot_head, int grid,
-                        size_t smem, unsigned long long limit_ns, int stall, cudaStream_t s, bool pair, int nt) {
+                        size_t smem, unsigned long long limit_ns, int stall, cudaStream_t s, bool pair, int mode,
+                        bool solo, int nt) {
   if (smem > kTeamSmemLimit || (nt != kTeamNT && nt != kTeamNTSmall)) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
@@ -1016,11 +1176,7 @@ cudaError_t launch_team(const TeamItem *items, const int2 *slots, const int *nsl
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (nt == kTeamNTSmall)
-    return pair ? cudaLaunchKernelEx(&cfg, k_team<kTeamNTSmall, true>, items, slots, nslots, slot_head, limit_ns, stall)
-                : cudaLaunchKernelEx(&cfg, k_team<kTeamNTSmall, false>, items, slots, nslots, slot_head, limit_ns, stall);
-  return pair ? cudaLaunchKernelEx(&cfg, k_team<kTeamNT, true>, items, slots, nslots, slot_head, limit_ns, stall)
-              : cudaLaunchKernelEx(&cfg, k_team<kTeamNT, false>, items, slots, nslots, slot_head, limit_ns, stall);
+  return cudaLaunchKernelEx(&cfg, team_kernel(nt, pair, mode, solo), items, slots, nslots, slot_head, limit_ns, stall);
 }
 
 cudaError_t launch_rows_sorted(const NetView &v, int *unsorted, cudaStream_t s) {
@@ -1179,7 +1335,8 @@ cudaError_t launch_pairs(const NetView &v, cudaStream_t s) {
   int dev = 0, sms = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  k_pairs<<<(unsigned)(sms * 8), 512, 0, s>>>(v, const_cast<int2 *>(v.pair));
+  k_pairs<<<(unsigned)(sms * 4), 512, 0, s>>>(
+      v, reinterpret_cast<ulonglong2 *>(const_cast<unsigned long long *>(v.pair)));
   return cudaGetLastError();
 }
 

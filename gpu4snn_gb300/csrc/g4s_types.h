@@ -49,8 +49,9 @@ struct NetView {
   SpikeStat *sstat;
   const int *idx;   // [n][stride] targets
   const float *w;   // [n][stride] weights
-  const int2 *pair;  // [n][stride] the same rows interleaved (target, weight bits): one
-                     // contiguous run per segment for the team kernel (may be null)
+  const unsigned long long *pair;  // [n][stride] the same rows, one word a synapse for the team kernel:
+                                   // Q32.32 weight << pair_bits | target (may be null)
+  int32_t pair_bits;               // bits of the target field, 16..31
   int *raster;      // spike ids of the current chunk, step after step
   int64_t raster_cap;
   int *counts;      // spikes per step of the current chunk
@@ -64,8 +65,8 @@ struct NetView {
 struct TeamItem {
   NetView v;
   const uint16_t *seg;  // [n][team+1] row segment offsets (team > 1)
-  unsigned long long *list;  // [4][n] tagged spike ids, by step parity: [par] beyond a rank's record
-                             // lines (at its neuron offset), [2 + par] the step's dense list
+  unsigned long long *list;  // [2][n] tagged spike ids beyond a rank's record lines (at its neuron
+                             // offset), by step parity
   unsigned long long *rec;   // [2][team][2 x 16] tagged spike records, by step parity (zero at launch)
   int64_t t_abs0;       // absolute step of the first step of this launch
   int steps;            // steps of this launch (0: nothing to do)
@@ -73,21 +74,19 @@ struct TeamItem {
   int team;             // CTAs of the team
   int rc;               // neurons per CTA slice
   GridSync *sync;       // error word of the team
-  int mode;             // delivery mapping of a multi-CTA team (kDeliverRun or kDeliverGroup)
-  int cap;              // delivery window of a multi-CTA rank (spike ids in shared memory)
   unsigned tag0;        // record tag of step lt: tag0 + lt + 1 (never repeats for the list's words)
 };
 
 // Delivery mappings of a multi-CTA team: warps walk the concatenated segments of 32
-// spikes, each synapse finding its spike by a search over the batch (kDeliverRun, for
-// short segments), or groups of eight lanes walk one spike's segment each (kDeliverGroup,
-// for long segments: no search); kDeliverAuto picks by the mean segment length.
+// spikes (kDeliverRun, for short segments), or groups of eight lanes walk one spike's
+// segment each (kDeliverGroup, for long segments); kDeliverAuto picks by the mean segment
+// length.
 constexpr int kDeliverAuto = -1;
 constexpr int kDeliverRun = 0;
 constexpr int kDeliverGroup = 1;
 // mean synapses of a rank's segment of a row (Nsyn / team) from which kDeliverAuto takes the
-// eight-lane groups (measured in the team kernel: even with the runs at ~26 synapses, 14%
-// faster per step at ~66)
+// eight-lane groups (us per step, groups / runs: segments of ~26 synapses 7.4 / 6.4 at
+// N=30,000 and 14.7 / 12.2 at 100,000, ~40 24.8 / 24.6 at 200,000, ~66 40.0 / 43.1 at 250,000)
 constexpr int kGroupMinSegment = 24;
 
 }  // namespace g4s

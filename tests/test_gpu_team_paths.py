@@ -1,0 +1,58 @@
+"""The team kernel's exchange and table layouts at their edges, against the oracle: team
+sizes around the one from which warps poll source ranks of their own, ranks with more spikes
+than their record lines hold, and weights too large to be packed beside their targets."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def run_both(g4s, oracle, n, nsyn, seed, drive, steps, geometry, threads, scale=None):
+    d = oracle.make_desc(n, nsyn, seed, drive_scale=drive)
+    idx, w = oracle.conn_philox(d)
+    if scale is not None:  # a few weights scaled up, at the ends of rows and of the table
+        w = w.copy()
+        for pos in (0, n * nsyn // 2, n * w.shape[1] - 1 - (w.shape[1] - nsyn)):
+            w.flat[pos] = scale
+    sim = oracle.Sim(d, idx, w)
+    sim.run(steps, threads=8)
+    with g4s.Network(n, nsyn, seed=seed, drive_scale=drive, tables=(idx, w)) as net:
+        net.set_geometry(*geometry)
+        net.set_block_threads(threads)
+        net.run(steps // 2, 4)
+        net.run(steps - steps // 2, 4)
+        assert np.array_equal(np.stack(net.raster()), np.stack(sim.raster()))
+        s, o = net.state(), sim.state()
+        for k in ("v", "u", "I"):
+            # (a neuron whose potential overflows ends with u = NaN, whose bits differ by machine)
+            a, b = s[k], o[k]
+            assert np.array_equal(np.isnan(a), np.isnan(b)), k
+            assert np.array_equal(a[~np.isnan(a)].view(np.uint32), b[~np.isnan(b)].view(np.uint32)), k
+        assert np.array_equal(s["nospks"], o["nospks"])
+        assert np.array_equal(net.currents(), sim.acc())
+        return net.counts()
+
+
+@pytest.mark.parametrize("threads", [768, 1024])
+@pytest.mark.parametrize("p", [2, 11, 12, 13, 22, 23, 25, 33])
+def test_source_ranks(g4s, oracle, p, threads):
+    """A rank's few hundred neurons at drive 2 (about 60 spikes a step in the first burst):
+    more ids than a record's lines hold, in teams on both sides of every split of the ranks
+    over the warps."""
+    counts = run_both(g4s, oracle, 3001, 203, 51, 2.0, 60, (p, 0), threads)
+    assert counts.max() > 31 * 2
+
+
+@pytest.mark.parametrize("delivery", [0, 1])
+def test_single_spikes_and_bursts(g4s, oracle, delivery):
+    """Steps without any spike, and a burst with more than 64 spikes a rank."""
+    counts = run_both(g4s, oracle, 5003, 203, 52, 2.0, 60, (16, delivery), 0)
+    assert counts.max() > 16 * 64 and counts.min() == 0
+
+
+@pytest.mark.parametrize("geometry", [(0, 0), (40, 1), (9, 0)])
+@pytest.mark.parametrize("scale", [16383.0, 20000.0, -20000.0])
+def test_weights_at_the_packing_limit(g4s, oracle, geometry, scale):
+    """70,000 targets take 17 bits of a packed word, which leaves Q32.32 weights below 2^14:
+    16383 is packed, +-20000 sends the network to the separate arrays."""
+    run_both(g4s, oracle, 70_000, 8, 53, 2.0, 40, geometry, 0, scale)
