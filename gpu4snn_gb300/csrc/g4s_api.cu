@@ -952,6 +952,7 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
     g4s_net *n = nets[i];
     TeamItem &it = L.h_items[i];
     it.v = n->v;
+    if (!n->desc.record_raster) it.v.raster_cap = 0;  // (its raster is never read)
     it.seg = n->seg;
     it.list = n->list;
     it.rec = reinterpret_cast<unsigned long long *>(n->gs + 1);
