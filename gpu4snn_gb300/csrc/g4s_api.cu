@@ -199,6 +199,7 @@ struct g4s_net {
   long long *h_base = nullptr;
   unsigned long long *h_stamps = nullptr;
   int *h_raster = nullptr;
+  float *h_state = nullptr;  // pinned staging of the neuron state (made at its first read)
   // host results since the last reset
   std::vector<int32_t> rt, rid, counts;
   std::vector<float> upd_ms, step_ms;
@@ -288,6 +289,7 @@ static void free_net(g4s_net *n) {
   cudaFreeHost(n->h_base);
   cudaFreeHost(n->h_stamps);
   cudaFreeHost(n->h_raster);
+  cudaFreeHost(n->h_state);
   if (n->ev0) cudaEventDestroy(n->ev0);
   if (n->ev1) cudaEventDestroy(n->ev1);
   if (n->ek0) cudaEventDestroy(n->ek0);
@@ -1785,32 +1787,71 @@ int g4s_net_step_times(g4s_net *n, float *upd, float *step, int64_t cap, int64_t
 int g4s_net_state(g4s_net *n, float *v, float *u, float *i_last, float *a, float *b, float *c, float *d,
                   int32_t *nospks) {
   if (!n) return set_error(G4S_ERR_INVALID, "null handle");
-  const size_t N = (size_t)n->v.n;
-  std::vector<float2> vu;
-  std::vector<float4> p;
-  std::vector<SpikeStat> ss;
-  try {
-    if (v || u) vu.resize(N);
-    if (a || b || c || d) p.resize(N);
-    if (nospks) ss.resize(N);
-  } catch (...) {
-    return set_error(G4S_ERR_NOMEM, "host staging");
+  void *const dst[8] = {v, u, i_last, a, b, c, d, nospks};
+  unsigned fields = 0;
+  for (int k = 0; k < 8; ++k)
+    if (dst[k]) fields |= 1u << k;
+  if (!fields) return G4S_OK;
+  // Blocks of kStateBlock neurons: the device packs a block field by field into the pinned
+  // staging buffer (two blocks, one being packed while the other is copied out).  Large
+  // networks are copied out by a thread per field: a fresh destination is mostly page faults
+  // (N=10^6: 2.5 ms of them on one thread).
+  const int64_t N = n->v.n;
+  const int nb = (int)((N + kStateBlock - 1) / kStateBlock);
+  const int64_t blk = std::min<int64_t>(N, kStateBlock);
+  if (!n->h_state) G4S_CUDA(cudaMallocHost((void **)&n->h_state, (size_t)blk * 32 * (nb > 1 ? 2 : 1)));
+  float *const half[2] = {n->h_state, n->h_state + (nb > 1 ? blk * 8 : 0)};
+  auto count = [&](int b) { return (int)std::min<int64_t>(kStateBlock, N - (int64_t)b * kStateBlock); };
+  auto copy = [&](int b, int slot, int k) {  // field k, the slot-th of those asked for, of block b
+    const size_t cnt = (size_t)count(b);
+    memcpy((char *)dst[k] + (size_t)b * kStateBlock * 4, half[b & 1] + (size_t)slot * cnt, cnt * 4);
+  };
+  std::atomic<int> ready{0}, out[2] = {{0}, {0}};  // blocks packed (-1: give up); fields copied out of each half
+  std::vector<std::thread> pool;
+  int nf = 0;
+  for (int k = 0; k < 8; ++k) nf += dst[k] ? 1 : 0;
+  bool threads = nb >= kStateThreadBlocks;
+  if (threads) {
+    try {
+      for (int k = 0, slot = 0; k < 8; ++k)
+        if (dst[k])
+          pool.emplace_back([&, k, slot = slot++] {
+            for (int b = 0; b < nb; ++b) {
+              int r;
+              while ((r = ready.load(std::memory_order_acquire)) <= b && r >= 0) std::this_thread::yield();
+              if (r < 0) return;
+              copy(b, slot, k);
+              out[b & 1].fetch_add(1, std::memory_order_release);
+            }
+          });
+    } catch (...) {  // (no thread to be had: this one copies)
+      ready.store(-1, std::memory_order_release);
+      for (auto &t : pool) t.join();
+      pool.clear();
+      threads = false;
+    }
   }
-  if (v || u) G4S_CUDA(cudaMemcpyAsync(vu.data(), n->v.vu, N * 8, cudaMemcpyDeviceToHost, n->stream));
-  if (a || b || c || d) G4S_CUDA(cudaMemcpyAsync(p.data(), n->v.abcd, N * 16, cudaMemcpyDeviceToHost, n->stream));
-  if (nospks) G4S_CUDA(cudaMemcpyAsync(ss.data(), n->v.sstat, N * sizeof(SpikeStat), cudaMemcpyDeviceToHost, n->stream));
-  if (i_last) G4S_CUDA(cudaMemcpyAsync(i_last, n->v.ilast, N * 4, cudaMemcpyDeviceToHost, n->stream));
-  G4S_CUDA(cudaStreamSynchronize(n->stream));
-  for (size_t i = 0; i < N; ++i) {
-    if (v) v[i] = vu[i].x;
-    if (u) u[i] = vu[i].y;
-    if (a) a[i] = p[i].x;
-    if (b) b[i] = p[i].y;
-    if (c) c[i] = p[i].z;
-    if (d) d[i] = p[i].w;
-    if (nospks) nospks[i] = ss[i].nospks;
+  cudaError_t e = launch_state_pack(n->v, 0, count(0), fields, half[0], n->stream);
+  for (int b = 0; b < nb && e == cudaSuccess; ++b) {
+    e = cudaStreamSynchronize(n->stream);  // block b is packed
+    if (e != cudaSuccess) break;
+    if (b + 1 < nb) {
+      // (the next block's half is free once block b - 1 has been copied out of it)
+      if (threads)
+        while (out[(b + 1) & 1].load(std::memory_order_acquire) < nf * ((b + 1) / 2)) std::this_thread::yield();
+      e = launch_state_pack(n->v, (int64_t)(b + 1) * kStateBlock, count(b + 1), fields, half[(b + 1) & 1], n->stream);
+      if (e != cudaSuccess) break;
+    }
+    if (threads) {
+      ready.store(b + 1, std::memory_order_release);
+    } else {
+      for (int k = 0, slot = 0; k < 8; ++k)
+        if (dst[k]) copy(b, slot++, k);
+    }
   }
-  return G4S_OK;
+  if (e != cudaSuccess) ready.store(-1, std::memory_order_release);
+  for (auto &t : pool) t.join();
+  return e == cudaSuccess ? G4S_OK : cuda_error(e, "reading the neuron state");
 }
 
 int g4s_net_currents(g4s_net *n, int64_t *acc) {

@@ -36,6 +36,9 @@ cudaError_t launch_deliver(const NetView &v, int lt, int alg, const DeliverShape
 cudaError_t launch_persistent(const NetView &v, int64_t t_abs0, int nsteps, bool last_chunk, GridSync *gs,
                               unsigned long long limit_ns, int group, int stall, cudaStream_t s);
 cudaError_t launch_stats(const NetView &v, double *out, cudaStream_t s);
+// fields of neurons [i0, i0 + cnt) as separate arrays: bits 0..7 of `fields` are v, u, I, a, b,
+// c, d and the spike count; `out` is device-accessible, cnt values per field asked for
+cudaError_t launch_state_pack(const NetView &v, int64_t i0, int cnt, unsigned fields, float *out, cudaStream_t s);
 int persistent_blocks();
 
 // SKL team kernel (g4s_team.cu).
@@ -52,6 +55,8 @@ constexpr int64_t kSoloSlice = 128;            // neurons per CTA of a network r
 constexpr int64_t kBatchSlice = 8192;          // neurons per CTA of a batched network (measured on the
                                                // 256-network ensemble: 510 ms against 534 at 4096 and
                                                // 824 at 16384; served requests 41.9/s, 40.1, 32.7)
+constexpr int kStateBlock = 65536;             // neurons of the state read back at a time
+constexpr int kStateThreadBlocks = 3;          // ... in this many blocks or more, a thread per field
 constexpr int kStepGraphSteps = 512;          // longest chunk of the host-driven schemes (one CUDA graph)
 constexpr int kStepGraphs = 4;                 // captured chunks kept per network
 constexpr int kMaxTeam = 176;                  // CTAs of one team (eight source ranks a warp, 22 such warps)
