@@ -2,8 +2,8 @@
 // reference's result files and its experiment sweep.
 //
 // A run is executed in chunks of at most `chunk_steps` steps; a chunk's spike ids go to a
-// device raster buffer sized so that every neuron could fire at every step of the chunk,
-// so it can never overflow.  After each chunk the per-step counts, raster offsets and
+// device raster buffer sized so that every neuron could fire at every step of the chunk
+// (or of the run, if that is shorter), so it can never overflow.  After each chunk the per-step counts, raster offsets and
 // globaltimer stamps come back to the host (and the raster, when it is recorded).
 #include <cuda_runtime.h>
 #include <sys/stat.h>
@@ -53,110 +53,58 @@ int cuda_error(cudaError_t e, const char *what) {
     if (e_ != cudaSuccess) return cuda_error(e_, #call); \
   } while (0)
 
+// Buffers of the launches of one handle, or of one thread's batches: what a round uploads
+// (descriptors, the networks' places in the pack, queue slots, control words: one copy) and
+// the pack that it brings back, each side one allocation.
 struct TeamLaunch {
-  TeamItem *d_items = nullptr, *h_items = nullptr;
-  int2 *d_slots = nullptr, *h_slots = nullptr;
-  int *d_ctl = nullptr, *h_ctl = nullptr;  // [0] slot count, [1] queue head
-  int *h_status = nullptr;                 // per item: status word, team error word
-  int64_t *d_off = nullptr, *h_off = nullptr;  // per item: its share of the pack (many networks)
-  unsigned char *d_pack = nullptr, *h_pack = nullptr;
-  size_t cap_pack = 0;
-  int cap_items = 0, cap_slots = 0;
+  unsigned char *d_mem = nullptr, *h_mem = nullptr;
+  size_t cap = 0;
+  // the round's parts, at the same offsets on both sides
+  size_t o_off = 0, o_slots = 0, o_ctl = 0, o_pack = 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
-  // the round as a CUDA graph, replayed while its shape (networks, teams, buffers) holds
-  cudaGraphExec_t exec = nullptr;
-  std::vector<uint64_t> sig;
   std::vector<int> order;  // networks of the round in flight (team_round_start .. finish)
-  // a round of many networks, launched directly: its networks and steps, read back by pack
-  bool direct = false;
   std::vector<g4s_net *> nets;
   std::vector<int> steps;
+  std::vector<size_t> at;  // per network: its share of the pack
   TeamLaunch() = default;
   TeamLaunch(const TeamLaunch &) = delete;
   TeamLaunch &operator=(const TeamLaunch &) = delete;
   ~TeamLaunch() { release(); }  // (a thread's own launch buffers go when the thread ends)
-  void drop_graph() {
-    if (exec) cudaGraphExecDestroy(exec);
-    exec = nullptr;
-    sig.clear();
-  }
   void release() {
-    drop_graph();
-    cudaFree(d_items);
-    cudaFree(d_slots);
-    cudaFree(d_ctl);
-    cudaFreeHost(h_items);
-    cudaFreeHost(h_slots);
-    cudaFreeHost(h_ctl);
-    cudaFreeHost(h_status);
-    cudaFree(d_off);
-    cudaFreeHost(h_off);
-    cudaFree(d_pack);
-    cudaFreeHost(h_pack);
+    cudaFree(d_mem);
+    cudaFreeHost(h_mem);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    d_items = h_items = nullptr;
-    d_slots = h_slots = nullptr;
-    d_ctl = h_ctl = nullptr;
-    h_status = nullptr;
-    d_off = h_off = nullptr;
-    d_pack = h_pack = nullptr;
-    cap_pack = 0;
-    cap_items = cap_slots = 0;
+    d_mem = h_mem = nullptr;
+    cap = 0;
     e0 = e1 = nullptr;
     order.clear();
-    direct = false;
   }
-  int reserve(int items, int slots) {
+  int reserve(int items, int slots, size_t pack) {
     if (!e0 && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
       return set_error(G4S_ERR_CUDA, "team launch events");
-    if (!d_ctl && (cudaMalloc((void **)&d_ctl, 16) != cudaSuccess || cudaMallocHost((void **)&h_ctl, 16) != cudaSuccess))
-      return set_error(G4S_ERR_NOMEM, "team launch control words");
-    if (items > cap_items) {
-      drop_graph();
-      cudaFree(d_items);
-      cudaFreeHost(h_items);
-      cudaFreeHost(h_status);
-      cudaFree(d_off);
-      cudaFreeHost(h_off);
-      d_items = h_items = nullptr;
-      h_status = nullptr;
-      d_off = h_off = nullptr;
-      cap_items = 0;  // (until the new buffers exist)
-      if (cudaMalloc((void **)&d_items, sizeof(TeamItem) * items) != cudaSuccess ||
-          cudaMallocHost((void **)&h_items, sizeof(TeamItem) * items) != cudaSuccess ||
-          cudaMallocHost((void **)&h_status, sizeof(int) * 2 * items) != cudaSuccess ||
-          cudaMalloc((void **)&d_off, sizeof(int64_t) * items) != cudaSuccess ||
-          cudaMallocHost((void **)&h_off, sizeof(int64_t) * items) != cudaSuccess)
-        return set_error(G4S_ERR_NOMEM, "team items");
-      cap_items = items;
-    }
-    if (slots > cap_slots) {
-      drop_graph();
-      cudaFree(d_slots);
-      cudaFreeHost(h_slots);
-      d_slots = h_slots = nullptr;
-      cap_slots = 0;
-      if (cudaMalloc((void **)&d_slots, sizeof(int2) * slots) != cudaSuccess ||
-          cudaMallocHost((void **)&h_slots, sizeof(int2) * slots) != cudaSuccess)
-        return set_error(G4S_ERR_NOMEM, "team slots");
-      cap_slots = slots;
-    }
+    o_off = sizeof(TeamItem) * (size_t)items;
+    o_slots = o_off + sizeof(int64_t) * (size_t)items;
+    o_ctl = o_slots + sizeof(int2) * (size_t)slots;
+    o_pack = (o_ctl + 16 + 15) / 16 * 16;
+    const size_t bytes = o_pack + pack;
+    if (bytes <= cap) return G4S_OK;
+    cudaFree(d_mem);
+    cudaFreeHost(h_mem);
+    d_mem = h_mem = nullptr;
+    const size_t want = std::max({bytes, 2 * cap, (size_t)1 << 16});
+    cap = 0;  // (until the new buffers exist)
+    if (cudaMalloc((void **)&d_mem, want) != cudaSuccess || cudaMallocHost((void **)&h_mem, want) != cudaSuccess)
+      return set_error(G4S_ERR_NOMEM, "team launch buffers");
+    cap = want;
     return G4S_OK;
   }
-  int reserve_pack(size_t bytes) {
-    if (bytes <= cap_pack) return G4S_OK;
-    bytes = std::max(bytes, 2 * cap_pack);
-    cudaFree(d_pack);
-    cudaFreeHost(h_pack);
-    d_pack = h_pack = nullptr;
-    cap_pack = 0;
-    if (cudaMalloc((void **)&d_pack, bytes) != cudaSuccess || cudaMallocHost((void **)&h_pack, bytes) != cudaSuccess)
-      return set_error(G4S_ERR_NOMEM, "team round read-back buffer");
-    cap_pack = bytes;
-    return G4S_OK;
-  }
+  TeamItem *items(unsigned char *m) const { return reinterpret_cast<TeamItem *>(m); }
+  int64_t *off(unsigned char *m) const { return reinterpret_cast<int64_t *>(m + o_off); }
+  int2 *slots(unsigned char *m) const { return reinterpret_cast<int2 *>(m + o_slots); }
+  int *ctl(unsigned char *m) const { return reinterpret_cast<int *>(m + o_ctl); }  // slot count, queue head
 };
+static_assert(sizeof(TeamItem) % 8 == 0, "the upload's parts follow one another");
 
 // A scheme and, for SKL, a team size chosen by the autotuner (0 = the default team).
 struct TuneChoice {
@@ -164,6 +112,28 @@ struct TuneChoice {
   int team = 0;
   int mode = kDeliverAuto;
   int nt = 0;  // threads per CTA of the team kernel (0: chosen from the step size)
+};
+
+// Spike ids of a handle's recorded chunks: a growing array that is not cleared when it grows
+// (every id is written once, by the thread that files its step).
+struct IdStore {
+  int32_t *p = nullptr;
+  size_t n = 0, cap = 0;
+  IdStore() = default;
+  IdStore(const IdStore &) = delete;
+  IdStore &operator=(const IdStore &) = delete;
+  ~IdStore() { free(p); }
+  int32_t *extend(size_t more) {  // (null: no memory; the ids so far stay)
+    if (n + more > cap) {
+      const size_t want = std::max(n + more, cap + cap / 2);
+      void *q = realloc(p, want * sizeof(int32_t));
+      if (!q) return nullptr;
+      p = static_cast<int32_t *>(q);
+      cap = want;
+    }
+    n += more;
+    return p + (n - more);
+  }
 };
 
 // ---------------------------------------------------------------------------------------
@@ -191,17 +161,29 @@ struct g4s_net {
   std::vector<StepGraph> step_graphs;
   int64_t t_abs = 0;
   uint32_t tag_next = 0;  // record tags of the team kernel: never repeated for this handle's lists
-  uint64_t serial = 0;    // creation number, unique in the process (keys the captured rounds)
   unsigned long long barrier_ns = 2000000000ull;
   size_t device_bytes = 0;
-  // pinned staging of one chunk
-  int *h_counts = nullptr;
-  long long *h_base = nullptr;
-  unsigned long long *h_stamps = nullptr;
-  int *h_raster = nullptr;
-  float *h_state = nullptr;  // pinned staging of the neuron state (made at its first read)
-  // host results since the last reset
-  std::vector<int32_t> rt, rid, counts;
+  // per-step arrays of the last finished chunk
+  std::vector<int> c_counts;
+  std::vector<long long> c_base;
+  std::vector<unsigned long long> c_stamps;
+  // pinned staging, sized by need: a chunk's raster on its way to the host record, or blocks
+  // of the neuron state (never both at once)
+  unsigned char *h_stage = nullptr;
+  size_t stage_bytes = 0;
+  int *h_raster = nullptr;  // the staged raster (in h_stage)
+  void *arena = nullptr;    // device memory of the neuron state and the per-step arrays
+  int64_t raster_full = 0;  // raster ids of a full chunk (the buffer holds v.raster_cap, by need)
+  // host results since the last reset: the recorded ids, and for each recorded chunk its
+  // first step, its steps' place in `counts` and its ids' place in `rid`
+  std::vector<int32_t> counts;
+  IdStore rid;
+  struct Recorded {
+    int64_t t0;
+    size_t c0, off;
+    int cs;
+  };
+  std::vector<Recorded> recorded;
   std::vector<float> upd_ms, step_ms;
   int64_t total_spikes = 0;
   double last_ms = 0, last_wall_ms = 0;
@@ -261,35 +243,19 @@ static void free_net(g4s_net *n) {
     raster_close(n->rstream);
     n->rstream = nullptr;
   }
-  n->launch.release();  // its captured round refers to the buffers below
-  for (auto &gr : n->step_graphs)  // (and so do the captured chunks)
+  n->launch.release();
+  for (auto &gr : n->step_graphs)  // (the captured chunks refer to the buffers below)
     if (gr.exec) cudaGraphExecDestroy(gr.exec);
   n->step_graphs.clear();
-  net_free(n, n->d_t0);
   cudaFreeHost(n->h_t0);
   net_free(n, const_cast<unsigned long long *>(v.pair));
-  net_free(n, v.vu);
-  net_free(n, v.abcd);
-  net_free(n, v.rpar);
-  net_free(n, v.acc);
-  net_free(n, v.ilast);
-  net_free(n, v.sstat);
+  net_free(n, n->arena);
   net_free(n, const_cast<int *>(v.idx));
   net_free(n, const_cast<float *>(v.w));
   net_free(n, v.raster);
-  net_free(n, v.counts);
-  net_free(n, v.base);
-  net_free(n, v.stamps);
-  net_free(n, v.status);
-  net_free(n, n->gs);
-  net_free(n, n->d_stats);
   net_free(n, n->seg);
   net_free(n, n->list);
-  cudaFreeHost(n->h_counts);
-  cudaFreeHost(n->h_base);
-  cudaFreeHost(n->h_stamps);
-  cudaFreeHost(n->h_raster);
-  cudaFreeHost(n->h_state);
+  cudaFreeHost(n->h_stage);
   if (n->ev0) cudaEventDestroy(n->ev0);
   if (n->ev1) cudaEventDestroy(n->ev1);
   if (n->ek0) cudaEventDestroy(n->ek0);
@@ -340,8 +306,6 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
   g4s_net *n = new (std::nothrow) g4s_net;
   if (!n) return set_error(G4S_ERR_NOMEM, "host allocation");
   n->pool = pool;
-  static std::atomic<uint64_t> next_serial{1};
-  n->serial = next_serial++;
   n->desc = *d;
   NetView &v = n->v;
   v.n = d->n;
@@ -363,7 +327,7 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
   if (cs > 100000) cs = 100000;
   n->chunk_legacy = cs;
   n->chunk_steps = d->record_raster ? cs : 16384;
-  v.raster_cap = cs * (int64_t)N;
+  n->raster_full = cs * (int64_t)N;
   cs = std::max<int64_t>(cs, n->chunk_steps);
   size_t free_b = 0, total_b = 0;
   cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
@@ -383,42 +347,59 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
       return cuda_error(e, "stream");
     }
   }
-  const size_t need = N * S * 8 + N * (8 + 16 + 4 + 8 + 4 + 32) + (size_t)v.raster_cap * 4 + (size_t)cs * 32;
+  const size_t need = N * S * 8 + N * (8 + 16 + 4 + 8 + 4 + 32) + (size_t)n->raster_full * 4 + (size_t)cs * 32;
   if (need + ((size_t)256 << 20) > free_b) {
     free_net(n);
     return set_error(G4S_ERR_NOMEM, "network needs " + std::to_string(need) + " bytes of device memory, " +
                                         std::to_string(free_b) + " free");
   }
-  if ((rc = dalloc(n, &v.vu, N, "v,u")) || (rc = dalloc(n, &v.abcd, N, "a,b,c,d")) ||
-      (rc = dalloc(n, &v.rpar, N, "parameter r")) ||
-      (rc = dalloc(n, &v.acc, N, "currents")) || (rc = dalloc(n, &v.ilast, N, "input current")) ||
-      (rc = dalloc(n, &v.sstat, N, "spike statistics")) ||
-      (rc = dalloc(n, const_cast<int **>(&v.idx), N * S, "targets")) ||
-      (rc = dalloc(n, const_cast<float **>(&v.w), N * S, "weights")) ||
-      (rc = dalloc(n, &v.raster, (size_t)v.raster_cap, "raster")) ||
-      (rc = dalloc(n, &v.counts, (size_t)cs, "counts")) || (rc = dalloc(n, &v.base, (size_t)cs, "offsets")) ||
-      (rc = dalloc(n, &v.stamps, (size_t)cs * 2 + 2, "stamps")) || (rc = dalloc(n, &v.status, 1, "status")) ||
-      (rc = dalloc(n, &n->gs, 1 + 2 * (size_t)kMaxTeam * kRecLines, "barrier and spike records")) ||
-      (rc = dalloc(n, &n->d_stats, 2, "stats")) || (rc = dalloc(n, &n->d_t0, 1, "chunk start"))) {
+  // The neuron state and the per-step arrays in one allocation (a cudaMalloc and its cudaFree
+  // take 0.14 ms, a small network has little else to pay for), each on a 256-byte boundary.
+  size_t bytes = 0;
+  auto place = [&](size_t b) {
+    const size_t at = bytes;
+    bytes = (bytes + b + 255) / 256 * 256;
+    return at;
+  };
+  const size_t o_vu = place(N * sizeof(float2)), o_abcd = place(N * sizeof(float4)), o_rpar = place(N * sizeof(float)),
+               o_acc = place(N * sizeof(long long)), o_ilast = place(N * sizeof(float)),
+               o_sstat = place(N * sizeof(SpikeStat)), o_counts = place((size_t)cs * sizeof(int)),
+               o_base = place((size_t)cs * sizeof(long long)),
+               o_stamps = place(((size_t)cs * 2 + 2) * sizeof(unsigned long long)), o_status = place(sizeof(int)),
+               o_gs = place(sizeof(GridSync) * (1 + 2 * (size_t)kMaxTeam * kRecLines)), o_stats = place(2 * sizeof(double)),
+               o_t0 = place(sizeof(long long));
+  unsigned char *mem = nullptr;
+  if ((rc = dalloc(n, &mem, bytes, "neuron state and per-step arrays"))) {
     free_net(n);
     return rc;
   }
+  n->arena = mem;
+  v.vu = reinterpret_cast<float2 *>(mem + o_vu);
+  v.abcd = reinterpret_cast<float4 *>(mem + o_abcd);
+  v.rpar = reinterpret_cast<float *>(mem + o_rpar);
+  v.acc = reinterpret_cast<long long *>(mem + o_acc);
+  v.ilast = reinterpret_cast<float *>(mem + o_ilast);
+  v.sstat = reinterpret_cast<SpikeStat *>(mem + o_sstat);
+  v.counts = reinterpret_cast<int *>(mem + o_counts);
+  v.base = reinterpret_cast<long long *>(mem + o_base);
+  v.stamps = reinterpret_cast<unsigned long long *>(mem + o_stamps);
+  v.status = reinterpret_cast<int *>(mem + o_status);
+  n->gs = reinterpret_cast<GridSync *>(mem + o_gs);
+  n->d_stats = reinterpret_cast<double *>(mem + o_stats);
+  n->d_t0 = reinterpret_cast<long long *>(mem + o_t0);
+  if ((rc = dalloc(n, const_cast<int **>(&v.idx), N * S, "targets")) ||
+      (rc = dalloc(n, const_cast<float **>(&v.w), N * S, "weights")) ||
+      // (a pool's network gets its whole raster now: a run may use another network's stream)
+      (pool && (rc = dalloc(n, &v.raster, (size_t)n->raster_full, "raster")))) {
+    free_net(n);
+    return rc;
+  }
+  v.raster_cap = pool ? n->raster_full : 0;
   if ((!n->stream && (e = cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking)) != cudaSuccess) ||
       (e = cudaEventCreate(&n->ev0)) != cudaSuccess || (e = cudaEventCreate(&n->ev1)) != cudaSuccess ||
-      (e = cudaEventCreate(&n->ek0)) != cudaSuccess || (e = cudaEventCreate(&n->ek1)) != cudaSuccess ||
-      (e = cudaMallocHost((void **)&n->h_counts, (size_t)cs * 4)) != cudaSuccess ||
-      (e = cudaMallocHost((void **)&n->h_base, (size_t)cs * 8)) != cudaSuccess ||
-      (e = cudaMallocHost((void **)&n->h_stamps, ((size_t)cs * 2 + 2) * 8)) != cudaSuccess ||
-      (e = cudaMallocHost((void **)&n->h_t0, sizeof(long long))) != cudaSuccess) {
+      (e = cudaEventCreate(&n->ek0)) != cudaSuccess || (e = cudaEventCreate(&n->ek1)) != cudaSuccess) {
     free_net(n);
-    return cuda_error(e, "stream/event/pinned allocation");
-  }
-  if (d->record_raster) {
-    e = cudaMallocHost((void **)&n->h_raster, (size_t)v.raster_cap * 4);
-    if (e != cudaSuccess) {
-      free_net(n);
-      return cuda_error(e, "pinned raster staging");
-    }
+    return cuda_error(e, "stream/event");
   }
   if ((e = cudaMemsetAsync(v.status, 0, sizeof(int), n->stream)) != cudaSuccess ||
       (e = cudaMemsetAsync(n->gs, 0, sizeof(GridSync), n->stream)) != cudaSuccess) {
@@ -462,8 +443,8 @@ static int reset_net(g4s_net *n) {
   G4S_CUDA(launch_init(v, n->stream));
   G4S_CUDA(cudaStreamSynchronize(n->stream));
   n->t_abs = 0;
-  n->rt.clear();
-  n->rid.clear();
+  n->rid.n = 0;
+  n->recorded.clear();
   n->counts.clear();
   n->upd_ms.clear();
   n->step_ms.clear();
@@ -781,90 +762,118 @@ static int finish_tables(g4s_net *n, bool may_be_sorted) {
 // networks that record it, then the host-side bookkeeping.
 static int chunk_copy_meta(g4s_net *n, int cs, cudaStream_t s) {
   NetView &v = n->v;
-  G4S_CUDA(cudaMemcpyAsync(n->h_counts, v.counts, (size_t)cs * 4, cudaMemcpyDeviceToHost, s));
-  G4S_CUDA(cudaMemcpyAsync(n->h_base, v.base, (size_t)cs * 8, cudaMemcpyDeviceToHost, s));
-  G4S_CUDA(cudaMemcpyAsync(n->h_stamps, v.stamps, (size_t)cs * 16, cudaMemcpyDeviceToHost, s));
+  n->c_counts.resize((size_t)cs);
+  n->c_base.resize((size_t)cs);
+  n->c_stamps.resize((size_t)cs * 2);
+  G4S_CUDA(cudaMemcpyAsync(n->c_counts.data(), v.counts, (size_t)cs * 4, cudaMemcpyDeviceToHost, s));
+  G4S_CUDA(cudaMemcpyAsync(n->c_base.data(), v.base, (size_t)cs * 8, cudaMemcpyDeviceToHost, s));
+  G4S_CUDA(cudaMemcpyAsync(n->c_stamps.data(), v.stamps, (size_t)cs * 16, cudaMemcpyDeviceToHost, s));
   return G4S_OK;
 }
 
-static int64_t chunk_total(const g4s_net *n, int cs) { return (int64_t)n->h_base[cs - 1] + n->h_counts[cs - 1]; }
+static int64_t chunk_total(const g4s_net *n, int cs) { return (int64_t)n->c_base[cs - 1] + n->c_counts[cs - 1]; }
+
+// At least `bytes` of pinned staging (its contents are not kept).
+static int need_stage(g4s_net *n, size_t bytes) {
+  if (bytes <= n->stage_bytes) return G4S_OK;
+  bytes = std::max(bytes, (size_t)1 << 18);
+  cudaFreeHost(n->h_stage);
+  n->h_stage = nullptr;
+  n->stage_bytes = 0;
+  G4S_CUDA(cudaMallocHost((void **)&n->h_stage, bytes));
+  n->stage_bytes = bytes;
+  return G4S_OK;
+}
+
+// The raster buffer for chunks of up to `steps` steps (every neuron firing at every step).  A
+// full chunk's buffer is up to 1 GiB, of which a short run uses little: allocated by need.
+static int need_raster(g4s_net *n, int64_t steps) {
+  const int64_t want = std::min(n->raster_full, std::max<int64_t>(1, steps) * n->v.n);
+  if (want <= n->v.raster_cap) return G4S_OK;
+  const int64_t ids = std::min(n->raster_full, std::max(want, (int64_t)1 << 20));
+  for (auto &gr : n->step_graphs)  // (captured chunks hold the buffer's address)
+    if (gr.exec) cudaGraphExecDestroy(gr.exec);
+  n->step_graphs.clear();
+  net_free(n, n->v.raster);
+  n->v.raster = nullptr;
+  n->device_bytes -= (size_t)n->v.raster_cap * 4;
+  n->v.raster_cap = 0;
+  const cudaError_t e = net_malloc(n, (void **)&n->v.raster, (size_t)ids * 4);
+  if (e != cudaSuccess) {
+    n->v.raster = nullptr;
+    return cuda_error(e, "raster buffer");
+  }
+  n->v.raster_cap = ids;
+  n->device_bytes += (size_t)ids * 4;
+  return G4S_OK;
+}
 
 static int chunk_copy_raster(g4s_net *n, int cs, cudaStream_t s) {
   const int64_t total = chunk_total(n, cs);
-  if (n->desc.record_raster && total > 0)
+  if (n->desc.record_raster && total > 0) {
+    const int rc = need_stage(n, (size_t)total * 4);
+    if (rc) return rc;
+    n->h_raster = reinterpret_cast<int *>(n->h_stage);
     G4S_CUDA(cudaMemcpyAsync(n->h_raster, n->v.raster, (size_t)total * 4, cudaMemcpyDeviceToHost, s));
+  }
   return G4S_OK;
 }
 
-// One step's ids in ascending order.  The team kernel writes them rank by rank (ranks own
-// ascending ranges), each rank's few ids in arrival order, so an insertion sort finishes in
-// a few shifts per id; an order far from sorted (a one-CTA team's ids) goes to std::sort
-// once the shifts exceed a small multiple of the count.
+// One step's ids in ascending order: the team kernel writes them in order (but for a rank's
+// bursts and with the host-driven schemes, whose blocks append as they come).
 static void sort_step_ids(int *b, int cnt) {
-  int64_t budget = 4 * (int64_t)cnt + 64;
-  for (int i = 1; i < cnt; ++i) {
-    const int x = b[i];
-    int j = i;
-    while (j > 0 && b[j - 1] > x) {
-      b[j] = b[j - 1];
-      --j;
-      if (--budget < 0) {
-        b[j] = x;
-        std::sort(b, b + cnt);
-        return;
-      }
-    }
-    b[j] = x;
-  }
+  int back = 0;
+  for (int i = 1; i < cnt; ++i) back |= b[i - 1] > b[i];
+  if (back) std::sort(b, b + cnt);
 }
 
-// The host side of a finished chunk that began at step t0, from its per-step counts, raster
-// offsets and stamps and the raster in the pinned staging buffer: the sorted raster (kept
-// or streamed to its file), the counts and the per-step times.
-static void chunk_finish_from(g4s_net *n, int cs, const int *counts, const long long *base,
-                              const unsigned long long *stamps, int64_t t0, int64_t *spikes) {
+// Steps [0, cs) of a chunk in runs of about equal ids, f(l0, l1) on each, on a host thread per
+// 2^18 ids (a thread's start costs about what it saves on fewer; here, if none is to be had).
+template <class F>
+static void for_step_runs(int cs, const long long *base, int64_t total, F f) {
+  const int64_t hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+  const int parts = (int)std::max<int64_t>(1, std::min({hw, (int64_t)cs, total >> 18}));
+  std::vector<std::thread> pool;
+  int l0 = 0;
+  for (int p = 0; p < parts; ++p) {
+    const int64_t goal = total * (p + 1) / parts;  // the steps up to the p+1-th share of the ids
+    int l1 = l0;
+    while (l1 < cs && (p == parts - 1 || (int64_t)base[l1] < goal)) ++l1;
+    if (l1 > l0) {
+      bool here = p == parts - 1;
+      if (!here) try {
+          pool.emplace_back(f, l0, l1);
+        } catch (...) {
+          here = true;
+        }
+      if (here) f(l0, l1);
+    }
+    l0 = l1;
+  }
+  for (auto &th : pool) th.join();
+}
+
+// The host side of a finished chunk that began at step t0, from its per-step arrays and the
+// raster in the pinned staging buffer: the raster in order (kept or streamed to its file), the
+// counts and the per-step times.
+static int chunk_finish_from(g4s_net *n, int cs, int64_t t0, int64_t *spikes) {
+  const int *counts = n->c_counts.data();
+  const long long *base = n->c_base.data();
+  const unsigned long long *stamps = n->c_stamps.data();
   const int64_t total = (int64_t)base[cs - 1] + counts[cs - 1];
   if (n->desc.record_raster && n->rstream) {
     for (int lt = 0; lt < cs; ++lt) sort_step_ids(n->h_raster + base[lt], counts[lt]);
     raster_push(n->rstream, counts, cs, n->h_raster, total);
   } else if (n->desc.record_raster && total > 0) {
-    const size_t off = n->rt.size();
-    n->rt.resize(off + (size_t)total);
-    n->rid.resize(off + (size_t)total);
-    auto steps = [&](int l0, int l1) {
-      for (int lt = l0; lt < l1; ++lt) {
-        int *b = n->h_raster + base[lt];
-        sort_step_ids(b, counts[lt]);
-        const int32_t t = (int32_t)(t0 + lt);
-        int32_t *rt = n->rt.data() + off + (size_t)base[lt], *rid = n->rid.data() + off + (size_t)base[lt];
-        for (int q = 0; q < counts[lt]; ++q) {
-          rt[q] = t;
-          rid[q] = b[q];
-        }
-      }
-    };
-    // a large chunk on several host threads, each a run of whole steps (steps are independent)
-    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    const int parts = total >= ((int64_t)1 << 20) ? (int)std::min<int64_t>(hw, cs) : 1;
-    if (parts <= 1) {
-      steps(0, cs);
-    } else {
-      std::vector<std::thread> pool;
-      int l0 = 0;
-      for (int p = 0; p < parts; ++p) {
-        // the steps up to the p+1-th share of the chunk's ids
-        const int64_t goal = total * (p + 1) / parts;
-        int l1 = l0;
-        while (l1 < cs && (p == parts - 1 || (int64_t)base[l1] < goal)) ++l1;
-        if (p == parts - 1) {
-          steps(l0, l1);
-        } else if (l1 > l0) {
-          pool.emplace_back(steps, l0, l1);
-        }
-        l0 = l1;
-      }
-      for (auto &th : pool) th.join();
-    }
+    const size_t off = n->rid.n;
+    int32_t *ids = n->rid.extend((size_t)total);
+    if (!ids) return set_error(G4S_ERR_NOMEM, "host raster");
+    n->recorded.push_back({t0, n->counts.size(), off, cs});
+    for_step_runs(cs, base, total, [=](int l0, int l1) {
+      for (int lt = l0; lt < l1; ++lt) sort_step_ids(n->h_raster + base[lt], counts[lt]);
+      const size_t i0 = (size_t)base[l0], i1 = (size_t)base[l1 - 1] + (size_t)counts[l1 - 1];
+      memcpy(ids + i0, n->h_raster + i0, (i1 - i0) * 4);
+    });
   }
   for (int lt = 0; lt < cs; ++lt) {
     n->counts.push_back(counts[lt]);
@@ -874,24 +883,45 @@ static void chunk_finish_from(g4s_net *n, int cs, const int *counts, const long 
     n->step_ms.push_back(s2 > s0 ? (float)((s2 - s0) * 1e-6) : 0.0f);
   }
   *spikes = total;
+  return G4S_OK;
 }
 
-static void chunk_finish(g4s_net *n, int cs, int64_t *spikes) {
-  chunk_finish_from(n, cs, n->h_counts, n->h_base, n->h_stamps, n->t_abs, spikes);
+static int chunk_finish(g4s_net *n, int cs, int64_t *spikes) {
+  const int rc = chunk_finish_from(n, cs, n->t_abs, spikes);
   n->t_abs += cs;
+  return rc;
 }
 
 // Results of one chunk of `cs` steps of one network: per-step counts, raster offsets and
-// stamps, and the raster itself when recorded; each step's ids sorted (the device order
-// is by CTA).
+// stamps, and the raster itself when recorded, each step's ids in order.
 static int absorb_chunk(g4s_net *n, int cs, int64_t *spikes) {
   int rc = chunk_copy_meta(n, cs, n->stream);
   if (rc) return rc;
   G4S_CUDA(cudaStreamSynchronize(n->stream));
   if ((rc = chunk_copy_raster(n, cs, n->stream))) return rc;
   G4S_CUDA(cudaStreamSynchronize(n->stream));
-  chunk_finish(n, cs, spikes);
-  return G4S_OK;
+  return chunk_finish(n, cs, spikes);
+}
+
+// The recorded raster's first m spikes: the step of each (t) and its id.  Large rasters on
+// several host threads (a fresh destination is mostly page faults).
+static void raster_copy_out(const g4s_net *n, int32_t *t, int32_t *id, int64_t m) {
+  for (const auto &r : n->recorded) {
+    if ((int64_t)r.off >= m) break;
+    std::vector<long long> base((size_t)r.cs);
+    int64_t total = 0;
+    for (int lt = 0; lt < r.cs; ++lt) {
+      base[(size_t)lt] = total;
+      total += n->counts[r.c0 + (size_t)lt];
+    }
+    for_step_runs(r.cs, base.data(), total, [&](int l0, int l1) {
+      for (int lt = l0; lt < l1; ++lt) {
+        const int64_t q0 = (int64_t)r.off + base[(size_t)lt], q1 = std::min(m, q0 + n->counts[r.c0 + (size_t)lt]);
+        for (int64_t q = q0; q < q1; ++q) t[q] = (int32_t)(r.t0 + lt);
+        if (q1 > q0) memcpy(id + q0, n->rid.p + q0, (size_t)(q1 - q0) * 4);
+      }
+    });
+  }
 }
 
 // Delivery mapping of a network's multi-CTA team: the one set or tuned, else eight-lane
@@ -908,8 +938,8 @@ static int deliver_mode_of(const g4s_net *n) {
 // ---------------------------------------------------------------------------------------
 // team_round_start enqueues the round on stream s and returns; team_round_finish waits for
 // it and checks every network's status words.  Between the two, the host may work on the
-// previous round's results, but must not touch the pinned per-step buffers (the round's
-// graph writes them at its end) nor the networks' device arrays.
+// previous round's results, but must not touch the launch buffers (the round writes its pack
+// at its end) nor the networks' device arrays.
 static int team_round_start(g4s_net *const *nets, const int *steps, const bool *last, int count, TeamLaunch &L,
                             cudaStream_t s, unsigned long long limit_ns, int stall) {
   std::vector<int> order;
@@ -930,7 +960,13 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
     if (x->team_p != y->team_p) return x->team_p > y->team_p;
     return (double)x->v.n * steps[a] * x->v.nsyn > (double)y->v.n * steps[b] * y->v.nsyn;
   });
-  int rc = L.reserve(count, nslots);
+  size_t pack = 0;
+  L.at.assign((size_t)count, 0);
+  for (int i : order) {
+    L.at[(size_t)i] = pack;
+    pack += round_pack_bytes(steps[i]);
+  }
+  int rc = L.reserve(count, nslots, pack);
   if (rc) return rc;
   bool pair = true;  // every network of the round has its packed rows
   for (int i : order) pair = pair && nets[i]->v.pair != nullptr;
@@ -949,11 +985,11 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
   G4S_CUDA(team_max_blocks(smem, &gmax, nt));  // also raises the kernel's shared-memory ceiling
   if (gmax < maxteam) return set_error(G4S_ERR_CUDA, "team larger than the co-resident grid");
   const int grid = std::min(nslots, gmax);
-  // this round's descriptors, in pinned host memory the graph copies from
+  // this round's descriptors, in pinned host memory
   int k = 0;
   for (int i : order) {
     g4s_net *n = nets[i];
-    TeamItem &it = L.h_items[i];
+    TeamItem &it = L.items(L.h_mem)[i];
     it.v = n->v;
     if (!n->desc.record_raster) it.v.raster_cap = 0;  // (its raster is never read)
     it.seg = n->seg;
@@ -971,100 +1007,28 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
     }
     it.tag0 = n->tag_next;
     n->tag_next += (uint32_t)steps[i];
-    for (int r = 0; r < n->team_p; ++r) L.h_slots[k++] = make_int2(i, r);
+    for (int r = 0; r < n->team_p; ++r) L.slots(L.h_mem)[k++] = make_int2(i, r);
+    L.off(L.h_mem)[i] = (int64_t)L.at[(size_t)i];
   }
   for (int i = 0; i < count; ++i)
-    if (steps[i] <= 0) L.h_items[i].steps = 0;
-  L.h_ctl[0] = nslots;
-  L.h_ctl[1] = 0;
-  L.direct = count > 1;
-  if (L.direct) {
-    // Many networks: the set changes from round to round (a server admits and retires
-    // requests), so a graph would be captured and instantiated for almost every round, at a
-    // cost that grows with the networks.  Launched directly instead, in a fixed number of
-    // calls: descriptors up, one kernel clearing every network's per-launch words, the team
-    // kernel between two events, one kernel packing every network's results, one copy down.
-    size_t total = 0;
-    for (int i : order) {
-      L.h_off[i] = (int64_t)total;
-      total += round_pack_bytes(steps[i]);
-    }
-    if ((rc = L.reserve_pack(total))) return rc;
-    L.nets.assign(nets, nets + count);
-    L.steps.assign(steps, steps + count);
-    G4S_CUDA(cudaMemcpyAsync(L.d_items, L.h_items, sizeof(TeamItem) * count, cudaMemcpyHostToDevice, s));
-    G4S_CUDA(cudaMemcpyAsync(L.d_slots, L.h_slots, sizeof(int2) * nslots, cudaMemcpyHostToDevice, s));
-    G4S_CUDA(cudaMemcpyAsync(L.d_ctl, L.h_ctl, 8, cudaMemcpyHostToDevice, s));
-    G4S_CUDA(cudaMemcpyAsync(L.d_off, L.h_off, sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
-    G4S_CUDA(launch_round_clear(L.d_items, count, s));
-    G4S_CUDA(cudaEventRecord(L.e0, s));
-    G4S_CUDA(launch_team(L.d_items, L.d_slots, L.d_ctl, L.d_ctl + 1, grid, smem, limit_ns, stall, s, pair, mode, solo, nt));
-    G4S_CUDA(cudaEventRecord(L.e1, s));
-    G4S_CUDA(launch_round_gather(L.d_items, L.d_off, count, L.d_pack, s));
-    G4S_CUDA(cudaMemcpyAsync(L.h_pack, L.d_pack, total, cudaMemcpyDeviceToHost, s));
-    L.order = order;
-    return G4S_OK;
-  }
-  // The round's graph: clear the networks' per-chunk arrays, error words and spike records,
-  // upload the descriptors, the persistent launch between two timing events, and copy
-  // back each network's per-step counts, offsets and stamps and its status words.  Its
-  // shape depends only on which networks run, their teams and chunk lengths, and the
-  // launch parameters; the descriptors' contents are read from pinned memory at replay.
-  // A graph must not outlive the buffers it copies to and from: a network freed and another
-  // created in its place (often at the same device and pinned host addresses) gets a new
-  // graph, so the key holds each network's creation number as well as its addresses.
-  auto u = [](const void *p) { return (uint64_t)(uintptr_t)p; };
-  std::vector<uint64_t> sig = {(uint64_t)count, (uint64_t)nslots, (uint64_t)grid, (uint64_t)smem, limit_ns,
-                               (uint64_t)stall, (uint64_t)pair, (uint64_t)mode, (uint64_t)nt, u(L.d_items), u(L.d_slots), u(L.d_ctl), u(L.h_items),
-                               u(L.h_slots), u(L.h_ctl), u(L.h_status), u(L.e0), u(L.e1)};
-  for (int i : order) {
-    const g4s_net *n = nets[i];
-    for (uint64_t x : {(uint64_t)i, n->serial, (uint64_t)n->team_p, (uint64_t)n->chunk_steps, u(n->v.counts), u(n->v.stamps),
-                       u(n->v.status), u(n->gs), u(n->v.base), u(n->h_counts), u(n->h_base), u(n->h_stamps)})
-      sig.push_back(x);
-  }
-  if (!L.exec || sig != L.sig) {
-    L.drop_graph();
-    G4S_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = cudaSuccess;
-    for (int i : order) {
-      const g4s_net *n = nets[i];
-      const size_t cs = (size_t)n->chunk_steps;
-      if (e == cudaSuccess) e = cudaMemsetAsync(n->v.counts, 0, cs * sizeof(int), s);
-      if (e == cudaSuccess) e = cudaMemsetAsync(n->v.stamps, 0, (cs * 2 + 2) * 8, s);
-      if (e == cudaSuccess) e = cudaMemsetAsync(n->v.status, 0, sizeof(int), s);
-      // error word and the team's spike records (two sets of kRecLines 128-byte lines per rank)
-      if (e == cudaSuccess) e = cudaMemsetAsync(n->gs, 0, sizeof(GridSync) * (1 + 2 * (size_t)n->team_p * kRecLines), s);
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(L.d_items, L.h_items, sizeof(TeamItem) * count, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(L.d_slots, L.h_slots, sizeof(int2) * nslots, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(L.d_ctl, L.h_ctl, 8, cudaMemcpyHostToDevice, s);
-    // (external records: the graph records the events at every replay)
-    if (e == cudaSuccess) e = cudaEventRecordWithFlags(L.e0, s, cudaEventRecordExternal);
-    if (e == cudaSuccess) e = launch_team(L.d_items, L.d_slots, L.d_ctl, L.d_ctl + 1, grid, smem, limit_ns, stall, s, pair, mode, solo, nt);
-    if (e == cudaSuccess) e = cudaEventRecordWithFlags(L.e1, s, cudaEventRecordExternal);
-    for (int i : order) {
-      const g4s_net *n = nets[i];
-      const size_t cs = (size_t)n->chunk_steps;
-      if (e == cudaSuccess) e = cudaMemcpyAsync(n->h_counts, n->v.counts, cs * 4, cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(n->h_base, n->v.base, cs * 8, cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(n->h_stamps, n->v.stamps, cs * 16, cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(L.h_status + 2 * i, n->v.status, sizeof(int), cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(L.h_status + 2 * i + 1, &n->gs->error, sizeof(int), cudaMemcpyDeviceToHost, s);
-    }
-    cudaGraph_t g = nullptr;
-    const cudaError_t e_end = cudaStreamEndCapture(s, &g);
-    if (e == cudaSuccess) e = e_end;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&L.exec, g, 0);
-    if (g) cudaGraphDestroy(g);
-    if (e != cudaSuccess) {
-      L.exec = nullptr;
-      return cuda_error(e, "capturing the team round as a CUDA graph");
-    }
-    L.sig = sig;
-  }
-  G4S_CUDA(cudaGraphLaunch(L.exec, s));
+    if (steps[i] <= 0) L.items(L.h_mem)[i].steps = 0;
+  L.ctl(L.h_mem)[0] = nslots;
+  L.ctl(L.h_mem)[1] = 0;
+  L.nets.assign(nets, nets + count);
+  L.steps.assign(steps, steps + count);
+  // One copy up, one kernel clearing every network's words of the launch, the team kernel
+  // between two events, one kernel packing every network's results, one copy down: sized by
+  // the round's own steps and networks.  (As a CUDA graph, a lone network's round cleared and
+  // copied arrays of its longest chunk: 0.18 ms beside the kernel for 2000 steps of N=2,500,
+  // 0.04 so, and a new network had its graph to build first.)
+  G4S_CUDA(cudaMemcpyAsync(L.d_mem, L.h_mem, L.o_pack, cudaMemcpyHostToDevice, s));
+  G4S_CUDA(launch_round_clear(L.items(L.d_mem), count, s));
+  G4S_CUDA(cudaEventRecord(L.e0, s));
+  G4S_CUDA(launch_team(L.items(L.d_mem), L.slots(L.d_mem), L.ctl(L.d_mem), L.ctl(L.d_mem) + 1, grid, smem, limit_ns,
+                       stall, s, pair, mode, solo, nt));
+  G4S_CUDA(cudaEventRecord(L.e1, s));
+  G4S_CUDA(launch_round_gather(L.items(L.d_mem), L.off(L.d_mem), count, L.d_mem + L.o_pack, s));
+  G4S_CUDA(cudaMemcpyAsync(L.h_mem + L.o_pack, L.d_mem + L.o_pack, pack, cudaMemcpyDeviceToHost, s));
   L.order = order;
   return G4S_OK;
 }
@@ -1076,18 +1040,21 @@ static int team_round_finish(TeamLaunch &L, cudaStream_t s, double *kernel_ms, i
   G4S_CUDA(cudaEventElapsedTime(&ms, L.e0, L.e1));
   *kernel_ms += ms;
   *launches += 1;
-  if (L.direct)  // each network's share of the pack into its own pinned per-step buffers
-    for (int i : L.order) {
-      g4s_net *n = L.nets[(size_t)i];
-      const size_t st = (size_t)L.steps[(size_t)i];
-      const unsigned char *p = L.h_pack + L.h_off[i];
-      std::memcpy(L.h_status + 2 * i, p, 8);
-      std::memcpy(n->h_counts, p + 8, st * 4);
-      std::memcpy(n->h_base, p + 8 + ((st * 4 + 7) & ~(size_t)7), st * 8);
-      std::memcpy(n->h_stamps, p + 8 + ((st * 4 + 7) & ~(size_t)7) + st * 8, st * 16);
-    }
   for (int i : L.order) {
-    const int rc = status_rc(L.h_status[2 * i], L.h_status[2 * i + 1], "team step kernel");
+    // each network's share of the pack: status words, counts, raster offsets, stamps
+    g4s_net *n = L.nets[(size_t)i];
+    const size_t st = (size_t)L.steps[(size_t)i];
+    const unsigned char *p = L.h_mem + L.o_pack + L.at[(size_t)i];
+    const int *status = reinterpret_cast<const int *>(p), *counts = status + 2;
+    const long long *base = reinterpret_cast<const long long *>(p + 8 + ((st * 4 + 7) & ~(size_t)7));
+    const unsigned long long *stamps = reinterpret_cast<const unsigned long long *>(base + st);
+    n->c_counts.assign(counts, counts + st);
+    n->c_base.assign(base, base + st);
+    n->c_stamps.assign(stamps, stamps + 2 * st);
+  }
+  for (int i : L.order) {
+    const int *status = reinterpret_cast<const int *>(L.h_mem + L.o_pack + L.at[(size_t)i]);
+    const int rc = status_rc(status[0], status[1], "team step kernel");
     if (rc) return rc;
   }
   return G4S_OK;
@@ -1111,6 +1078,13 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
     if (rc0) return rc0;
   }
   const bool team = alg == kAlgSKL && n->team_ok && n->team_ready;
+  // (the team kernel writes a raster only where it is recorded; the other schemes' spike lists
+  // are the raster)
+  if (!team || n->desc.record_raster) {
+    const int64_t longest = team ? n->chunk_steps : alg == kAlgSKL ? n->chunk_legacy : std::min<int64_t>(n->chunk_legacy, kStepGraphSteps);
+    const int rcr = need_raster(n, std::min<int64_t>(steps, longest));
+    if (rcr) return rcr;
+  }
   const auto w0 = std::chrono::steady_clock::now();
   G4S_CUDA(cudaEventRecord(n->ev0, n->stream));
   int64_t remaining = steps, spikes = 0, launches = 0;
@@ -1119,9 +1093,6 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
     // Chunks as team rounds, pipelined: once a round has ended and its raster is copied
     // down, the next round is launched, and the host sorts and files the finished chunk
     // while the GPU runs the next one.
-    std::vector<int> mc;
-    std::vector<long long> mb;
-    std::vector<unsigned long long> ms;
     int cs = 0;
     auto start = [&]() -> int {
       cs = (int)std::min<int64_t>(remaining, n->chunk_steps);
@@ -1136,11 +1107,7 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
     if (rc) return rc;
     while (cs > 0) {
       if ((rc = team_round_finish(n->launch, n->stream, &kernel_ms, &launches))) return rc;
-      // this chunk's per-step arrays, out of the pinned buffers the next round's graph
-      // writes, and its raster, out of the device buffer the next round overwrites
-      mc.assign(n->h_counts, n->h_counts + cs);
-      mb.assign(n->h_base, n->h_base + cs);
-      ms.assign(n->h_stamps, n->h_stamps + 2 * (size_t)cs);
+      // (this chunk's raster out of the device buffer that the next round overwrites)
       if ((rc = chunk_copy_raster(n, cs, n->stream))) return rc;
       G4S_CUDA(cudaStreamSynchronize(n->stream));
       const int done = cs;
@@ -1149,9 +1116,12 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
       cs = 0;
       const int rs = remaining > 0 ? start() : G4S_OK;
       int64_t chunk_spikes = 0;  // (the finished chunk is filed even if the next launch failed)
-      chunk_finish_from(n, done, mc.data(), mb.data(), ms.data(), t0, &chunk_spikes);
+      rc = chunk_finish_from(n, done, t0, &chunk_spikes);
       spikes += chunk_spikes;
-      if (rs) return rs;
+      if (rs || rc) {
+        if (!rs && cs > 0) team_round_finish(n->launch, n->stream, &kernel_ms, &launches);  // (the round in flight ends first)
+        return rs ? rs : rc;
+      }
     }
   }
   while (!team && remaining > 0) {
@@ -1176,6 +1146,7 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
       // chunk is captured only when its graph will be replayed (a graph of this shape
       // exists, or at least two more chunks of its length follow); otherwise it is
       // launched step by step.
+      if (!n->h_t0) G4S_CUDA(cudaMallocHost((void **)&n->h_t0, sizeof(long long)));
       *n->h_t0 = n->t_abs;
       const std::vector<uint64_t> key = {(uint64_t)alg, (uint64_t)cs, (uint64_t)last_chunk,
                                          (uint64_t)n->shape.group, (uint64_t)n->shape.blocks_per_sm,
@@ -1287,6 +1258,7 @@ static int run_nets(g4s_net *const *nets, const int32_t *steps, int count, doubl
     if (rc) return rc;
     if (!nets[i]->team_ok)
       return set_error(G4S_ERR_INVALID, "a network of the batch does not fit the team kernel");
+    if (nets[i]->desc.record_raster && (rc = need_raster(nets[i], std::min<int64_t>(steps[i], nets[i]->chunk_steps)))) return rc;
     remaining[i] = steps[i];
     nets[i]->last_spikes = 0;
   }
@@ -1313,7 +1285,7 @@ static int run_nets(g4s_net *const *nets, const int32_t *steps, int count, doubl
     for (int i = 0; i < count; ++i)
       if (cs[i] > 0) {
         int64_t sp = 0;
-        chunk_finish(nets[i], cs[i], &sp);
+        if ((rc = chunk_finish(nets[i], cs[i], &sp))) return rc;
         nets[i]->last_spikes += sp;
         nets[i]->total_spikes += sp;
         remaining[i] -= cs[i];
@@ -1344,7 +1316,7 @@ struct StateSnapshot {
   SpikeStat *ss = nullptr;
   float *il = nullptr;
   int64_t t_abs = 0, total = 0;
-  size_t nr = 0, nc = 0;
+  size_t nr = 0, nrec = 0, nc = 0;
   ~StateSnapshot() {
     cudaFree(vu);
     cudaFree(acc);
@@ -1366,7 +1338,8 @@ static int snapshot_take(g4s_net *n, StateSnapshot &s) {
   G4S_CUDA(cudaStreamSynchronize(n->stream));
   s.t_abs = n->t_abs;
   s.total = n->total_spikes;
-  s.nr = n->rt.size();
+  s.nr = n->rid.n;
+  s.nrec = n->recorded.size();
   s.nc = n->counts.size();
   return G4S_OK;
 }
@@ -1380,8 +1353,8 @@ static int snapshot_restore(g4s_net *n, const StateSnapshot &s) {
   G4S_CUDA(cudaStreamSynchronize(n->stream));
   n->t_abs = s.t_abs;
   n->total_spikes = s.total;
-  n->rt.resize(s.nr);
-  n->rid.resize(s.nr);
+  n->rid.n = s.nr;
+  n->recorded.resize(s.nrec);
   n->counts.resize(s.nc);
   n->upd_ms.resize(s.nc);
   n->step_ms.resize(s.nc);
@@ -1495,7 +1468,11 @@ static int write_results(g4s_net *n, const std::string &dir, double elapsed, dou
     std::ofstream o(p + "spiketimes.csv");
     if (!o.is_open()) return set_error(G4S_ERR_IO, "cannot open " + p + "spiketimes.csv");
     o << "SpkTime NeuronID" << "\n";
-    for (size_t q = 0; q < n->rt.size(); ++q) o << n->rt[q] << " " << n->rid[q] << "\n";
+    for (const auto &r : n->recorded) {
+      size_t q = r.off;
+      for (int lt = 0; lt < r.cs; ++lt)
+        for (int k = 0; k < n->counts[r.c0 + (size_t)lt]; ++k) o << r.t0 + lt << " " << n->rid.p[q++] << "\n";
+    }
   }
   {
     std::ofstream o(p + "computetime.csv");
@@ -1712,7 +1689,7 @@ int g4s_net_get_info(g4s_net *n, g4s_net_info *info) {
   info->stride = n->v.stride;
   info->steps_done = n->t_abs;
   info->total_spikes = n->total_spikes;
-  info->raster_size = (int64_t)n->rt.size();
+  info->raster_size = (int64_t)n->rid.n;
   info->last_run_ms = n->last_ms;
   info->last_run_wall_ms = n->last_wall_ms;
   info->last_run_spikes = n->last_spikes;
@@ -1738,24 +1715,12 @@ int g4s_pinned_free(void *p) {
 
 int g4s_net_raster(g4s_net *n, int32_t *t, int32_t *id, int64_t cap, int64_t *size) {
   if (!n) return set_error(G4S_ERR_INVALID, "null handle");
-  const int64_t s = (int64_t)n->rt.size();
+  const int64_t s = (int64_t)n->rid.n;
   if (size) *size = s;
   const int64_t m = std::min(s, cap);
   if (m > 0) {
     if (!t || !id) return set_error(G4S_ERR_INVALID, "null raster buffer");
-    // large rasters on several host threads (a fresh destination is mostly page faults)
-    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    const int64_t parts = m >= ((int64_t)1 << 21) ? (int64_t)hw : 1, per = (m + parts - 1) / parts;
-    auto part = [&](int64_t p) {
-      const int64_t lo = p * per, hi = std::min(m, lo + per);
-      if (lo >= hi) return;
-      memcpy(t + lo, n->rt.data() + lo, (size_t)(hi - lo) * 4);
-      memcpy(id + lo, n->rid.data() + lo, (size_t)(hi - lo) * 4);
-    };
-    std::vector<std::thread> pool;
-    for (int64_t p = 1; p < parts; ++p) pool.emplace_back(part, p);
-    part(0);
-    for (auto &th : pool) th.join();
+    raster_copy_out(n, t, id, m);
   }
   return G4S_OK;
 }
@@ -1799,8 +1764,10 @@ int g4s_net_state(g4s_net *n, float *v, float *u, float *i_last, float *a, float
   const int64_t N = n->v.n;
   const int nb = (int)((N + kStateBlock - 1) / kStateBlock);
   const int64_t blk = std::min<int64_t>(N, kStateBlock);
-  if (!n->h_state) G4S_CUDA(cudaMallocHost((void **)&n->h_state, (size_t)blk * 32 * (nb > 1 ? 2 : 1)));
-  float *const half[2] = {n->h_state, n->h_state + (nb > 1 ? blk * 8 : 0)};
+  const int rcs = need_stage(n, (size_t)blk * 32 * (nb > 1 ? 2 : 1));
+  if (rcs) return rcs;
+  float *const h_state = reinterpret_cast<float *>(n->h_stage);
+  float *const half[2] = {h_state, h_state + (nb > 1 ? blk * 8 : 0)};
   auto count = [&](int b) { return (int)std::min<int64_t>(kStateBlock, N - (int64_t)b * kStateBlock); };
   auto copy = [&](int b, int slot, int k) {  // field k, the slot-th of those asked for, of block b
     const size_t cnt = (size_t)count(b);
@@ -1977,10 +1944,10 @@ int g4s_net_stream_raster(g4s_net *n, const char *path) {
 
 int g4s_net_write_raster_file(g4s_net *n, const char *path) {
   if (!n || !path) return set_error(G4S_ERR_INVALID, "null argument");
-  if (n->rid.size() != (size_t)n->total_spikes || n->counts.size() != (size_t)n->t_abs)
+  if (n->rid.n != (size_t)n->total_spikes || n->counts.size() != (size_t)n->t_abs)
     return set_error(G4S_ERR_STATE, "the host raster does not hold every step since the reset "
                                     "(not recorded, or streamed to a file)");
-  return raster_write_all(path, n->v.n, 0, n->counts, n->rid);
+  return raster_write_all(path, n->v.n, 0, n->counts, n->rid.p, n->rid.n);
 }
 
 int g4s_net_save_tables(g4s_net *n, const char *path) {

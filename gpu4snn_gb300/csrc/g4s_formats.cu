@@ -118,13 +118,13 @@ int raster_close(RasterFile *r) {
 }
 
 int raster_write_all(const char *path, int64_t n, int64_t t0, const std::vector<int32_t> &counts,
-                     const std::vector<int32_t> &ids) {
+                     const int32_t *ids, size_t nids) {
   FILE *f = fopen(path, "wb");
   if (!f) return set_error(G4S_ERR_IO, std::string("cannot open ") + path);
   const int32_t cs = (int32_t)counts.size();
-  bool ok = write_raster_header(f, n, t0, (int64_t)counts.size(), (int64_t)ids.size()) &&
+  bool ok = write_raster_header(f, n, t0, (int64_t)counts.size(), (int64_t)nids) &&
             (cs == 0 || (fwrite(&cs, 4, 1, f) == 1 && fwrite(counts.data(), 4, counts.size(), f) == counts.size() &&
-                         (ids.empty() || fwrite(ids.data(), 4, ids.size(), f) == ids.size())));
+                         (nids == 0 || fwrite(ids, 4, nids, f) == nids)));
   ok = fclose(f) == 0 && ok;
   return ok ? G4S_OK : set_error(G4S_ERR_IO, std::string("writing ") + path + " failed");
 }

@@ -169,7 +169,7 @@ int raster_open(const char *path, int64_t n, int64_t t0, RasterFile **out);
 void raster_push(RasterFile *f, const int32_t *counts, int cs, const int32_t *ids, int64_t nids);
 int raster_close(RasterFile *f);
 int raster_write_all(const char *path, int64_t n, int64_t t0, const std::vector<int32_t> &counts,
-                     const std::vector<int32_t> &ids);
+                     const int32_t *ids, size_t nids);
 struct TableHeader {
   int64_t n;
   int32_t nsyn, stride;

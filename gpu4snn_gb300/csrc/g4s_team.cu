@@ -1314,13 +1314,13 @@ __global__ void k_round_gather(const TeamItem *items, const int64_t *off, unsign
 }
 
 cudaError_t launch_round_clear(const TeamItem *items, int count, cudaStream_t s) {
-  k_round_clear<<<(unsigned)count, 256, 0, s>>>(items);
+  k_round_clear<<<(unsigned)count, 512, 0, s>>>(items);
   return cudaGetLastError();
 }
 
 cudaError_t launch_round_gather(const TeamItem *items, const int64_t *off, int count, unsigned char *pack,
                                 cudaStream_t s) {
-  k_round_gather<<<(unsigned)count, 256, 0, s>>>(items, off, pack);
+  k_round_gather<<<(unsigned)count, 512, 0, s>>>(items, off, pack);
   return cudaGetLastError();
 }
 
