@@ -114,6 +114,8 @@ struct TuneChoice {
   int nt = 0;  // threads per CTA of the team kernel (0: chosen from the step size)
 };
 
+constexpr unsigned long long kBarrierNs = 2000000000ull;  // default time limit of a grid barrier
+
 // Spike ids of a handle's recorded chunks: a growing array that is not cleared when it grows
 // (every id is written once, by the thread that files its step).
 struct IdStore {
@@ -150,18 +152,9 @@ struct g4s_net {
   double *d_stats = nullptr;
   int64_t chunk_steps = 0;   // steps per chunk of the team kernel
   int64_t chunk_legacy = 0;  // steps per chunk of the other kernels (raster = spike list)
-  // chunks of the host-driven schemes as CUDA graphs: the chunk's first step (device word,
-  // set from pinned memory at each replay) and up to kStepGraphs captured chunks, keyed by
-  // scheme, length, last-chunk flag and launch shape
-  long long *d_t0 = nullptr, *h_t0 = nullptr;
-  struct StepGraph {
-    std::vector<uint64_t> key;
-    cudaGraphExec_t exec = nullptr;
-  };
-  std::vector<StepGraph> step_graphs;
   int64_t t_abs = 0;
   uint32_t tag_next = 0;  // record tags of the team kernel: never repeated for this handle's lists
-  unsigned long long barrier_ns = 2000000000ull;
+  unsigned long long barrier_ns = kBarrierNs;
   size_t device_bytes = 0;
   // per-step arrays of the last finished chunk
   std::vector<int> c_counts;
@@ -189,7 +182,6 @@ struct g4s_net {
   double last_ms = 0, last_wall_ms = 0;
   int64_t last_spikes = 0;
   int last_alg = -1;
-  DeliverShape shape;
   int barrier_stall = 0;  // injected: extra arrivals the next SKL launch waits for
   // SKL team kernel: team size and slice, per-step spike lists, per-row segment table,
   // requested team size (0 = auto), whether the tables satisfy the exactness bound of the
@@ -244,10 +236,6 @@ static void free_net(g4s_net *n) {
     n->rstream = nullptr;
   }
   n->launch.release();
-  for (auto &gr : n->step_graphs)  // (the captured chunks refer to the buffers below)
-    if (gr.exec) cudaGraphExecDestroy(gr.exec);
-  n->step_graphs.clear();
-  cudaFreeHost(n->h_t0);
   net_free(n, const_cast<unsigned long long *>(v.pair));
   net_free(n, n->arena);
   net_free(n, const_cast<int *>(v.idx));
@@ -366,8 +354,7 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
                o_sstat = place(N * sizeof(SpikeStat)), o_counts = place((size_t)cs * sizeof(int)),
                o_base = place((size_t)cs * sizeof(long long)),
                o_stamps = place(((size_t)cs * 2 + 2) * sizeof(unsigned long long)), o_status = place(sizeof(int)),
-               o_gs = place(sizeof(GridSync) * (1 + 2 * (size_t)kMaxTeam * kRecLines)), o_stats = place(2 * sizeof(double)),
-               o_t0 = place(sizeof(long long));
+               o_gs = place(sizeof(GridSync) * (1 + 2 * (size_t)kMaxTeam * kRecLines)), o_stats = place(2 * sizeof(double));
   unsigned char *mem = nullptr;
   if ((rc = dalloc(n, &mem, bytes, "neuron state and per-step arrays"))) {
     free_net(n);
@@ -386,7 +373,6 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
   v.status = reinterpret_cast<int *>(mem + o_status);
   n->gs = reinterpret_cast<GridSync *>(mem + o_gs);
   n->d_stats = reinterpret_cast<double *>(mem + o_stats);
-  n->d_t0 = reinterpret_cast<long long *>(mem + o_t0);
   if ((rc = dalloc(n, const_cast<int **>(&v.idx), N * S, "targets")) ||
       (rc = dalloc(n, const_cast<float **>(&v.w), N * S, "weights")) ||
       // (a pool's network gets its whole raster now: a run may use another network's stream)
@@ -548,8 +534,6 @@ static double recent_rate(const g4s_net *n) {
 
 static int resolve_alg(g4s_net *n, int alg) {
   if (alg != kAlgAuto) return alg;
-  n->shape = DeliverShape{};
-  n->shape.group = 0;
   TuneChoice c;
   if (n->tuned) {
     c = n->tune;
@@ -791,9 +775,6 @@ static int need_raster(g4s_net *n, int64_t steps) {
   const int64_t want = std::min(n->raster_full, std::max<int64_t>(1, steps) * n->v.n);
   if (want <= n->v.raster_cap) return G4S_OK;
   const int64_t ids = std::min(n->raster_full, std::max(want, (int64_t)1 << 20));
-  for (auto &gr : n->step_graphs)  // (captured chunks hold the buffer's address)
-    if (gr.exec) cudaGraphExecDestroy(gr.exec);
-  n->step_graphs.clear();
   net_free(n, n->v.raster);
   n->v.raster = nullptr;
   n->device_bytes -= (size_t)n->v.raster_cap * 4;
@@ -1072,7 +1053,6 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
   if (n->t_abs + steps > (int64_t)INT32_MAX) return set_error(G4S_ERR_INVALID, "step counter limit");
   const int alg = resolve_alg(n, alg_in);
   NetView &v = n->v;
-  if (n->shape.k_hint <= 0) n->shape.k_hint = (int)std::max<int64_t>(1, v.n / 20);
   if (alg == kAlgSKL) {
     int rc0 = prepare_team(n);
     if (rc0) return rc0;
@@ -1081,7 +1061,7 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
   // (the team kernel writes a raster only where it is recorded; the other schemes' spike lists
   // are the raster)
   if (!team || n->desc.record_raster) {
-    const int64_t longest = team ? n->chunk_steps : alg == kAlgSKL ? n->chunk_legacy : std::min<int64_t>(n->chunk_legacy, kStepGraphSteps);
+    const int64_t longest = team ? n->chunk_steps : n->chunk_legacy;
     const int rcr = need_raster(n, std::min<int64_t>(steps, longest));
     if (rcr) return rcr;
   }
@@ -1125,74 +1105,22 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
     }
   }
   while (!team && remaining > 0) {
-    // (host-driven chunks stay short enough for their graphs to instantiate quickly)
-    const int64_t chunk = alg == kAlgSKL ? n->chunk_legacy : std::min<int64_t>(n->chunk_legacy, kStepGraphSteps);
-    const int cs = (int)std::min<int64_t>(remaining, chunk);
+    const int cs = (int)std::min<int64_t>(remaining, n->chunk_legacy);
     const bool last_chunk = remaining == cs;
-    if (alg == kAlgSKL) {
-      G4S_CUDA(cudaMemsetAsync(v.counts, 0, (size_t)cs * sizeof(int), n->stream));
-      G4S_CUDA(cudaMemsetAsync(v.stamps, 0, ((size_t)cs * 2 + 2) * 8, n->stream));
-      G4S_CUDA(cudaMemsetAsync(n->gs, 0, sizeof(GridSync), n->stream));
-      G4S_CUDA(cudaEventRecord(n->ek0, n->stream));
-      G4S_CUDA(launch_persistent(v, n->t_abs, cs, last_chunk, n->gs, n->barrier_ns, n->shape.group,
-                                 n->barrier_stall, n->stream));
-      n->barrier_stall = 0;
-      launches += 1;
-      G4S_CUDA(cudaEventRecord(n->ek1, n->stream));
-    } else {
-      // The chunk as a CUDA graph (two launches per step would otherwise each cost a host
-      // launch and a gap on the GPU): the chunk's first step from pinned memory, the
-      // clears, then update and delivery for every step between two timing events.  A
-      // chunk is captured only when its graph will be replayed (a graph of this shape
-      // exists, or at least two more chunks of its length follow); otherwise it is
-      // launched step by step.
-      if (!n->h_t0) G4S_CUDA(cudaMallocHost((void **)&n->h_t0, sizeof(long long)));
-      *n->h_t0 = n->t_abs;
-      const std::vector<uint64_t> key = {(uint64_t)alg, (uint64_t)cs, (uint64_t)last_chunk,
-                                         (uint64_t)n->shape.group, (uint64_t)n->shape.blocks_per_sm,
-                                         (uint64_t)n->shape.k_hint};
-      cudaGraphExec_t exec = nullptr;
-      for (auto &gr : n->step_graphs)
-        if (gr.key == key) exec = gr.exec;
-      const bool replayed = exec || (!last_chunk && remaining >= 2 * (int64_t)cs);
-      if (!replayed) {
-        G4S_CUDA(cudaMemcpyAsync(n->d_t0, n->h_t0, sizeof(long long), cudaMemcpyHostToDevice, n->stream));
-        G4S_CUDA(cudaMemsetAsync(v.counts, 0, (size_t)cs * sizeof(int), n->stream));
-        G4S_CUDA(cudaMemsetAsync(v.stamps, 0, ((size_t)cs * 2 + 2) * 8, n->stream));
-        G4S_CUDA(cudaEventRecord(n->ek0, n->stream));
-        for (int lt = 0; lt < cs; ++lt) {
-          G4S_CUDA(launch_update(v, n->d_t0, lt, last_chunk && lt == cs - 1, n->stream));
-          G4S_CUDA(launch_deliver(v, lt, alg, n->shape, n->stream));
-        }
-        G4S_CUDA(cudaEventRecord(n->ek1, n->stream));
-      } else if (!exec) {
-        if ((int)n->step_graphs.size() >= kStepGraphs) {  // the oldest goes
-          cudaGraphExecDestroy(n->step_graphs.front().exec);
-          n->step_graphs.erase(n->step_graphs.begin());
-        }
-        G4S_CUDA(cudaStreamBeginCapture(n->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = cudaMemcpyAsync(n->d_t0, n->h_t0, sizeof(long long), cudaMemcpyHostToDevice, n->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(v.counts, 0, (size_t)cs * sizeof(int), n->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(v.stamps, 0, ((size_t)cs * 2 + 2) * 8, n->stream);
-        if (e == cudaSuccess) e = cudaEventRecordWithFlags(n->ek0, n->stream, cudaEventRecordExternal);
-        for (int lt = 0; lt < cs && e == cudaSuccess; ++lt) {
-          e = launch_update(v, n->d_t0, lt, last_chunk && lt == cs - 1, n->stream);
-          if (e == cudaSuccess) e = launch_deliver(v, lt, alg, n->shape, n->stream);
-        }
-        if (e == cudaSuccess) e = cudaEventRecordWithFlags(n->ek1, n->stream, cudaEventRecordExternal);
-        cudaGraph_t g = nullptr;
-        const cudaError_t e_end = cudaStreamEndCapture(n->stream, &g);
-        if (e == cudaSuccess) e = e_end;
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
-        if (g) cudaGraphDestroy(g);
-        if (e != cudaSuccess) return cuda_error(e, "capturing a chunk of the step kernels");
-        n->step_graphs.push_back({key, exec});
-      }
-      if (exec) G4S_CUDA(cudaGraphLaunch(exec, n->stream));
-      launches += 2 * (int64_t)cs;
-    }
+    // (the time limit and injected faults are the SKL scheme's)
+    const bool skl = alg == kAlgSKL;
+    G4S_CUDA(cudaMemsetAsync(v.counts, 0, (size_t)cs * sizeof(int), n->stream));
+    G4S_CUDA(cudaMemsetAsync(v.stamps, 0, ((size_t)cs * 2 + 2) * 8, n->stream));
+    G4S_CUDA(cudaMemsetAsync(n->gs, 0, sizeof(GridSync), n->stream));
+    G4S_CUDA(cudaEventRecord(n->ek0, n->stream));
+    int made = 0;
+    G4S_CUDA(launch_steps(v, n->t_abs, cs, last_chunk, n->gs, skl ? n->barrier_ns : kBarrierNs, alg,
+                          skl ? n->barrier_stall : 0, n->stream, &made));
+    if (skl) n->barrier_stall = 0;
+    launches += made;
+    G4S_CUDA(cudaEventRecord(n->ek1, n->stream));
     {
-      int rc = check_status(n, alg == kAlgSKL ? "persistent step kernel" : "step kernels");
+      int rc = check_status(n, "persistent step kernel");
       if (rc) return rc;
       float kms = 0.0f;
       G4S_CUDA(cudaEventElapsedTime(&kms, n->ek0, n->ek1));

@@ -21,20 +21,12 @@ constexpr int kAlgAB = 3;
 constexpr int kAlgSKL = 4;
 constexpr int kAlgAuto = 5;
 
-// Launch shape of a delivery scheme (the autotuner's output).
-struct DeliverShape {
-  int k_hint = 0;         // S: expected spikes per step, sizes the oversubscribed grid
-  int group = 0;          // AP and SKL: threads per spiking row (0 = flat split for SKL)
-  int blocks_per_sm = 4;  // AP and AB: resident blocks per SM
-};
-
 cudaError_t launch_init(const NetView &v, cudaStream_t s);
 cudaError_t launch_conngen(const NetView &v, int self_loops, cudaStream_t s);
-// t0: device word holding the absolute step of the chunk's step 0
-cudaError_t launch_update(const NetView &v, const long long *t0, int lt, bool last, cudaStream_t s);
-cudaError_t launch_deliver(const NetView &v, int lt, int alg, const DeliverShape &sh, cudaStream_t s);
-cudaError_t launch_persistent(const NetView &v, int64_t t_abs0, int nsteps, bool last_chunk, GridSync *gs,
-                              unsigned long long limit_ns, int group, int stall, cudaStream_t s);
+// nsteps steps of a scheme (kAlgSKL: the fallback of the team kernel) with the currents in
+// global memory; *launches: kernel launches made
+cudaError_t launch_steps(const NetView &v, int64_t t_abs0, int nsteps, bool last_chunk, GridSync *gs,
+                         unsigned long long limit_ns, int alg, int stall, cudaStream_t s, int *launches);
 cudaError_t launch_stats(const NetView &v, double *out, cudaStream_t s);
 // fields of neurons [i0, i0 + cnt) as separate arrays: bits 0..7 of `fields` are v, u, I, a, b,
 // c, d and the spike count; `out` is device-accessible, cnt values per field asked for
@@ -57,8 +49,6 @@ constexpr int64_t kBatchSlice = 8192;          // neurons per CTA of a batched n
                                                // 824 at 16384; served requests 41.9/s, 40.1, 32.7)
 constexpr int kStateBlock = 65536;             // neurons of the state read back at a time
 constexpr int kStateThreadBlocks = 3;          // ... in this many blocks or more, a thread per field
-constexpr int kStepGraphSteps = 512;          // longest chunk of the host-driven schemes (one CUDA graph)
-constexpr int kStepGraphs = 4;                 // captured chunks kept per network
 constexpr int kMaxTeam = 176;                  // CTAs of one team (eight source ranks a warp, 22 such warps)
 // Spike records of a multi-CTA team: per rank and step parity kRecLines lines of 16
 // tagged 64-bit words (count, then up to 16 kRecLines - 1 ids); readers fetch the second

@@ -2,14 +2,15 @@
 //
 //   k_init_state   neuron parameters and initial state        (initNeuron, gpu4snn.cu:286-320)
 //   k_conngen      distinct-target tables, Philox law          (host generator, gpu4snn.cu:873-905)
-//   k_update       update fused with spike compaction          (stateupdate, gpu4snn.cu:334-417)
-//   k_deliver_*    spike delivery, four schemes:
-//                    N  thread per spiking neuron              (deliverspks1, gpu4snn.cu:420-443)
-//                    S  thread per 4 synapses, oversubscribed  (deliverspks2, gpu4snn.cu:446-467)
+//   k_persistent   the steps of a chunk of the N, S, AP and AB schemes (and of SKL where the team
+//                  kernel does not fit): update (stateupdate, gpu4snn.cu:334-417) and delivery in
+//                  one cooperative launch with timed grid barriers (k_update and k_deliver, two
+//                  launches a step, for S on large networks):
+//                    N  a warp per spiking neuron              (deliverspks1, gpu4snn.cu:420-443)
+//                    S  flat over the step's synapses          (deliverspks2, gpu4snn.cu:446-467)
 //                    AP thread group per spiking row           (propagatespikes, gpu4snn.cu:323-331)
-//                    AB persistent grid over the synapse range (AB_deliverspks, gpu4snn.cu:554-584)
-//   k_persistent   all steps of a chunk in one cooperative launch with timed grid barriers
-//                                                              (SKL_deliverspks, gpu4snn.cu:669-716)
+//                    AB flat over the step's synapses          (AB_deliverspks, gpu4snn.cu:554-584)
+//   k_state_pack   the neuron record for the host
 //   k_stats        FP64 firing rate and ISI CV reductions
 //
 // Delivery reads the compacted spike list of the step (int32 ids), streams each spiking row
@@ -132,91 +133,111 @@ __global__ void k_conngen(NetView v, int self_loops, int log2h, int bits, int64_
 }
 
 // ---------------------------------------------------------------------------------------
-// Update of one neuron; returns its spike flag.  Writes the current back only when it was
-// non-zero, and the spike statistics only on a spike.
+// The step loop of the schemes that add into global memory: every step of a chunk in one
+// cooperative launch.  Per step: update and compaction of the spikes into the raster, grid
+// barrier, delivery, grid barrier.  Bound by the two barriers and the chain of global round
+// trips between them for small networks, by the L2's additions for large ones.  (Two
+// launches a step instead took 8.5 us of host time, or 6.1 us a step as a captured graph,
+// for N=2,500.)
+//
+// The drive of a thread's first neuron is drawn while it waits at the second barrier.
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ bool update_one(const NetView &v, int64_t i, int64_t t_abs, bool last) {
-  float2 s = v.vu[i];
-  const float4 p = v.abcd[i];
-  const long long a = __ldcg(v.acc + i);
-  const float g = i < v.nexc ? v.ge : v.gi;
-  const float z = normal(v.seed, (uint64_t)i, (uint64_t)t_abs);
-  float I;
-  const bool spk = izh_step(s.x, s.y, I, p, g, z, q32_current(a));
-  v.vu[i] = s;
-  if (a != 0) v.acc[i] = 0;
-  if (last) v.ilast[i] = I;
-  if (spk) {
-    SpikeStat st = v.sstat[i];
-    st.nospks += 1;
-    if (st.last >= 0) {
-      const long long isi = t_abs - st.last;
-      st.nisi += 1;
-      st.s1 += isi;
-      st.s2 += isi * isi;
+// The update of a block's neurons (tiles of NT, every gridDim.x-th), the next tile's state in
+// flight while a tile's drive is drawn (1024 threads an SM so, 64 registers each: N=10^6 at
+// drive 0.5 22.1 us a step against 23.9 with 1536 and nothing in flight); spikes are collected in
+// shared memory and appended to the raster at base_t with one global atomic per kSpikeTiles
+// tiles.  z0: the drive of the block's first tile (kDrawn; else it is drawn here).  Returns
+// the block's spikes.
+constexpr int kSpikeTiles = 8;
+template <int NT, bool kDrawn>
+__device__ __forceinline__ unsigned update_phase(const NetView &v, int lt, int64_t t_abs, long long base_t, bool last,
+                                                 float z0, int *s_ids, int *s_n, long long *s_slot) {
+  unsigned mine = 0;
+  const int64_t tiles = (v.n + NT - 1) / NT;
+  for (int64_t g = blockIdx.x; g < tiles; g += (int64_t)gridDim.x * kSpikeTiles) {
+    const int64_t end = min(tiles, g + (int64_t)gridDim.x * kSpikeTiles);
+    int64_t i = g * NT + threadIdx.x;
+    float2 sn = make_float2(0.0f, 0.0f);
+    float rn = 0.0f;
+    long long an = 0;
+    if (i < v.n) {
+      sn = v.vu[i];
+      rn = v.rpar[i];
+      an = __ldcg(v.acc + i);
     }
-    st.last = (int)t_abs;
-    v.sstat[i] = st;
-  }
-  return spk;
-}
-
-// Update all neurons of step lt (absolute step t_abs) and append the spiking ids to the
-// raster at base_t, one global atomic per block tile.
-template <int NT>
-__device__ __forceinline__ void update_phase(const NetView &v, int lt, int64_t t_abs, long long base_t,
-                                             bool last, int *s_warp, long long *s_slot) {
-  for (int64_t tile = blockIdx.x; tile * NT < v.n; tile += gridDim.x) {
-    const int64_t i = tile * NT + threadIdx.x;
-    bool spk = false;
-    if (i < v.n) spk = update_one(v, i, t_abs, last);
-    int total;
-    const int slot = block_compact<NT>(spk, s_warp, &total);
-    if (threadIdx.x == 0 && total) *s_slot = atomicAdd(v.counts + lt, total);
+    for (int64_t tile = g; tile < end; tile += gridDim.x, i += (int64_t)gridDim.x * NT) {
+      if (i < v.n) {
+        float2 s = sn;
+        const float r = rn;
+        const long long a = an;
+        const int64_t in = i + (int64_t)gridDim.x * NT;
+        if (in < v.n && tile + gridDim.x < end) {
+          sn = v.vu[in];
+          rn = v.rpar[in];
+          an = __ldcg(v.acc + in);
+        }
+        const float z = kDrawn && tile == blockIdx.x ? z0 : normal(v.seed, (uint64_t)i, (uint64_t)t_abs);
+        float I;
+        const bool spk = izh_step(s.x, s.y, I, izh_abcd(r, i < v.nexc), i < v.nexc ? v.ge : v.gi, z, q32_current(a));
+        v.vu[i] = s;
+        if (a != 0) v.acc[i] = 0;  // (written back only when it was non-zero)
+        if (last) v.ilast[i] = I;
+        if (spk) {
+          s_ids[atomicAdd(s_n, 1)] = (int)i;
+          SpikeStat st = v.sstat[i];
+          st.nospks += 1;
+          if (st.last >= 0) {
+            const long long isi = t_abs - st.last;
+            st.nisi += 1;
+            st.s1 += isi;
+            st.s2 += isi * isi;
+          }
+          st.last = (int)t_abs;
+          v.sstat[i] = st;
+        }
+      }
+    }
     __syncthreads();
-    if (spk) {
-      const long long pos = base_t + *s_slot + slot;
-      if (pos < v.raster_cap)
-        v.raster[pos] = (int)i;
-      else
-        atomicCAS(v.status, 0, kErrOverflowCode);
+    const int total = *s_n;
+    if (total) {  // (the same for the whole block)
+      if (threadIdx.x == 0) *s_slot = base_t + atomicAdd(v.counts + lt, total);
+      __syncthreads();
+      for (int k = threadIdx.x; k < total; k += NT) {
+        const long long pos = *s_slot + k;
+        if (pos < v.raster_cap)
+          v.raster[pos] = s_ids[k];
+        else
+          atomicCAS(v.status, 0, kErrOverflowCode);
+      }
+      mine += total;
+      __syncthreads();
+      if (threadIdx.x == 0) *s_n = 0;
     }
     __syncthreads();
   }
+  return mine;
 }
 
-// (the chunk's first step is read from device memory, so that a captured chunk replays for
-// any chunk of the run)
-template <int NT>
-__global__ void __launch_bounds__(NT) k_update(NetView v, const long long *t0, int lt, int last) {
-  const int64_t t_abs0 = *t0;
-  __shared__ int s_warp[NT / 32 + 1];
-  __shared__ long long s_slot;
-  const long long base_t = lt == 0 ? 0ll : __ldcg(v.base + lt - 1) + __ldcg(v.counts + lt - 1);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    v.base[lt] = base_t;
-    v.stamps[2 * lt] = globaltimer();
-  }
-  update_phase<NT>(v, lt, t_abs0 + lt, base_t, last != 0, s_warp, &s_slot);
-}
-
-// ---------------------------------------------------------------------------------------
-// Delivery.
-// ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void deliver_vec(const NetView &v, int row, uint32_t j) {
+// Four synapses of a row.
+struct Vec4 {
+  int4 t;
+  float4 w;
+};
+__device__ __forceinline__ Vec4 load_vec(const NetView &v, int row, uint32_t j) {
   const size_t off = (size_t)row * (size_t)(v.stride >> 2) + j;
   const uint64_t pol = policy_evict_first();
-  const int4 t = ld_stream_i4(reinterpret_cast<const int4 *>(v.idx) + off, pol);
-  const float4 w = ld_stream_f4(reinterpret_cast<const float4 *>(v.w) + off, pol);
-  deliver4(v.acc, t, w);
+  return Vec4{ld_stream_i4(reinterpret_cast<const int4 *>(v.idx) + off, pol),
+              ld_stream_f4(reinterpret_cast<const float4 *>(v.w) + off, pol)};
 }
 
-// Flat split of the step's K x (stride/4) vectors over all threads of the grid; the
-// (row, vector) pair advances by a fixed stride without a division per iteration.
+// Flat split of the step's K x (stride/4) vectors over all threads of the grid (S, AB); the
+// (row, vector) pair advances by a fixed stride without a division per vector.  Consecutive
+// warps' worths of vectors go to different blocks, so that a small step uses every SM (N=
+// 2,500 5.0 us a step against 5.4, N=10^6 at drive 0.5 20.4 against 21.9).
 __device__ __forceinline__ void deliver_flat(const NetView &v, const int *list, int K) {
   const uint32_t rv = (uint32_t)(v.stride >> 2);
   const uint64_t total = (uint64_t)K * rv;
-  const uint64_t g0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t g0 = ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
   const uint64_t gs = (uint64_t)gridDim.x * blockDim.x;
   if (g0 >= total) return;
   uint64_t q = g0 / rv;
@@ -224,7 +245,8 @@ __device__ __forceinline__ void deliver_flat(const NetView &v, const int *list, 
   const uint64_t dq = gs / rv;
   const uint32_t dj = (uint32_t)(gs - dq * rv);
   for (uint64_t g = g0; g < total; g += gs) {
-    deliver_vec(v, __ldcg(list + q), j);
+    const Vec4 x = load_vec(v, __ldcg(list + q), j);
+    deliver4(v.acc, x.t, x.w);
     q += dq;
     j += dj;
     if (j >= rv) {
@@ -234,89 +256,81 @@ __device__ __forceinline__ void deliver_flat(const NetView &v, const int *list, 
   }
 }
 
-// Groups of `group` consecutive threads take whole spiking rows.
+// Groups of `group` consecutive threads take whole spiking rows (N, AP).
 __device__ __forceinline__ void deliver_groups(const NetView &v, const int *list, int K, int group) {
   const uint32_t rv = (uint32_t)(v.stride >> 2);
   const int gpb = blockDim.x / group;
   const int lig = threadIdx.x % group;
   const int64_t ngroups = (int64_t)gridDim.x * gpb;
-  for (int64_t q = (int64_t)blockIdx.x * gpb + threadIdx.x / group; q < K; q += ngroups) {
+  // (consecutive rows to different blocks: a step's few rows spread over the SMs)
+  for (int64_t q = (int64_t)(threadIdx.x / group) * gridDim.x + blockIdx.x; q < K; q += ngroups) {
     const int row = __ldcg(list + q);
-    for (uint32_t j = lig; j < rv; j += group) deliver_vec(v, row, j);
+    for (uint32_t j = lig; j < rv; j += group) {
+      const Vec4 x = load_vec(v, row, j);
+      deliver4(v.acc, x.t, x.w);
+    }
   }
 }
 
-__device__ __forceinline__ void step_list(const NetView &v, int lt, const int *&list, int &K) {
-  K = __ldcg(v.counts + lt);
-  list = v.raster + __ldcg(v.base + lt);
-}
-
-__device__ __forceinline__ void stamp_delivery(const NetView &v, int lt) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) v.stamps[2 * lt + 1] = globaltimer();
-}
-
-// N: one thread per spiking neuron walks its whole row.
-__global__ void k_deliver_n(NetView v, int lt) {
-  stamp_delivery(v, lt);
-  const int *list;
-  int K;
-  step_list(v, lt, list, K);
-  const uint32_t rv = (uint32_t)(v.stride >> 2);
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < K; q += (int64_t)gridDim.x * blockDim.x) {
-    const int row = __ldcg(list + q);
-    for (uint32_t j = 0; j < rv; ++j) deliver_vec(v, row, j);
-  }
-}
-
-// S and AB: flat split (S launches an oversubscribed grid, AB a persistent one).
-__global__ void k_deliver_flat(NetView v, int lt) {
-  stamp_delivery(v, lt);
-  const int *list;
-  int K;
-  step_list(v, lt, list, K);
-  deliver_flat(v, list, K);
-}
-
-// AP: a thread group per spiking row (the nested fan-out, without device launches).
-__global__ void k_deliver_ap(NetView v, int lt, int group) {
-  stamp_delivery(v, lt);
-  const int *list;
-  int K;
-  step_list(v, lt, list, K);
-  deliver_groups(v, list, K, group);
-}
-
-// ---------------------------------------------------------------------------------------
-// SKL: every step of the chunk in one cooperative launch.  Per step: update + compaction,
-// barrier, delivery (flat or grouped), barrier.  The running raster offset is kept in a
-// register by every block (the step's count is final after the first barrier).
-// ---------------------------------------------------------------------------------------
+// The barrier's counter carries the chunk's spikes so far in its high half: past the step's
+// first barrier every block knows the step's count.  group: threads per spiking row, 0 = flat.
 template <int NT>
-__global__ void __launch_bounds__(NT) k_persistent(NetView v, int64_t t_abs0, int nsteps, int last_chunk,
-                                                   GridSync *gs, unsigned long long limit_ns, int group,
-                                                   int stall) {
-  __shared__ int s_warp[NT / 32 + 1];
+__global__ void __launch_bounds__(NT, 1024 / NT) k_persistent(NetView v, int64_t t_abs0, int nsteps, int last_chunk,
+                                                      GridSync *gs, unsigned long long limit_ns, int group,
+                                                      int stall) {
+  __shared__ int s_ids[kSpikeTiles * NT];
+  __shared__ int s_n;
   __shared__ long long s_slot;
   unsigned epoch = 0;
   long long base = 0;
   const unsigned nb = gridDim.x + (unsigned)stall;  // stall > 0 only under fault injection
+  const int64_t first = (int64_t)blockIdx.x * NT + threadIdx.x;
+  float z0 = first < v.n ? normal(v.seed, (uint64_t)first, (uint64_t)t_abs0) : 0.0f;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
   for (int lt = 0; lt < nsteps; ++lt) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       v.base[lt] = base;
       v.stamps[2 * lt] = globaltimer();
     }
-    update_phase<NT>(v, lt, t_abs0 + lt, base, last_chunk && lt == nsteps - 1, s_warp, &s_slot);
-    if (!grid_barrier(gs, nb, epoch, limit_ns)) return;
-    stamp_delivery(v, lt);
-    const int K = __ldcg(v.counts + lt);
+    const unsigned mine =
+        update_phase<NT, true>(v, lt, t_abs0 + lt, base, last_chunk && lt == nsteps - 1, z0, s_ids, &s_n, &s_slot);
+    grid_arrive(gs, epoch, mine);
+    unsigned spikes;
+    if (!grid_wait(gs, epoch, nb, limit_ns, spikes)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) v.stamps[2 * lt + 1] = globaltimer();
+    const int K = (int)(spikes - (unsigned)base);
     const int *list = v.raster + base;
     if (group > 0)
       deliver_groups(v, list, K, group);
     else
       deliver_flat(v, list, K);
-    if (!grid_barrier(gs, nb, epoch, limit_ns)) return;
+    grid_arrive(gs, epoch, 0u);
+    if (first < v.n && lt + 1 < nsteps) z0 = normal(v.seed, (uint64_t)first, (uint64_t)(t_abs0 + lt + 1));
+    if (!grid_wait(gs, epoch, nb, limit_ns, spikes)) return;
     base += K;
   }
+}
+
+// A step as two launches: the update, and a flat delivery with a grid sized for its work.
+template <int NT>
+__global__ void __launch_bounds__(NT) k_update(NetView v, int64_t t_abs0, int lt, int last) {
+  __shared__ int s_ids[kSpikeTiles * NT];
+  __shared__ int s_n;
+  __shared__ long long s_slot;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  const long long base_t = lt == 0 ? 0ll : __ldcg(v.base + lt - 1) + __ldcg(v.counts + lt - 1);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    v.base[lt] = base_t;
+    v.stamps[2 * lt] = globaltimer();
+  }
+  update_phase<NT, false>(v, lt, t_abs0 + lt, base_t, last != 0, 0.0f, s_ids, &s_n, &s_slot);
+}
+
+__global__ void k_deliver(NetView v, int lt) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) v.stamps[2 * lt + 1] = globaltimer();
+  deliver_flat(v, v.raster + __ldcg(v.base + lt), __ldcg(v.counts + lt));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -435,50 +449,32 @@ cudaError_t launch_conngen(const NetView &v, int self_loops, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-constexpr int kUpdNT = 256;
-constexpr int kPerNT = 512;
+// CTA size of the persistent kernel by the neurons: 256 threads and one block per SM where
+// that covers them (N=2,500 S 5.1 us a step against 5.9), else 512 (N=100,000 13.1 against
+// 19.4), two blocks per SM if one does not cover them.
+constexpr int kPerSmall = 256, kPerLarge = 512;
 
-cudaError_t launch_update(const NetView &v, const long long *t0, int lt, bool last, cudaStream_t s) {
-  k_update<kUpdNT><<<grid_for(v.n, kUpdNT, 8), kUpdNT, 0, s>>>(v, t0, lt, last ? 1 : 0);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_deliver(const NetView &v, int lt, int alg, const DeliverShape &sh, cudaStream_t s) {
-  switch (alg) {
-    case kAlgN:
-      k_deliver_n<<<grid_for(v.n, 128, 64), 128, 0, s>>>(v, lt);
-      break;
-    case kAlgS: {
-      const int64_t vecs = (int64_t)(sh.k_hint > 0 ? sh.k_hint : 1) * (v.stride >> 2);
-      k_deliver_flat<<<grid_for(vecs, 256, 64), 256, 0, s>>>(v, lt);
-      break;
-    }
-    case kAlgAP: {
-      const int group = sh.group > 0 ? sh.group : 64;
-      k_deliver_ap<<<(unsigned)(sm_count() * sh.blocks_per_sm), 256, 0, s>>>(v, lt, group);
-      break;
-    }
-    case kAlgAB:
-      k_deliver_flat<<<(unsigned)(sm_count() * sh.blocks_per_sm), 256, 0, s>>>(v, lt);
-      break;
-    default:
-      return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
-int persistent_blocks() {
+template <int NT>
+static int persistent_occupancy() {
   int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_persistent<kPerNT>, kPerNT, 0);
-  if (occ < 1) occ = 1;
-  return occ * sm_count();
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_persistent<NT>, NT, 0);
+  return occ < 1 ? 1 : occ;
 }
 
-cudaError_t launch_persistent(const NetView &v, int64_t t_abs0, int nsteps, bool last_chunk, GridSync *gs,
-                              unsigned long long limit_ns, int group, int stall, cudaStream_t s) {
+int persistent_blocks() { return persistent_occupancy<kPerLarge>() * sm_count(); }
+
+// Threads per spiking row of a scheme: N a warp for each spiking neuron (one thread, the
+// reference's choice, walks a row as a chain of loads: 88 us a step for N=2,500 x 1000 against
+// 7), AP a group of 64, S and AB flat over all synapses of the step, as the SKL fallback.
+static int deliver_group(int alg) { return alg == kAlgN ? 32 : alg == kAlgAP ? 64 : 0; }
+
+template <int NT>
+static cudaError_t persistent_nt(const NetView &v, int64_t t_abs0, int nsteps, bool last_chunk, GridSync *gs,
+                                 unsigned long long limit_ns, int group, int stall, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)persistent_blocks());
-  cfg.blockDim = dim3(kPerNT);
+  const int sms = sm_count();
+  cfg.gridDim = dim3((unsigned)(v.n <= (int64_t)sms * NT ? sms : sms * persistent_occupancy<NT>()));
+  cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -486,8 +482,29 @@ cudaError_t launch_persistent(const NetView &v, int64_t t_abs0, int nsteps, bool
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_persistent<kPerNT>, v, t_abs0, nsteps, last_chunk ? 1 : 0, gs, limit_ns,
-                            group, stall);
+  return cudaLaunchKernelEx(&cfg, k_persistent<NT>, v, t_abs0, nsteps, last_chunk ? 1 : 0, gs, limit_ns, group, stall);
+}
+
+cudaError_t launch_steps(const NetView &v, int64_t t_abs0, int nsteps, bool last_chunk, GridSync *gs,
+                         unsigned long long limit_ns, int alg, int stall, cudaStream_t s, int *launches) {
+  const int group = deliver_group(alg);
+  *launches = 1;
+  // S on large networks with long rows: two launches a step, the delivery's grid oversubscribed
+  // (N=250,000 x 10,000 238 us a step against 266 persistent; N=10^6 x 1000 83 against 80)
+  if (!(alg == kAlgS && v.n >= 200000 && v.nsyn >= 4096))
+    return v.n <= (int64_t)sm_count() * kPerSmall
+               ? persistent_nt<kPerSmall>(v, t_abs0, nsteps, last_chunk, gs, limit_ns, group, stall, s)
+               : persistent_nt<kPerLarge>(v, t_abs0, nsteps, last_chunk, gs, limit_ns, group, stall, s);
+  *launches = 2 * nsteps;
+  // (a thread per vector for up to 5% of the neurons firing)
+  const unsigned grid = grid_for(v.n / 20 * (v.stride >> 2), 256, 64);
+  for (int lt = 0; lt < nsteps; ++lt) {
+    k_update<256><<<grid_for(v.n, 256, 8), 256, 0, s>>>(v, t_abs0, lt, last_chunk && lt == nsteps - 1);
+    k_deliver<<<grid, 256, 0, s>>>(v, lt);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t launch_state_pack(const NetView &v, int64_t i0, int cnt, unsigned fields, float *out, cudaStream_t s) {

@@ -16,11 +16,12 @@ constexpr int kErrTimeoutCode = 1;   // a grid barrier waited longer than its li
 constexpr int kErrOverflowCode = 2;  // a spike did not fit the raster buffer
 constexpr int kErrConnCode = 3;      // connectivity generation ran out of draws
 
-// Grid barrier state: a monotone arrival counter and an error word (one 128 B line).
+// Grid barrier state: a monotone counter (arrivals, and a sum in its high half) and an error
+// word (one 128 B line).
 struct alignas(128) GridSync {
-  unsigned count;
+  unsigned long long count;
   int error;
-  unsigned pad[30];
+  unsigned pad[29];
 };
 
 // Per-neuron spike statistics, touched only when the neuron fires (32 B, one sector).
