@@ -1047,6 +1047,42 @@ static int team_round(g4s_net *const *nets, const int *steps, const bool *last, 
   return rc ? rc : team_round_finish(L, s, kernel_ms, launches);
 }
 
+// One chunk of steps by a launch that works on the handle's global arrays.
+static int run_chunk(g4s_net *n, int cs, bool last, bool skl, StepLaunch &launch, int64_t *spikes, double *kernel_ms) {
+  NetView &v = n->v;
+  G4S_CUDA(cudaMemsetAsync(v.counts, 0, (size_t)cs * sizeof(int), n->stream));
+  G4S_CUDA(cudaMemsetAsync(v.stamps, 0, ((size_t)cs * 2 + 2) * 8, n->stream));
+  G4S_CUDA(cudaMemsetAsync(n->gs, 0, sizeof(GridSync), n->stream));
+  G4S_CUDA(cudaEventRecord(n->ek0, n->stream));
+  G4S_CUDA(launch(v, n->t_abs, cs, last, n->gs, skl ? n->barrier_ns : kBarrierNs, skl ? n->barrier_stall : 0, n->stream));
+  if (skl) n->barrier_stall = 0;
+  G4S_CUDA(cudaEventRecord(n->ek1, n->stream));
+  int rc = check_status(n, "persistent step kernel");
+  if (rc) return rc;
+  float kms = 0.0f;
+  G4S_CUDA(cudaEventElapsedTime(&kms, n->ek0, n->ek1));
+  *kernel_ms += kms;
+  return absorb_chunk(n, cs, spikes);
+}
+
+namespace g4s {
+int64_t net_chunk_steps(const g4s_net *n) { return n->chunk_legacy; }
+
+int net_run_by(g4s_net *n, int steps, bool last, StepLaunch &launch) {
+  int rc = need_raster(n, steps);
+  int64_t spikes = 0;
+  double ms = 0.0;
+  if (!rc) rc = run_chunk(n, steps, last, true, launch, &spikes, &ms);
+  if (rc) return rc;
+  n->last_ms = n->last_wall_ms = n->last_kernel_ms = ms;
+  n->last_launches = 1;
+  n->last_spikes = spikes;
+  n->total_spikes += spikes;
+  n->last_alg = kAlgSKL;
+  return G4S_OK;
+}
+}  // namespace g4s
+
 static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
   if (steps < 0) return set_error(G4S_ERR_INVALID, "steps must be >= 0");
   if (alg_in < 0 || alg_in > kAlgAuto) return set_error(G4S_ERR_INVALID, "unknown algorithm");
@@ -1104,30 +1140,23 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
       }
     }
   }
+  struct Schemes : StepLaunch {  // (the time limit and injected faults are the SKL scheme's)
+    int alg;
+    int64_t *launches;
+    cudaError_t operator()(const NetView &v, int64_t t_abs0, int cs, bool last, GridSync *gs, unsigned long long limit_ns,
+                           int stall, cudaStream_t s) override {
+      int made = 0;
+      const cudaError_t e = launch_steps(v, t_abs0, cs, last, gs, limit_ns, alg, stall, s, &made);
+      *launches += made;
+      return e;
+    }
+  } schemes;
+  schemes.alg = alg;
+  schemes.launches = &launches;
   while (!team && remaining > 0) {
     const int cs = (int)std::min<int64_t>(remaining, n->chunk_legacy);
-    const bool last_chunk = remaining == cs;
-    // (the time limit and injected faults are the SKL scheme's)
-    const bool skl = alg == kAlgSKL;
-    G4S_CUDA(cudaMemsetAsync(v.counts, 0, (size_t)cs * sizeof(int), n->stream));
-    G4S_CUDA(cudaMemsetAsync(v.stamps, 0, ((size_t)cs * 2 + 2) * 8, n->stream));
-    G4S_CUDA(cudaMemsetAsync(n->gs, 0, sizeof(GridSync), n->stream));
-    G4S_CUDA(cudaEventRecord(n->ek0, n->stream));
-    int made = 0;
-    G4S_CUDA(launch_steps(v, n->t_abs, cs, last_chunk, n->gs, skl ? n->barrier_ns : kBarrierNs, alg,
-                          skl ? n->barrier_stall : 0, n->stream, &made));
-    if (skl) n->barrier_stall = 0;
-    launches += made;
-    G4S_CUDA(cudaEventRecord(n->ek1, n->stream));
-    {
-      int rc = check_status(n, "persistent step kernel");
-      if (rc) return rc;
-      float kms = 0.0f;
-      G4S_CUDA(cudaEventElapsedTime(&kms, n->ek0, n->ek1));
-      kernel_ms += kms;
-    }
     int64_t chunk_spikes = 0;
-    int rc = absorb_chunk(n, cs, &chunk_spikes);
+    const int rc = run_chunk(n, cs, remaining == cs, alg == kAlgSKL, schemes, &chunk_spikes, &kernel_ms);
     if (rc) return rc;
     spikes += chunk_spikes;
     remaining -= cs;

@@ -147,6 +147,15 @@ size_t team_smem(int64_t rc, int team);
 // A handle's arrays, stream and absolute step, for the library's other translation units
 // (the on-device FP64 check, g4s_fp64check.cu).
 const NetView &net_view(const g4s_net *n);
+// `steps` further steps of the handle (at most net_chunk_steps) by a launch of the caller's:
+// it does what the library's own step kernels do with the handle's arrays, and the handle's
+// record takes the results.  `stall`: blocks too many for its grid barrier to wait for.
+struct StepLaunch {
+  virtual cudaError_t operator()(const NetView &v, int64_t t_abs0, int steps, bool last, GridSync *gs,
+                                 unsigned long long limit_ns, int stall, cudaStream_t s) = 0;
+};
+int net_run_by(g4s_net *n, int steps, bool last, StepLaunch &launch);
+int64_t net_chunk_steps(const g4s_net *n);
 cudaStream_t net_stream(const g4s_net *n);
 int64_t net_steps_done(const g4s_net *n);
 // CTAs of the team the handle's last planned geometry uses (solo or batched), without

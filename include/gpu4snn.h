@@ -123,7 +123,8 @@ int g4s_net_stats(g4s_net *net, double *rate_hz, double *isi_cv, int64_t *total_
  * step t: dv_max[t], dv_p99[t], dv_median[t] = max, 99th and 50th nearest-rank percentile
  * of |v32 - v64| (mV) over all neurons; *first_divergent = first step whose spike sets
  * differ (-1: none); v64_out, u64_out [n] = the twin's final state.  Any output may be
- * NULL.  The network advances by `steps` steps.  Allocates ~41 bytes per neuron. */
+ * NULL.  The network advances by `steps` steps.  Allocates 36 bytes per
+ * neuron and up to 64 MB (8 bytes per neuron if that is more) for the differences. */
 int g4s_net_fp64_check(g4s_net *net, int32_t steps, double *dv_max, double *dv_p99, double *dv_median,
                        int32_t *first_divergent, double *v64_out, double *u64_out);
 /* Grid-barrier time limit of the SKL kernel in ns (default 2 s); 0 makes every barrier
