@@ -189,8 +189,7 @@ struct g4s_net {
   int team_p = 0;
   int64_t team_rc = 0;
   bool team_ready = false;
-  bool team_batch = false;  // geometry planned for a multi-network batch
-  int64_t team_slice = 0;   // ... with this many neurons per CTA
+  int team_batch = 0;       // geometry planned for a multi-network batch with this many CTAs (0: alone)
   bool team_ok = true;
   bool pair_ready = false;  // the packed rows match the tables
   bool pair_fits = false;   // every weight fits a packed word beside its target
@@ -526,7 +525,17 @@ static std::tuple<int, int, int> tune_key(const g4s_net *n, double rate_hz) {
 
 static double recent_rate(const g4s_net *n) {
   const size_t k = std::min<size_t>(n->counts.size(), 200);
-  if (!k) return 8.0;  // no history: assume the balanced regime
+  if (!k) {
+    // no history: the generated networks' rate at this drive (measured on 64 networks of 1,100
+    // to 46,000 neurons, and the same within 10% at 10^6)
+    static const double kDrive[] = {0.5, 0.6, 0.75, 1.0, 1.25, 1.5, 2.0}, kRate[] = {0.1, 0.4, 2.3, 7.5, 12.5, 16.9, 22.0};
+    const double d = n->desc.drive_scale;
+    for (int j = 0; j < 7; ++j)
+      if (d <= kDrive[j])
+        return j == 0 ? kRate[0]
+                      : kRate[j - 1] + (kRate[j] - kRate[j - 1]) * (d - kDrive[j - 1]) / (kDrive[j] - kDrive[j - 1]);
+    return kRate[6];
+  }
   double s = 0;
   for (size_t i = n->counts.size() - k; i < n->counts.size(); ++i) s += n->counts[i];
   return s / (double)k / (double)n->v.n * 1000.0;
@@ -564,7 +573,7 @@ static int resolve_alg(g4s_net *n, int alg) {
 // Returns false if the network does not fit or its tables break the exactness bound of
 // the split accumulation (the global-atomic persistent kernel is used instead).
 // ---------------------------------------------------------------------------------------
-static bool plan_team(g4s_net *n, int want, bool batch, int64_t slice, int *p_out, int64_t *rc_out) {
+static bool plan_team(g4s_net *n, int want, int batch_p, int *p_out, int64_t *rc_out) {
   const NetView &v = n->v;
   if (!n->tables_fit) return false;
   int pmax = 0;
@@ -575,9 +584,8 @@ static bool plan_team(g4s_net *n, int want, bool batch, int64_t slice, int *p_ou
   }
   pmax = std::min(pmax, kMaxTeam);
   // alone, a network spreads over the GPU (one CTA per 128 neurons, up to one per SM); in a
-  // batch it takes one CTA per `slice` neurons (8192 unless the batch is small), so that more
-  // networks run at once
-  int64_t p = want > 0 ? want : (batch ? (v.n + slice - 1) / slice : (v.n + kSoloSlice - 1) / kSoloSlice);
+  // batch it takes the CTAs that the batch's plan gives it
+  int64_t p = want > 0 ? want : batch_p > 0 ? batch_p : (v.n + kSoloSlice - 1) / kSoloSlice;
   if (p < 1) p = 1;
   if (p > pmax) p = pmax;
   int64_t rc = (v.n + p - 1) / p;
@@ -627,15 +635,15 @@ static int prepare_rows(g4s_net *n) {
   return G4S_OK;
 }
 
-// Team geometry, the per-step spike lists and, for teams of more than one CTA, the
-// per-row segment table.
-static int prepare_team(g4s_net *n, bool batch = false, int64_t slice = kBatchSlice) {
-  if (n->team_ready && n->team_batch == batch && (!batch || n->team_slice == slice)) return G4S_OK;
+// Team geometry (in a batch, of batch_p CTAs), the per-step spike lists and, for teams of more
+// than one CTA, the per-row segment table.
+static int prepare_team(g4s_net *n, int batch_p = 0) {
+  if (n->team_ready && n->team_batch == batch_p) return G4S_OK;
   int p = 0;
   int64_t rc = 0;
-  n->team_batch = batch;
-  n->team_slice = slice;
-  if (!plan_team(n, n->want_p, batch, slice, &p, &rc)) {
+  const bool batch = batch_p > 0;
+  n->team_batch = batch_p;
+  if (!plan_team(n, n->want_p, batch_p, &p, &rc)) {
     n->team_ok = false;
     return G4S_OK;
   }
@@ -1175,6 +1183,72 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
   return G4S_OK;
 }
 
+// Estimated device time in us of one step of a network on a team of p CTAs: a chain of round
+// trips, the update and drive of a CTA's neurons, and its share of the step's synapses (by the
+// length of its segments).  Fitted to networks of 1,100 to 10^6 neurons, most within 10%
+// (measured / model: one CTA, 4,189 neurons and 108,000 synapses a step 32 / 40, 1,120 and
+// 24,000 8.9 / 10.8; 8 CTAs, 43,005 and 1.05 million 40 / 39; 152 CTAs, 10^6 and 7.4 million
+// 41 / 41).
+static double team_step_us(const g4s_net *n, double syn, int p) {
+  const double neurons = (double)n->v.n / p, seg = std::max(1.0, (double)n->v.nsyn / p);
+  return p == 1 ? 2.2 + 1.6e-3 * neurons + 0.285e-3 * syn : 3.6 + 1.6e-3 * neurons + (0.19e-3 + 2.2e-3 / seg) * syn / p;
+}
+
+// CTAs of each network of a batch.  At one CTA per kBatchSlice neurons the networks take about
+// their share of a full GPU's time.  Where those teams would leave SMs idle the launch lasts
+// as long as its slowest network, so the CTAs go where the estimated time is: the shortest
+// time for which every network's smallest sufficient team fits one CTA per SM together (64
+// networks of 10^3 to 5 x 10^4 neurons, 16-fold apart in work: 44.3 ms by equal slices, 32.7 so).
+// Teams of an earlier plan are kept while they are within a fifth of that time (a new team has
+// its segment table to build).
+static void plan_batch(g4s_net *const *nets, const int32_t *steps, int count, std::vector<int> &teams) {
+  teams.assign((size_t)count, 1);
+  int gmax = 0;
+  if (team_max_blocks(kTeamSmemLimit, &gmax) != cudaSuccess || gmax < 1) {
+    (void)cudaGetLastError();
+    gmax = 1;
+  }
+  const int pcap = std::min(gmax, kMaxTeam);
+  std::vector<double> syn((size_t)count);
+  int64_t least = 0, held = 0;
+  double held_us = 0.0;
+  bool planned = true;  // every network has a team of an earlier plan
+  for (int i = 0; i < count; ++i) {
+    const g4s_net *n = nets[i];
+    teams[(size_t)i] = (int)std::min<int64_t>(pcap, (n->v.n + kBatchSlice - 1) / kBatchSlice);
+    syn[(size_t)i] = (double)n->v.n * recent_rate(n) * 1e-3 * (double)n->v.nsyn;
+    if (steps[i] <= 0) continue;
+    least += teams[(size_t)i];
+    planned = planned && n->team_ready && n->team_batch > 0;
+    held += n->team_p;
+    if (n->team_p > 0) held_us = std::max(held_us, steps[i] * team_step_us(n, syn[(size_t)i], n->team_p));
+  }
+  if (least >= gmax) return;
+  // the CTAs that network i needs to finish in `us` (more than the GPU has: too many)
+  auto need = [&](int i, double us) {
+    const g4s_net *n = nets[i];
+    const int most = (int)std::min<int64_t>(pcap, (n->v.n + kSoloSlice - 1) / kSoloSlice);
+    int lo = teams[(size_t)i], hi = std::max(lo, most);
+    while (lo < hi && steps[i] * team_step_us(n, syn[(size_t)i], lo) > us) ++lo;
+    return lo;
+  };
+  auto total = [&](double us) {
+    int64_t t = 0;
+    for (int i = 0; i < count && t <= gmax; ++i)
+      if (steps[i] > 0) t += need(i, us);
+    return t;
+  };
+  double lo = 0.0, hi = 0.0;
+  for (int i = 0; i < count; ++i) hi = std::max(hi, steps[i] * team_step_us(nets[i], syn[(size_t)i], teams[(size_t)i]));
+  for (int k = 0; k < 24; ++k) {
+    const double mid = 0.5 * (lo + hi);
+    (total(mid) <= gmax ? hi : lo) = mid;
+  }
+  const bool keep = planned && held <= gmax && held_us <= 1.2 * hi;
+  for (int i = 0; i < count; ++i)
+    if (steps[i] > 0) teams[(size_t)i] = keep ? nets[i]->team_batch : need(i, hi);
+}
+
 // Several networks advanced together by the SKL team kernel: network i runs steps[i]
 // further steps; each round advances every unfinished network by up to its chunk length
 // in one persistent launch.
@@ -1182,36 +1256,15 @@ static int run_nets(g4s_net *const *nets, const int32_t *steps, int count, doubl
   if (count <= 0) return set_error(G4S_ERR_INVALID, "count must be > 0");
   for (int i = 0; i < count; ++i)
     if (!nets[i]) return set_error(G4S_ERR_INVALID, "null handle in batch");
-  // Neurons per CTA of the batch: kBatchSlice, unless the teams that gives leave SMs idle
-  // (few networks, as at a server's start and end): then the smallest slice of a fixed
-  // ladder (half octaves down to a lone network's), whose teams still fit one CTA per SM
-  // together.  (A ladder, so that a network's team, and its segment table, change only when
-  // the batch changes by a factor.)
-  static const int64_t kSlices[] = {kBatchSlice, 6144, 4096, 3072, 2048, 1536, 1024, 768, 512, 384, 256, 192, kSoloSlice};
-  int64_t slice = kBatchSlice;
-  if (count > 1) {
-    int gmax = 0;
-    if (team_max_blocks(kTeamSmemLimit, &gmax) != cudaSuccess || gmax < 1) {
-      (void)cudaGetLastError();
-      gmax = 0;
-    }
-    const int64_t pcap = std::min(gmax, kMaxTeam);
-    auto slots = [&](int64_t sl) {
-      int64_t t = 0;
-      for (int i = 0; i < count; ++i)
-        if (steps[i] > 0) t += std::min(pcap, (nets[i]->v.n + sl - 1) / sl);
-      return t;
-    };
-    for (size_t k = 1; gmax > 0 && k < sizeof(kSlices) / sizeof(kSlices[0]) && slots(kSlices[k]) <= gmax; ++k)
-      slice = kSlices[k];
-  }
+  std::vector<int> teams;
+  if (count > 1) plan_batch(nets, steps, count, teams);
   std::vector<int64_t> remaining(count);
   for (int i = 0; i < count; ++i) {
     if (steps[i] < 0 || nets[i]->t_abs + steps[i] > (int64_t)INT32_MAX)
       return set_error(G4S_ERR_INVALID, "bad step count in batch");
     for (int j = 0; j < i; ++j)
       if (nets[j] == nets[i]) return set_error(G4S_ERR_INVALID, "a handle appears twice in the batch");
-    int rc = prepare_team(nets[i], count > 1, slice);
+    int rc = prepare_team(nets[i], count > 1 ? teams[(size_t)i] : 0);
     if (rc) return rc;
     if (!nets[i]->team_ok)
       return set_error(G4S_ERR_INVALID, "a network of the batch does not fit the team kernel");

@@ -44,9 +44,8 @@ constexpr int64_t kAbcdSlice = 2048;           // ... keep a, b, c, d in shared 
 constexpr int64_t kSoloSlice = 128;            // neurons per CTA of a network running alone (at
                                                // most: it spreads over every SM; measured best from
                                                // N = 2500 to 10^6)
-constexpr int64_t kBatchSlice = 8192;          // neurons per CTA of a batched network (measured on the
-                                               // 256-network ensemble: 510 ms against 534 at 4096 and
-                                               // 824 at 16384; served requests 41.9/s, 40.1, 32.7)
+constexpr int64_t kBatchSlice = 8192;          // neurons per CTA of a network in a batch that fills the
+                                               // GPU (the 256-network ensemble: 364 ms)
 constexpr int kStateBlock = 65536;             // neurons of the state read back at a time
 constexpr int kStateThreadBlocks = 3;          // ... in this many blocks or more, a thread per field
 constexpr int kMaxTeam = 176;                  // CTAs of one team (eight source ranks a warp, 22 such warps)

@@ -62,6 +62,8 @@
 #include <algorithm>
 #include <climits>
 #include <cstdint>
+#include <map>
+#include <mutex>
 
 #include "g4s_device.cuh"
 #include "g4s_internal.h"
@@ -1164,19 +1166,28 @@ cudaError_t team_smem_ceiling() {
 
 cudaError_t team_max_blocks(size_t smem, int *out, int nt) {
   if (smem > kTeamSmemLimit || (nt != kTeamNT && nt != kTeamNTSmall)) return cudaErrorInvalidValue;
-  cudaError_t e = team_smem_ceiling();
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  int least = INT_MAX;  // (of the instantiations, which need nearly the same resources)
-  for (int k = 0; k < kTeamVariants; ++k) {
-    int occ = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, team_variant(nt, k), nt, smem);
-    if (e != cudaSuccess) return e;
-    least = std::min(least, occ);
+  // Constants of the device (a CTA's registers leave room for one per SM, whatever its shared
+  // memory): asked for once, a batch plans with them once per network.
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, int> known;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = known.find({dev, nt});
+  if (it == known.end()) {
+    if ((e = team_smem_ceiling()) != cudaSuccess) return e;
+    int least = INT_MAX, sms = 1;  // (of the instantiations, which need nearly the same resources)
+    for (int k = 0; k < kTeamVariants; ++k) {
+      int occ = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, team_variant(nt, k), nt, kTeamSmemLimit);
+      if (e != cudaSuccess) return e;
+      least = std::min(least, occ);
+    }
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    it = known.emplace(std::make_pair(dev, nt), least * sms).first;
   }
-  int dev = 0, sms = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  *out = least * sms;
+  *out = it->second;
   return cudaSuccess;
 }
 
