@@ -15,11 +15,12 @@
 // neurons per CTA (the shared-memory slice of the team kernel).  Every call shares the
 // scratch array and leaves its contents behind; calls that overlap on the GPU (on
 // different streams, or without ordering between them) race on it and must not be made.
-// A multi-CTA call rebuilds the per-row segment table from the caller's tables (a binary
-// search of every row per team boundary, reading about team x log2(stride) targets a row),
+// A multi-CTA call rebuilds the per-row segment table from the caller's tables (a search of
+// every row, reading 32 targets and 32 per team boundary of a row of 1000),
 // since it cannot know whether they changed since the last call.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <mutex>
@@ -39,7 +40,7 @@ constexpr int64_t kNoAllocMaxSlice = 16384;
 // Layout of the scratch array.
 constexpr size_t kOffSync = 0;                                       // GridSync (128 B): error word
 constexpr size_t kOffRec = 128;                                      // spike records: [2][team][4 x 16] u64
-constexpr size_t kOffCtl = kOffRec + 2 * kNoAllocMaxTeam * kRecLines * 128;  // int[4]: slot count, queue head, status
+constexpr size_t kOffCtl = kOffRec + 2 * kNoAllocMaxTeam * kRecLines * 128;  // int[5]: slot count, queue head, status, -, next tag
 constexpr size_t kOffSlots = kOffCtl + 128;                          // int2[kNoAllocMaxTeam]
 constexpr size_t kOffItem = kOffSlots + 256;                         // TeamItem
 constexpr size_t kOffList = 16384;                                   // u64[4][kNoAllocMaxNeurons]: overflow, dense ids
@@ -53,17 +54,83 @@ static_assert(kNoAllocMaxTeam <= 32, "one setup thread per slot");
 // about 6.5 MB: the documented size of the array in gpu4snn.h
 static_assert(kScratchBytes > 6400000 && kScratchBytes < 6600000, "scratch size as documented");
 
-// Writes the work-queue words, the team's slots and the launch descriptor into the
-// scratch array.  The descriptor arrives by value as a kernel argument, so the call stages
-// nothing through host memory.
-__global__ void k_noalloc_setup(TeamItem item, int *ctl, int2 *slots, TeamItem *dst) {
-  const int r = threadIdx.x;
-  if (r < item.team) slots[r] = make_int2(0, r);
-  if (r == 0) {
-    ctl[0] = item.team;  // slots in the queue
-    ctl[1] = 0;          // queue head
-    ctl[2] = 0;          // status word
-    *dst = item;
+// Everything a call needs before the team kernel, in one launch: the work-queue words, the
+// team's slots and the launch descriptor (which arrives by value as a kernel argument, so the
+// call stages nothing through host memory), cleared counts, status and error words, and the
+// team's segment table.  The records and id lists keep the words of earlier calls: their tags
+// go on from call to call (a device word, so that a captured call replays), and no stale word
+// carries a tag that is still to come; they are cleared when the tags would wrap.  (As three
+// memsets, two kernels and a copy of the status word these took 20 us of a 34 us call of one
+// step of N=2,500.)
+//
+// Segment table, a warp per row: 32 probes at a time narrow every boundary's range 32-fold, the
+// first probes shared by all of them (rows of 1000: two dependent loads in place of ten).
+constexpr int kSetupNT = 256;
+__global__ void __launch_bounds__(kSetupNT) k_noalloc_setup(TeamItem item, int *ctl, int2 *slots, TeamItem *dst,
+                                                            uint16_t *seg, int64_t scratch_words) {
+  const int T = item.team;
+  if (blockIdx.x == 0) {
+    __shared__ unsigned s_tag;
+    __shared__ int s_wrap;
+    if (threadIdx.x == 0) {
+      unsigned *next = reinterpret_cast<unsigned *>(ctl + 4);
+      s_wrap = (unsigned long long)*next + (unsigned)item.steps + 2ull >= 0xFFFFFFFFull;
+      s_tag = s_wrap ? 0u : *next;
+      *next = s_tag + (unsigned)item.steps;
+      ctl[0] = T;  // slots in the queue
+      ctl[1] = 0;  // queue head
+      *item.v.status = 0;
+      item.sync->error = 0;
+      item.tag0 = s_tag;
+      *dst = item;
+    }
+    if ((int)threadIdx.x < T) slots[threadIdx.x] = make_int2(0, (int)threadIdx.x);
+    __syncthreads();
+    if (s_wrap) {
+      for (int k = threadIdx.x; k < 2 * kNoAllocMaxTeam * kRecLines * kRecWords; k += kSetupNT) item.rec[k] = 0ull;
+      for (int64_t k = threadIdx.x; k < scratch_words; k += kSetupNT) item.list[k] = 0ull;
+    }
+  }
+  for (int k = blockIdx.x * kSetupNT + threadIdx.x; k < item.steps; k += gridDim.x * kSetupNT) item.v.counts[k] = 0;
+  if (T == 1) return;
+  const int lane = threadIdx.x & 31, stride = item.v.stride;
+  const int64_t nwarps = (int64_t)gridDim.x * (kSetupNT / 32);
+  for (int64_t row = (int64_t)blockIdx.x * (kSetupNT / 32) + (threadIdx.x >> 5); row < item.v.n; row += nwarps) {
+    const unsigned *ri = reinterpret_cast<const unsigned *>(item.v.idx) + row * stride;
+    int lo[kNoAllocMaxTeam], len[kNoAllocMaxTeam];  // where boundary k + 1 lies
+    const int step0 = (stride + 31) >> 5;
+    const unsigned t0 = lane * step0 < stride ? ri[lane * step0] : 0xFFFFFFFFu;
+    int most = 0;
+#pragma unroll
+    for (int k = 0; k < kNoAllocMaxTeam; ++k) {
+      const int c = __popc(__ballot_sync(0xFFFFFFFFu, t0 < (unsigned)(k + 1) * (unsigned)item.rc));
+      lo[k] = c ? (c - 1) * step0 + 1 : 0;
+      len[k] = c && k < T ? min(stride, c * step0) - lo[k] : 0;
+      most = max(most, len[k]);
+    }
+    while (most > 0) {
+      most = 0;
+      unsigned t[kNoAllocMaxTeam];
+#pragma unroll
+      for (int k = 0; k < kNoAllocMaxTeam; ++k) {
+        const int at = lane * ((len[k] + 31) >> 5);
+        t[k] = at < len[k] ? ri[lo[k] + at] : 0xFFFFFFFFu;
+      }
+#pragma unroll
+      for (int k = 0; k < kNoAllocMaxTeam; ++k) {
+        const int step = (len[k] + 31) >> 5;
+        const int c = __popc(__ballot_sync(0xFFFFFFFFu, t[k] < (unsigned)(k + 1) * (unsigned)item.rc));
+        const int end = c ? min(lo[k] + len[k], lo[k] + c * step) : lo[k];
+        if (c) lo[k] += (c - 1) * step + 1;
+        len[k] = end - lo[k];
+        most = max(most, len[k]);
+      }
+    }
+    uint16_t *so = seg + row * (T + 1);
+    if (lane == 0) so[0] = 0;
+#pragma unroll
+    for (int k = 0; k < kNoAllocMaxTeam; ++k)
+      if (lane == k && k < T) so[k + 1] = (uint16_t)lo[k];
   }
 }
 
@@ -153,30 +220,24 @@ extern "C" int g4s_run_noalloc(const g4s_dev_net *d, int64_t t_abs0, int32_t ste
   v.counts = d_counts;
   v.base = reinterpret_cast<long long *>(d_base);
   v.stamps = nullptr;
-  v.status = ctl + 2;
+  v.status = d_status ? d_status : ctl + 2;
   h.seg = seg;
   h.list = list;
   h.rec = reinterpret_cast<unsigned long long *>(scr + kOffRec);
-  h.tag0 = 0;
   h.t_abs0 = t_abs0;
   h.steps = steps;
   h.last = last ? 1 : 0;
   h.team = team;
   h.rc = (int)rc;
   h.sync = sync;
-  // Everything that must start at zero: error word, spike records and overflow ids (their
-  // tags restart with every call), step counts; then the queue words and the descriptor.
-  cudaError_t e = cudaMemsetAsync(scr, 0, kOffSlots, s);
-  if (e == cudaSuccess && team > 1) e = cudaMemsetAsync(list, 0, (size_t)d->n * 2 * sizeof(unsigned long long), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_counts, 0, (size_t)steps * sizeof(int32_t), s);
-  if (e == cudaSuccess) {
-    k_noalloc_setup<<<1, 32, 0, s>>>(h, ctl, slots, item);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess && team > 1) e = launch_segoff(v, team, rc, seg, s);
+  const int64_t rows = team > 1 ? (d->n + kSetupNT / 32 - 1) / (kSetupNT / 32) : 1;
+  k_noalloc_setup<<<(unsigned)std::min<int64_t>(rows, 152 * 16), kSetupNT, 0, s>>>(h, ctl, slots, item, seg,
+                                                                                    2 * kNoAllocMaxNeurons);
+  cudaError_t e = cudaGetLastError();
+  // (768 threads for slices whose state lives in shared memory, as for small steps elsewhere)
   if (e == cudaSuccess)
-    e = launch_team(item, slots, ctl, ctl + 1, team, team_smem(rc, team), 2000000000ull, 0, s, false, kDeliverRun, team == 1);
-  if (e == cudaSuccess && d_status) e = cudaMemcpyAsync(d_status, &sync->error, sizeof(int32_t), cudaMemcpyDeviceToDevice, s);
+    e = launch_team(item, slots, ctl, ctl + 1, team, team_smem(rc, team), 2000000000ull, 0, s, false, kDeliverRun, team == 1,
+                    rc <= kVuSlice ? kTeamNTSmall : kTeamNT);
   if (e != cudaSuccess) return cuda_error(e, "g4s_run_noalloc launch");
   return G4S_OK;
 }

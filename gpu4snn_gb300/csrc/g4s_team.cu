@@ -446,13 +446,13 @@ constexpr int kInline = kRankWords - 1;
 constexpr int kLine1After = 7;  // line 1 of a rank is polled if it had more spikes in the previous step
 
 // Gives up a wait: first error wins, every CTA of the team leaves at its next check.
-__device__ __forceinline__ void give_up(TeamShared &sh, GridSync *gs) {
-  atomicCAS(&gs->error, 0, kErrTimeoutCode);
+__device__ __forceinline__ void give_up(const TeamItem &it, TeamShared &sh) {
+  if (atomicCAS(&it.sync->error, 0, kErrTimeoutCode) == 0) *(volatile int *)it.v.status = kErrTimeoutCode;
   *(volatile int *)&sh.fail = 1;
 }
 
 // One tagged word of another rank, polled until it carries `tag` (or the time limit).
-__device__ __forceinline__ int tagged_id(const unsigned long long *p, unsigned tag, TeamShared &sh, GridSync *gs,
+__device__ __forceinline__ int tagged_id(const unsigned long long *p, unsigned tag, const TeamItem &it, TeamShared &sh,
                                          unsigned long long lim) {
   unsigned long long w = ld_relaxed_u64(p);
   if ((unsigned)(w >> 32) == tag) return (int)(unsigned)w;
@@ -460,8 +460,8 @@ __device__ __forceinline__ int tagged_id(const unsigned long long *p, unsigned t
   for (;;) {
     w = ld_relaxed_u64(p);
     if ((unsigned)(w >> 32) == tag) return (int)(unsigned)w;
-    if (*(volatile int *)&sh.fail || ld_relaxed(&gs->error) != 0 || globaltimer() - t0 > lim) {
-      give_up(sh, gs);
+    if (*(volatile int *)&sh.fail || ld_relaxed(&it.sync->error) != 0 || globaltimer() - t0 > lim) {
+      give_up(it, sh);
       return 0;
     }
   }
@@ -469,16 +469,16 @@ __device__ __forceinline__ int tagged_id(const unsigned long long *p, unsigned t
 
 // One round of a poll's checks by a warp whose words are not all there yet (t0: the poll's
 // start, set in round 0): true when the wait is given up.
-__device__ __forceinline__ bool poll_check(TeamShared &sh, GridSync *gs, int iter, unsigned long long &t0,
+__device__ __forceinline__ bool poll_check(const TeamItem &it, TeamShared &sh, int iter, unsigned long long &t0,
                                            unsigned long long lim) {
   int f = 0;
   if ((threadIdx.x & 31) == 0) {
     const unsigned long long now = globaltimer();
     if (iter == 0) t0 = now;
     f = *(volatile int *)&sh.fail;
-    if (!f && threadIdx.x == 0 && ld_relaxed(&gs->error) != 0) f = 1;
+    if (!f && threadIdx.x == 0 && ld_relaxed(&it.sync->error) != 0) f = 1;
     if (!f && now - t0 > lim) {
-      give_up(sh, gs);
+      give_up(it, sh);
       f = 1;
     }
     if (f) *(volatile int *)&sh.fail = 1;
@@ -532,7 +532,7 @@ __device__ __forceinline__ void fetch_spike(const TeamItem &it, TeamShared &sh, 
       const int par = c.lt & 1;
       s = tagged_id(j < kInline ? it.rec + ((size_t)par * it.team + r) * kRankWords + 1 + j
                                 : it.list + (size_t)par * it.v.n + (size_t)r * it.rc + j,
-                    it.tag0 + (unsigned)c.lt + 1u, sh, it.sync, sh.lim);
+                    it.tag0 + (unsigned)c.lt + 1u, it, sh, sh.lim);
     }
     const uint16_t *so = it.seg + (size_t)s * (unsigned)(it.team + 1) + sh.rank;
     b = ld_keep_u16(so, pkeep);
@@ -933,7 +933,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
         const unsigned long long lim = sh.lim, t0 = globaltimer();
         while (ld_relaxed(&it.sync->error) == 0 && globaltimer() - t0 <= lim) {
         }
-        give_up(sh, it.sync);
+        give_up(it, sh);
       }
       __syncthreads();
       return;
@@ -1000,7 +1000,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
             }
           }
           if (__all_sync(0xFFFFFFFFu, need == 0) && stall == 0) break;
-          if (poll_check(sh, it.sync, iter, t0, sh.lim)) break;
+          if (poll_check(it, sh, iter, t0, sh.lim)) break;
         }
         __syncwarp();
         if (lane < n_src) cl = (int)s_pay()[(warp + lane * kSrc) * kRankWords];
@@ -1014,7 +1014,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
             cl = lane < n_src ? (int)(unsigned)w : 0;
             break;
           }
-          if (poll_check(sh, it.sync, iter, t0, sh.lim)) break;
+          if (poll_check(it, sh, iter, t0, sh.lim)) break;
         }
       }
       {
