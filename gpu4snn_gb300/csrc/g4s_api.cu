@@ -54,13 +54,13 @@ int cuda_error(cudaError_t e, const char *what) {
   } while (0)
 
 // Buffers of the launches of one handle, or of one thread's batches: what a round uploads
-// (descriptors, the networks' places in the pack, queue slots, control words: one copy) and
+// (descriptors, the networks' places in the pack, queue slots and head: one copy) and
 // the pack that it brings back, each side one allocation.
 struct TeamLaunch {
   unsigned char *d_mem = nullptr, *h_mem = nullptr;
   size_t cap = 0;
   // the round's parts, at the same offsets on both sides
-  size_t o_off = 0, o_slots = 0, o_ctl = 0, o_pack = 0;
+  size_t o_off = 0, o_slots = 0, o_head = 0, o_pack = 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   std::vector<int> order;  // networks of the round in flight (team_round_start .. finish)
   std::vector<g4s_net *> nets;
@@ -85,8 +85,8 @@ struct TeamLaunch {
       return set_error(G4S_ERR_CUDA, "team launch events");
     o_off = sizeof(TeamItem) * (size_t)items;
     o_slots = o_off + sizeof(int64_t) * (size_t)items;
-    o_ctl = o_slots + sizeof(int2) * (size_t)slots;
-    o_pack = (o_ctl + 16 + 15) / 16 * 16;
+    o_head = o_slots + sizeof(int2) * (size_t)slots;
+    o_pack = (o_head + 16 + 15) / 16 * 16;
     const size_t bytes = o_pack + pack;
     if (bytes <= cap) return G4S_OK;
     cudaFree(d_mem);
@@ -102,7 +102,7 @@ struct TeamLaunch {
   TeamItem *items(unsigned char *m) const { return reinterpret_cast<TeamItem *>(m); }
   int64_t *off(unsigned char *m) const { return reinterpret_cast<int64_t *>(m + o_off); }
   int2 *slots(unsigned char *m) const { return reinterpret_cast<int2 *>(m + o_slots); }
-  int *ctl(unsigned char *m) const { return reinterpret_cast<int *>(m + o_ctl); }  // slot count, queue head
+  int *head(unsigned char *m) const { return reinterpret_cast<int *>(m + o_head); }  // queue head
 };
 static_assert(sizeof(TeamItem) % 8 == 0, "the upload's parts follow one another");
 
@@ -1001,8 +1001,7 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
   }
   for (int i = 0; i < count; ++i)
     if (steps[i] <= 0) L.items(L.h_mem)[i].steps = 0;
-  L.ctl(L.h_mem)[0] = nslots;
-  L.ctl(L.h_mem)[1] = 0;
+  *L.head(L.h_mem) = 0;
   L.nets.assign(nets, nets + count);
   L.steps.assign(steps, steps + count);
   // One copy up, one kernel clearing every network's words of the launch, the team kernel
@@ -1013,7 +1012,7 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
   G4S_CUDA(cudaMemcpyAsync(L.d_mem, L.h_mem, L.o_pack, cudaMemcpyHostToDevice, s));
   G4S_CUDA(launch_round_clear(L.items(L.d_mem), count, s));
   G4S_CUDA(cudaEventRecord(L.e0, s));
-  G4S_CUDA(launch_team(L.items(L.d_mem), L.slots(L.d_mem), L.ctl(L.d_mem), L.ctl(L.d_mem) + 1, grid, smem, limit_ns,
+  G4S_CUDA(launch_team(L.items(L.d_mem), L.slots(L.d_mem), nslots, L.head(L.d_mem), grid, smem, limit_ns,
                        stall, s, pair, mode, solo, nt));
   G4S_CUDA(cudaEventRecord(L.e1, s));
   G4S_CUDA(launch_round_gather(L.items(L.d_mem), L.off(L.d_mem), count, L.d_mem + L.o_pack, s));

@@ -119,7 +119,8 @@ constexpr int kTeamNTSmall = 768;
 // pair: the tables are read from v.pair (packed words) instead of v.idx and v.w;
 // mode: delivery mapping of the launch's multi-CTA teams (kDeliverRun or kDeliverGroup);
 // solo: the launch has one-CTA teams; nt: kTeamNT or kTeamNTSmall threads per CTA
-cudaError_t launch_team(const TeamItem *items, const int2 *slots, const int *nslots, int *slot_head, int grid,
+// slot_head: device word, 0 at launch (the queue's slots beyond the grid)
+cudaError_t launch_team(const TeamItem *items, const int2 *slots, int nslots, int *slot_head, int grid,
                         size_t smem, unsigned long long limit_ns, int stall, cudaStream_t s, bool pair, int mode,
                         bool solo, int nt = kTeamNT);
 // v.pair <- the rows of v.idx and v.w as packed words (after every change of the tables)

@@ -40,7 +40,7 @@ constexpr int64_t kNoAllocMaxSlice = 16384;
 // Layout of the scratch array.
 constexpr size_t kOffSync = 0;                                       // GridSync (128 B): error word
 constexpr size_t kOffRec = 128;                                      // spike records: [2][team][4 x 16] u64
-constexpr size_t kOffCtl = kOffRec + 2 * kNoAllocMaxTeam * kRecLines * 128;  // int[5]: slot count, queue head, status, -, next tag
+constexpr size_t kOffCtl = kOffRec + 2 * kNoAllocMaxTeam * kRecLines * 128;  // int[5]: -, queue head, status, -, next tag
 constexpr size_t kOffSlots = kOffCtl + 128;                          // int2[kNoAllocMaxTeam]
 constexpr size_t kOffItem = kOffSlots + 256;                         // TeamItem
 constexpr size_t kOffList = 16384;                                   // u64[4][kNoAllocMaxNeurons]: overflow, dense ids
@@ -77,7 +77,6 @@ __global__ void __launch_bounds__(kSetupNT) k_noalloc_setup(TeamItem item, int *
       s_wrap = (unsigned long long)*next + (unsigned)item.steps + 2ull >= 0xFFFFFFFFull;
       s_tag = s_wrap ? 0u : *next;
       *next = s_tag + (unsigned)item.steps;
-      ctl[0] = T;  // slots in the queue
       ctl[1] = 0;  // queue head
       *item.v.status = 0;
       item.sync->error = 0;
@@ -236,7 +235,7 @@ extern "C" int g4s_run_noalloc(const g4s_dev_net *d, int64_t t_abs0, int32_t ste
   cudaError_t e = cudaGetLastError();
   // (768 threads for slices whose state lives in shared memory, as for small steps elsewhere)
   if (e == cudaSuccess)
-    e = launch_team(item, slots, ctl, ctl + 1, team, team_smem(rc, team), 2000000000ull, 0, s, false, kDeliverRun, team == 1,
+    e = launch_team(item, slots, team, ctl + 1, team, team_smem(rc, team), 2000000000ull, 0, s, false, kDeliverRun, team == 1,
                     rc <= kVuSlice ? kTeamNTSmall : kTeamNT);
   if (e != cudaSuccess) return cuda_error(e, "g4s_run_noalloc launch");
   return G4S_OK;

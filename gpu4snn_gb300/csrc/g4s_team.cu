@@ -1099,26 +1099,25 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
   __syncthreads();
 }
 
-// The persistent grid: CTAs take (network, rank) slots until the queue is empty.
+// The persistent grid: CTA b takes (network, rank) slot b, then the next ones of the queue
+// until it is empty (a launch whose slots all fit the grid makes no trip to the queue head).
 template <int NT, bool kPair, int kMode, bool kSolo>
 __global__ void __launch_bounds__(NT, 1) k_team(const TeamItem *__restrict__ items, const int2 *__restrict__ slots,
-                                                const int *nslots, int *slot_head, unsigned long long limit_ns,
-                                                int stall) {
+                                                int nslots, int *slot_head, unsigned long long limit_ns, int stall) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   __shared__ TeamShared sh;
-  const int ns = *nslots;
-  for (;;) {
-    if (threadIdx.x == 0) sh.slot = atomicAdd(slot_head, 1);
-    __syncthreads();
-    const int sl = sh.slot;
-    __syncthreads();
-    if (sl >= ns) break;
+  // the network's descriptor in shared memory: read on every step's dependent chains
+  __shared__ TeamItem s_it;
+  for (int sl = blockIdx.x; sl < nslots;) {
     const int2 x = slots[sl];
-    // the network's descriptor in shared memory: read on every step's dependent chains
-    __shared__ TeamItem s_it;
-    if (threadIdx.x == 0) s_it = items[x.x];
+    for (unsigned k = threadIdx.x; k < sizeof(TeamItem) / 8; k += NT)
+      reinterpret_cast<unsigned long long *>(&s_it)[k] = reinterpret_cast<const unsigned long long *>(items + x.x)[k];
     __syncthreads();
     if (s_it.steps > 0) team_run<NT, kPair, kMode, kSolo>(s_it, x.y, s_raw, sh, limit_ns, stall);
+    if (nslots <= (int)gridDim.x) break;
+    if (threadIdx.x == 0) sh.slot = (int)gridDim.x + atomicAdd(slot_head, 1);
+    __syncthreads();
+    sl = sh.slot;
     __syncthreads();
   }
 }
@@ -1134,7 +1133,7 @@ size_t team_smem(int64_t rc, int team) {
 }
 
 // The instantiation of the team kernel for a CTA size, table layout and delivery mapping.
-using TeamKernel = void (*)(const TeamItem *, const int2 *, const int *, int *, unsigned long long, int);
+using TeamKernel = void (*)(const TeamItem *, const int2 *, int, int *, unsigned long long, int);
 template <int NT, bool kPair, int kMode>
 static TeamKernel team_kernel_of(bool solo) {
   return solo ? k_team<NT, kPair, kMode, true> : k_team<NT, kPair, kMode, false>;
@@ -1191,7 +1190,7 @@ cudaError_t team_max_blocks(size_t smem, int *out, int nt) {
   return cudaSuccess;
 }
 
-cudaError_t launch_team(const TeamItem *items, const int2 *slots, const int *nslots, int *slot_head, int grid,
+cudaError_t launch_team(const TeamItem *items, const int2 *slots, int nslots, int *slot_head, int grid,
                         size_t smem, unsigned long long limit_ns, int stall, cudaStream_t s, bool pair, int mode,
                         bool solo, int nt) {
   if (smem > kTeamSmemLimit || (nt != kTeamNT && nt != kTeamNTSmall)) return cudaErrorInvalidValue;
