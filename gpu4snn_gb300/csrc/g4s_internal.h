@@ -97,6 +97,7 @@ __host__ __device__ inline TeamLayout team_layout(int64_t rc, int team) {
 // (-1, 0.0f)), which a narrower key sorts into the same order.
 cudaError_t launch_sort_rows(const NetView &v, bool generated, cudaStream_t s);
 // *unsorted <- 1 if some row is not in launch_sort_rows' order, else 0
+cudaError_t launch_first_bad(const int *idx, const NetView &v, unsigned long long *first, cudaStream_t s);
 cudaError_t launch_rows_sorted(const NetView &v, int *unsorted, cudaStream_t s);
 // A launch over many networks: clear (before it) and pack (after it) every network's
 // per-launch words; network i's share of the pack is round_pack_bytes(steps_i) bytes at

@@ -253,6 +253,19 @@ __global__ void k_rows_sorted(NetView v, int *unsorted) {
   if (__any_sync(0xFFFFFFFFu, bad) && lane == 0) *unsorted = 1;
 }
 
+// First slot of `idx` (a table of v's shape) that targets neuron n or a later one, into
+// *first (~0 at launch: none); four slots a thread, bound by memory.
+__global__ void k_first_bad(const int4 *idx, NetView v, unsigned long long *first) {
+  const int64_t quads = v.n * (int64_t)(v.stride >> 2);
+  unsigned long long mine = ~0ull;
+  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < quads; g += (int64_t)gridDim.x * blockDim.x) {
+    const int4 t = __ldcs(idx + g);
+    const int bad = t.x >= v.n ? 0 : t.y >= v.n ? 1 : t.z >= v.n ? 2 : t.w >= v.n ? 3 : 4;
+    if (bad < 4 && mine == ~0ull) mine = 4ull * (unsigned long long)g + (unsigned long long)bad;
+  }
+  if (mine != ~0ull) atomicMin(first, mine);
+}
+
 // Segment table: seg[row][k] = first slot of the sorted row whose target is >= k*Rc, for
 // k = 0..T (unused slots compare as huge and lie beyond seg[row][T]).  One warp per row,
 // one binary search per boundary.
@@ -1286,6 +1299,16 @@ cudaError_t launch_rows_sorted(const NetView &v, int *unsorted, cudaStream_t s) 
   cudaError_t e = cudaMemsetAsync(unsorted, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
   k_rows_sorted<<<(unsigned)(sms * 8), 512, 0, s>>>(v, unsorted);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_first_bad(const int *idx, const NetView &v, unsigned long long *first, cudaStream_t s) {
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaError_t e = cudaMemsetAsync(first, 0xFF, 8, s);
+  if (e != cudaSuccess) return e;
+  k_first_bad<<<(unsigned)(sms * 4), 512, 0, s>>>(reinterpret_cast<const int4 *>(idx), v, first);
   return cudaGetLastError();
 }
 

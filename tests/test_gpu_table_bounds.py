@@ -22,3 +22,32 @@ def test_bound(g4s, n, into, weight, fits):
             net.load_tables(idx, w)
             net.run(1)
             assert (net.geometry()[0] >= 1) == fits
+
+
+@pytest.mark.parametrize("ran", [False, True])
+@pytest.mark.parametrize("n,nsyn", [(7001, 9), (21846, 3), (20001, 300)])
+def test_refused_upload_keeps_the_tables(g4s, oracle, n, nsyn, ran):
+    """Uploads checked on the device (65,536 slots or more), before and after the packed rows
+    exist: the first offending slot is named, the network runs on as if there had been no
+    upload, and the same call with good tables is taken."""
+    d = oracle.make_desc(n, nsyn, 21, drive_scale=2.0)
+    idx, w = oracle.conn_philox(d)
+    sim = oracle.Sim(d, idx, w)
+    sim.run(40, threads=8)
+    with g4s.Network(n, nsyn, seed=21, drive_scale=2.0) as net:
+        own = net.tables()
+        net.run(20 if ran else 0)
+        for pos in (0, 3, idx.size // 2 + 1, idx.size - 1):
+            bad = np.where(own[0] < 0, -5, n - 1).astype(np.int32)
+            bad.flat[pos] = n
+            bad.flat[idx.size - 1] = np.iinfo(np.int32).max
+            with pytest.raises(g4s.G4SError) as e:
+                net.load_tables(bad, np.zeros_like(own[1]))
+            assert f"table entry {pos} targets neuron {bad.flat[pos]} " in str(e.value)
+        net.run(20 if ran else 40)
+        assert np.array_equal(np.stack(net.raster()), np.stack(sim.raster()))
+        net.load_tables(idx, w)
+        net.reset()
+        net.run(40)
+        assert np.array_equal(np.stack(net.raster()), np.stack(sim.raster()))
+        assert all(np.array_equal(a, b) for a, b in zip(own, net.tables()))
