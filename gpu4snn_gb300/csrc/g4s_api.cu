@@ -566,8 +566,25 @@ static int resolve_alg(g4s_net *n, int alg) {
 }
 
 // ---------------------------------------------------------------------------------------
+// CTAs of a network running alone: one up to kLoneNeurons, whose steps are then free of the
+// exchange (us per step with one CTA, one per 128 neurons and 12 CTAs: N=256 x 50 2.10, 2.98,
+// 2.70; 600 x 500 2.77, 3.75, 3.40, at drive 2 3.51, 3.90, 3.59; 800 x 500 at drive 2 4.26, 4.03,
+// 3.68); above, one per 52 neurons, as steps are bound by the longest chain of a rank and not by
+// its work (with one per 128 and per 52: N=1,000 x 500 3.89, 3.54; 2,500 x 1000 3.82, 3.66 and
+// 4.24, 3.85 at drive 2; 5,000 x 1000 4.09, 3.82), not below the size from which every warp
+// polls source ranks of its own (N=800 x 50 with 7 CTAs 3.57, 12 2.88), and as many as it takes,
+// where that is possible, for segments short enough to be walked as runs (N=2,500 x 2000 with
+// 77 CTAs 3.92, 88 3.72; 11,000 x 2000 5.15, 4.48).
+constexpr int64_t kLoneNeurons = 640, kLoneSlice = 52;
+static int64_t lone_team(int64_t n, int64_t nsyn, int64_t pmax) {
+  if (n <= kLoneNeurons) return 1;
+  const int64_t p = std::max<int64_t>(kOwnSources, (n + kLoneSlice - 1) / kLoneSlice);
+  const int64_t runs = nsyn / kGroupMinSegment + 1;
+  return runs <= pmax ? std::max(p, runs) : p;
+}
+
 // Team geometry of one network for the SKL team kernel: p CTAs (at most the co-resident
-// count, one per SM), by default one per 128 neurons alone and one per 8192 in a batch,
+// count, one per SM), by default lone_team's alone and the batch plan's in a batch,
 // and the currents plus the spike buffer of a slice within the shared-memory limit.
 // Returns false if the network does not fit or its tables break the exactness bound of
 // the split accumulation (the global-atomic persistent kernel is used instead).
@@ -582,9 +599,7 @@ static bool plan_team(g4s_net *n, int want, int batch_p, int *p_out, int64_t *rc
     return false;
   }
   pmax = std::min(pmax, kMaxTeam);
-  // alone, a network spreads over the GPU (one CTA per 128 neurons, up to one per SM); in a
-  // batch it takes the CTAs that the batch's plan gives it
-  int64_t p = want > 0 ? want : batch_p > 0 ? batch_p : (v.n + kSoloSlice - 1) / kSoloSlice;
+  int64_t p = want > 0 ? want : batch_p > 0 ? batch_p : lone_team(v.n, v.nsyn, pmax);
   if (p < 1) p = 1;
   if (p > pmax) p = pmax;
   int64_t rc = (v.n + p - 1) / p;
@@ -1231,7 +1246,7 @@ static void plan_batch(g4s_net *const *nets, const int32_t *steps, int count, st
   // the CTAs that network i needs to finish in `us` (more than the GPU has: too many)
   auto need = [&](int i, double us) {
     const g4s_net *n = nets[i];
-    const int most = (int)std::min<int64_t>(pcap, (n->v.n + kSoloSlice - 1) / kSoloSlice);
+    const int most = (int)std::min<int64_t>(pcap, (n->v.n + kBatchMinSlice - 1) / kBatchMinSlice);
     int lo = teams[(size_t)i], hi = std::max(lo, most);
     while (lo < hi && steps[i] * team_step_us(n, syn[(size_t)i], lo) > us) ++lo;
     return lo;

@@ -41,9 +41,8 @@ constexpr int64_t kVuSlice = 2048;             // ... keep v, u in shared memory
 constexpr int64_t kAbcdSlice = 2048;           // ... keep a, b, c, d in shared memory (larger slices
                                                // keep them in global memory: the L1 left by a larger
                                                // shared-memory carve-out holds fewer table loads in flight)
-constexpr int64_t kSoloSlice = 128;            // neurons per CTA of a network running alone (at
-                                               // most: it spreads over every SM; measured best from
-                                               // N = 2500 to 10^6)
+constexpr int64_t kBatchMinSlice = 128;        // a network in a batch takes at most one CTA per this
+                                               // many neurons
 constexpr int64_t kBatchSlice = 8192;          // neurons per CTA of a network in a batch that fills the
                                                // GPU (the 256-network ensemble: 364 ms)
 constexpr int kStateBlock = 65536;             // neurons of the state read back at a time

@@ -56,3 +56,13 @@ def test_weights_at_the_packing_limit(g4s, oracle, geometry, scale):
     """70,000 targets take 17 bits of a packed word, which leaves Q32.32 weights below 2^14:
     16383 is packed, +-20000 sends the network to the separate arrays."""
     run_both(g4s, oracle, 70_000, 8, 53, 2.0, 40, geometry, 0, scale)
+
+
+@pytest.mark.parametrize("n,nsyn,p", [(33, 30, 1), (640, 639, 1), (641, 30, 13), (641, 640, 27), (1000, 479, 20),
+                                      (4000, 3647, 152), (4000, 3648, 77), (7904, 30, 152), (7905, 30, 152)])
+def test_automatic_team(g4s, oracle, n, nsyn, p):
+    """The team a network alone gets: one CTA, one per 52 neurons, as many as segment runs take,
+    or one per SM (152)."""
+    with g4s.Network(n, nsyn, seed=54) as net:
+        assert net.geometry()[0] == p
+    run_both(g4s, oracle, n, nsyn, 54, 2.0, 60, (0, -1), 0)
