@@ -514,9 +514,9 @@ __device__ __forceinline__ unsigned lanemask_le() { return 0xFFFFFFFFu >> (31u -
 struct TeamShared {
   int nown[2];    // spikes of this rank in the step
   int work[2];    // next chunk of the next step's drive
-  int k[2];       // spikes of the team in the step ...
-  int off[2];     // ... of the ranks before this one
-  int polled[2];  // warps that have added their source ranks to k and off
+  int off[2];     // spikes of the ranks before this one in the step
+  unsigned k[2];  // spikes of the team, plus kPolled for every warp that has added its source
+                  // ranks' to off and to this
   long long base; // raster offset of the step
   int fail;       // the exchange gave up (time limit, or the team's error word was set)
   int slot;       // queue slot taken by this CTA
@@ -524,6 +524,9 @@ struct TeamShared {
   TeamLayout L;   // in registers they would spill the delivery's reads in flight)
   unsigned long long lim;  // time limit of the step's waits
 };
+
+// (a team holds fewer than 2^26 neurons: kMaxTeam slices within the shared memory)
+constexpr unsigned kPolled = 1u << 26;
 
 // Record words of a rank per step: word 0 = spike count, words 1.. = ids (kInline inline).
 constexpr int kRankWords = kRecLines * kRecWords;
@@ -552,14 +555,17 @@ __device__ __forceinline__ int tagged_id(const unsigned long long *p, unsigned t
   }
 }
 
-// One round of a poll's checks by a warp whose words are not all there yet (t0: the poll's
-// start, set in round 0): true when the wait is given up.
+// The checks of a poll by a warp whose words are not all there yet, every kPollCheck rounds
+// (a round is one trip to L2; t0: the time of the first check, 0 before it): true when the
+// wait is given up.
+constexpr int kPollCheck = 16;
 __device__ __forceinline__ bool poll_check(const TeamItem &it, TeamShared &sh, int iter, unsigned long long &t0,
                                            unsigned long long lim) {
+  if (iter % kPollCheck != kPollCheck - 1) return false;
   int f = 0;
   if ((threadIdx.x & 31) == 0) {
     const unsigned long long now = globaltimer();
-    if (iter == 0) t0 = now;
+    if (t0 == 0) t0 = now;
     f = *(volatile int *)&sh.fail;
     if (!f && threadIdx.x == 0 && ld_relaxed(&it.sync->error) != 0) f = 1;
     if (!f && now - t0 > lim) {
@@ -931,9 +937,8 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
     sh.rank = rank;
     sh.nown[0] = sh.nown[1] = 0;
     sh.work[0] = sh.work[1] = 0;
-    sh.k[0] = sh.k[1] = 0;
+    sh.k[0] = sh.k[1] = 0u;
     sh.off[0] = sh.off[1] = 0;
-    sh.polled[0] = sh.polled[1] = 0;
     sh.base = 0;
     sh.fail = 0;
   }
@@ -966,24 +971,24 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
     const int t_abs = (int)it.t_abs0 + lt;
     const bool last = it.last && lt == steps - 1;
     const int par = lt & 1;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == NT - 32) {  // (a warp with less to do than the first ones)
       // the previous step's counters are final: its team count, then cleared for the next step
-      if (lead && lt > 0) v.counts[lt - 1] = sh.k[par ^ 1];
-      sh.base += sh.k[par ^ 1];
+      const int k = (int)(sh.k[par ^ 1] & (kPolled - 1u));
+      if (rank == 0 && lt > 0) v.counts[lt - 1] = k;
+      sh.base += k;
       sh.lim = lt == 0 ? limit_ns * 16 : limit_ns;  // (members may start late)
       sh.nown[par ^ 1] = 0;
       sh.work[par ^ 1] = 0;
-      sh.k[par ^ 1] = 0;
+      sh.k[par ^ 1] = 0u;
       sh.off[par ^ 1] = 0;
-      sh.polled[par ^ 1] = 0;
-      if (lead) {
+      if (rank == 0) {
         v.base[lt] = sh.base;
         if (v.stamps) v.stamps[2 * lt] = globaltimer();
       }
     }
     // ---- update of the owned neurons, their state in shared memory for the launch when it
     // fits, else in global memory (a, b, c, d then recomputed from the parameter r)
-    if (L.prez) {
+    if (L.prez && warp * 32 < cnt) {
       const Update w{L.vu_sm ? s_vu() : v.vu + lo, L.abcd_sm ? s_abcd() : v.abcd + lo, v.rpar + lo, s_z(), s_a(), s_b(),
                      last ? v.ilast + lo : nullptr, s_own(), &sh.nown[par], cnt, (int)min(v.nexc - lo, (int64_t)cnt),
                      lo, v.ge, v.gi};
@@ -991,7 +996,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
         update_slice<NT, false>(w);
       else
         update_slice<NT, true>(w);
-    } else {
+    } else if (!L.prez) {
       // no room for the next step's drive: computed here, one neuron at a time with the next
       // one's state in flight
       float2 *vu = v.vu + lo;
@@ -1031,7 +1036,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
     const unsigned rel_b = (unsigned)__cvta_generic_to_shared(s_b()) - (unsigned)lo * 4u;
     if (solo) {
       if (threadIdx.x == 0) {
-        sh.k[par] = nown;
+        sh.k[par] = (unsigned)nown;
         if (lead && v.stamps) v.stamps[2 * lt + 1] = globaltimer();
       }
       deliver_solo<NT, kPair>(it, s_own(), nown, rel_a, rel_b);
@@ -1045,13 +1050,16 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
       // in the overflow list; every word tagged with the step, so no fence is needed
       {
         const unsigned long long tg = (unsigned long long)tag << 32;
-        if (threadIdx.x < kRankWords) {
-          const int j = threadIdx.x;
+        static_assert(kRankWords == 32, "one warp publishes");
+        if (warp == 0) {
+          const int j = lane;
           const unsigned pay = j == 0 ? (unsigned)nown : (j - 1 < nown ? (unsigned)s_own()[j - 1] : 0xFFFFFFFFu);
           st_relaxed_u64(it.rec + ((size_t)par * it.team + rank) * kRankWords + j, tg | pay);
         }
-        unsigned long long *ovf = it.list + (size_t)par * v.n + lo;
-        for (int j = kInline + threadIdx.x; j < nown; j += NT) st_relaxed_u64(ovf + j, tg | (unsigned)s_own()[j]);
+        if (nown > kInline) {
+          unsigned long long *ovf = it.list + (size_t)par * v.n + lo;
+          for (int j = kInline + threadIdx.x; j < nown; j += NT) st_relaxed_u64(ovf + j, tg | (unsigned)s_own()[j]);
+        }
       }
       // ---- the other ranks' spikes, polled until the words carry the step's tag
       int n_src, cl = 0;  // sources of this warp; this lane's source's spikes
@@ -1063,36 +1071,37 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
         // slots, eight a line, up to two lines' slots per lane.  No warp waits for another
         // one's sources: it delivers as soon as its own have arrived.
         n_src = warp < min(kSrc, it.team) ? (it.team - 1 - warp) / kSrc + 1 : 0;
-        if (lane < n_src) c.inl = (int)s_pay()[(warp + lane * kSrc) * kRankWords] > kLine1After ? kInline : kRecWords - 1;
-        unsigned need = 0;
+        if (n_src) {
+          const int mine = lane < n_src ? (int)s_pay()[(warp + lane * kSrc) * kRankWords] : 0;
+          const unsigned more = __ballot_sync(0xFFFFFFFFu, mine > kLine1After);
+          c.inl = mine > kLine1After ? kInline : kRecWords - 1;
+          const int src = lane >> 3;
+          unsigned need = (src < n_src ? 1u : 0u) | (src + 4 < n_src ? 2u : 0u);
+          need |= need << 2 & ((more >> src & 1u) << 2 | (more >> (src + 4) & 1u) << 3);
+          const unsigned long long *p = recs + (warp + src * kSrc) * kRankWords + 2 * (lane & 7);
+          unsigned *to = s_pay() + (warp + src * kSrc) * kRankWords + 2 * (lane & 7);
+          for (int iter = 0;; ++iter) {
+            ulonglong2 a[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int x = lane + 32 * (k & 1), src = x >> 3;
-          if (src < n_src && (k < 2 || (int)s_pay()[(warp + src * kSrc) * kRankWords] > kLine1After)) need |= 1u << k;
-        }
-        __syncwarp();
-        for (int iter = 0;; ++iter) {
-          ulonglong2 a[4];
+            for (int k = 0; k < 4; ++k)
+              if (need & (1u << k))
+                a[k] = ld_relaxed_u64x2(p + (k & 1) * 4 * kSrc * kRankWords + (k >> 1) * kRecWords);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int x = lane + 32 * (k & 1);
-            if (need & (1u << k))
-              a[k] = ld_relaxed_u64x2(recs + (warp + (x >> 3) * kSrc) * kRankWords + (k >> 1) * kRecWords + 2 * (x & 7));
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int x = lane + 32 * (k & 1);
-            if ((need & (1u << k)) && (unsigned)(a[k].x >> 32) == tag && (unsigned)(a[k].y >> 32) == tag) {
-              *reinterpret_cast<uint2 *>(s_pay() + (warp + (x >> 3) * kSrc) * kRankWords + (k >> 1) * kRecWords + 2 * (x & 7)) =
-                  make_uint2((unsigned)a[k].x, (unsigned)a[k].y);
-              need &= ~(1u << k);
+            for (int k = 0; k < 4; ++k)
+              if ((need & (1u << k)) && (unsigned)(a[k].x >> 32) == tag && (unsigned)(a[k].y >> 32) == tag) {
+                *reinterpret_cast<uint2 *>(to + (k & 1) * 4 * kSrc * kRankWords + (k >> 1) * kRecWords) =
+                    make_uint2((unsigned)a[k].x, (unsigned)a[k].y);
+                need &= ~(1u << k);
+              }
+            if (__all_sync(0xFFFFFFFFu, need == 0) && stall == 0) break;
+            if (poll_check(it, sh, iter, t0, sh.lim)) {
+              n_src = 0;  // (the words read may be old)
+              break;
             }
           }
-          if (__all_sync(0xFFFFFFFFu, need == 0) && stall == 0) break;
-          if (poll_check(it, sh, iter, t0, sh.lim)) break;
+          __syncwarp();
+          if (lane < n_src) cl = (int)s_pay()[(warp + lane * kSrc) * kRankWords];
         }
-        __syncwarp();
-        if (lane < n_src) cl = (int)s_pay()[(warp + lane * kSrc) * kRankWords];
       } else {
         // few ranks: every warp reads every rank's count and takes its share of the batches
         n_src = it.team;
@@ -1107,25 +1116,25 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
         }
       }
       {
-        int incl = cl, below = (own_sources ? warp + lane * kSrc : lane) < rank ? cl : 0;
+        int incl = cl;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
+        for (int o = 1; o < 16; o <<= 1) {  // (at most sixteen sources)
           const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
           if (lane >= o) incl += y;
-          below += __shfl_xor_sync(0xFFFFFFFFu, below, o);
         }
-        c.total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        c.total = __shfl_sync(0xFFFFFFFFu, incl, 15);
         c.off = lane < n_src ? incl - cl : INT_MAX;
-        if (lane == 0 && (own_sources || warp == 0)) {
-          // the step's team count and this rank's raster offset, for the tail
-          if (c.total) atomicAdd(&sh.k[par], c.total);
-          if (below) atomicAdd(&sh.off[par], below);
-          __threadfence_block();
-          atomicAdd(&sh.polled[par], 1);
-        }
+      }
+      if (c.total) {
+        const int below = __reduce_add_sync(0xFFFFFFFFu, (own_sources ? warp + lane * kSrc : lane) < rank ? cl : 0);
+        if (lane == 0 && below && (own_sources || warp == 0)) atomicAdd(&sh.off[par], below);
+      }
+      if (lane == 0 && (own_sources || warp == 0)) {
+        // the step's team count and this rank's raster offset, for the tail
+        __threadfence_block();
+        atomicAdd(&sh.k[par], kPolled + (unsigned)c.total);
       }
       if (lead && v.stamps) v.stamps[2 * lt + 1] = globaltimer();
-      if (*(volatile int *)&sh.fail) c.total = 0;  // (the words read may be old)
       c.q0 = 0;
       c.dq = 32;
       c.wi = 0;
@@ -1151,7 +1160,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
     if (NT - 32 - warp * 32 < nown) {
       if (!solo) {  // (every warp's sources are counted, unless the exchange gave up)
         const int all = L.pay_sm ? kWarps : 1;
-        while (*(volatile int *)&sh.polled[par] < all && !*(volatile int *)&sh.fail) {
+        while ((int)(*(volatile unsigned *)&sh.k[par] / kPolled) < all && !*(volatile int *)&sh.fail) {
         }
         __threadfence_block();
       }
@@ -1174,12 +1183,12 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
         v.sstat[n] = st;
       }
     }
-    if (L.prez && lt + 1 < steps)
+    if (L.prez && lt + 1 < steps && __any_sync(0xFFFFFFFFu, *(volatile int *)&sh.work[par] * 32 < cnt))
       drive_chunks(v.seed, lo, cnt, t_abs + 1, s_z(), &sh.work[par], s_ws[warp].retry);
     __syncthreads();
     if (!solo && sh.fail) return;
   }
-  if (lead) v.counts[steps - 1] = sh.k[(steps - 1) & 1];
+  if (lead) v.counts[steps - 1] = (int)(sh.k[(steps - 1) & 1] & (kPolled - 1u));
   // pending currents (from the last delivery) and the state back to global memory
   for (int i = threadIdx.x; i < cnt; i += NT) {
     v.acc[lo + i] = (long long)s_a()[i] * 65536 + s_b()[i];
