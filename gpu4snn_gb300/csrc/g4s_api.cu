@@ -945,6 +945,16 @@ static int deliver_mode_of(const g4s_net *n) {
 // steps[i] steps (at most its chunk length).  Multi-CTA teams are queued first, then the
 // one-CTA teams by decreasing work, so that long networks start early.
 // ---------------------------------------------------------------------------------------
+// A lone network's ranks keep their columns of the segment table in shared memory where they
+// fit beside the slice in 186 KB (up to about 40,000 neurons: the next larger carve-out leaves
+// the row reads 32 KB of L1 less, N=42,000 x 1000 5.11 -> 5.32), which takes a trip to L2 out of every
+// step (us a step without and with: N=2,500 x 1000 3.36, 3.30; 8,000 x 500 3.59, 3.54; 33,333 x
+// 777 at drive 1.5 5.32, 5.18), for launches of more than one step per kColumnRows rows: reading
+// a column costs about 0.6 ns a row (14,000 rows 8 us).  The 768-thread kernel only, whose steps
+// are short.
+constexpr int64_t kColumnRows = 128;
+constexpr size_t kColumnSmem = 186 * 1024;
+
 // team_round_start enqueues the round on stream s and returns; team_round_finish waits for
 // it and checks every network's status words.  Between the two, the host may work on the
 // previous round's results, but must not touch the launch buffers (the round writes its pack
@@ -963,6 +973,16 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
       smem = std::max(smem, team_smem(nets[i]->team_rc, nets[i]->team_p));
     }
   if (order.empty()) return G4S_OK;
+  int64_t col = 0;
+  if (order.size() == 1) {
+    const g4s_net *n = nets[order[0]];
+    const bool wants = n->team_p > 1 && n->team_nt_eff == kTeamNTSmall && steps[order[0]] > n->v.n / kColumnRows;
+    const size_t with = wants ? team_smem(n->team_rc, n->team_p, n->v.n) : 0;
+    if (with && with <= kColumnSmem) {
+      smem = with;
+      col = n->v.n;
+    }
+  }
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     const g4s_net *x = nets[a], *y = nets[b];
     if ((x->team_p > 1) != (y->team_p > 1)) return x->team_p > 1;
@@ -1009,6 +1029,7 @@ static int team_round_start(g4s_net *const *nets, const int *steps, const bool *
     it.last = last[i] ? 1 : 0;
     it.team = n->team_p;
     it.rc = (int)n->team_rc;
+    it.col = (int)col;
     it.sync = n->gs;
     if ((uint64_t)n->tag_next + (uint64_t)steps[i] + 2 >= 0xFFFFFFFFull) {  // tags would wrap: start over
       G4S_CUDA(cudaMemsetAsync(n->list, 0, (size_t)n->v.n * 2 * sizeof(unsigned long long), s));

@@ -63,11 +63,12 @@ constexpr int kOwnSources = 12;
 // Shared-memory layout of one team rank (byte offsets; the optional arrays are present
 // when their flag is set).
 struct TeamLayout {
-  unsigned abcd, vu, a, b, own, z, pay, bytes;
-  bool abcd_sm, vu_sm, prez, pay_sm;
+  unsigned abcd, vu, a, b, own, z, pay, col, bytes;
+  bool abcd_sm, vu_sm, prez, pay_sm, col_sm;
 };
+// (col: rows of the rank's column of the segment table, 0 if it stays in global memory)
 __host__ __device__ inline unsigned team_align16(size_t x) { return (unsigned)((x + 15) & ~(size_t)15); }
-__host__ __device__ inline TeamLayout team_layout(int64_t rc, int team) {
+__host__ __device__ inline TeamLayout team_layout(int64_t rc, int team, int64_t col) {
   TeamLayout L{};
   L.abcd_sm = rc <= kAbcdSlice;
   L.vu_sm = rc <= kVuSlice;
@@ -88,7 +89,10 @@ __host__ __device__ inline TeamLayout team_layout(int64_t rc, int team) {
   if (L.prez) o = team_align16(o + (size_t)rc * 4);
   L.pay = (unsigned)o;  // payloads of the record lines
   if (L.pay_sm) o = team_align16(o + (size_t)team * kRecLines * kRecWords * 4);
-  L.bytes = (unsigned)o;
+  L.col_sm = col > 0;
+  L.col = (unsigned)o;
+  o = team_align16(o + (size_t)col * 4);
+  L.bytes = o < 0xFFFFFFFFull ? (unsigned)o : 0xFFFFFFFFu;
   return L;
 }
 // Rows sorted by target (unsigned, so unused slots last), equal targets by weight bits;
@@ -142,7 +146,7 @@ int net_prepare_rows(g4s_net *n);
 int net_create_pooled(const g4s_net_desc *desc, cudaMemPool_t pool, g4s_net **out);
 cudaError_t team_smem_ceiling();  // the part of team_max_blocks that launch_team needs
 // shared memory of one rank of a team of `team` CTAs with `rc` neurons each (0: does not fit)
-size_t team_smem(int64_t rc, int team);
+size_t team_smem(int64_t rc, int team, int64_t col = 0);
 
 // A handle's arrays, stream and absolute step, for the library's other translation units
 // (the on-device FP64 check, g4s_fp64check.cu).

@@ -620,6 +620,7 @@ __device__ __forceinline__ void fetch_spike(const TeamItem &it, TeamShared &sh, 
     if (__shfl_sync(0xFFFFFFFFu, c.off, k + step) <= q) k += step;
   const int oi = __shfl_sync(0xFFFFFFFFu, (int)((unsigned)c.off << 5) | c.inl, k), j = q - (oi >> 5), staged = oi & 31;
   if (q < c.total) {
+    const bool col = NT == kTeamNTSmall && sh.L.col_sm;  // (read ahead of the id)
     const int r = sh.L.pay_sm ? (int)(threadIdx.x >> 5) + k * source_warps(NT, kMode) : k;
     if (j < staged) {
       s = reinterpret_cast<const int *>(s_raw + sh.L.pay)[r * kRankWords + 1 + j];
@@ -629,9 +630,15 @@ __device__ __forceinline__ void fetch_spike(const TeamItem &it, TeamShared &sh, 
                                 : it.list + (size_t)par * it.v.n + (size_t)r * it.rc + j,
                     it.tag0 + (unsigned)c.lt + 1u, it, sh, sh.lim);
     }
-    const uint16_t *so = it.seg + (size_t)s * (unsigned)(it.team + 1) + sh.rank;
-    b = ld_keep_u16(so, pkeep);
-    e = ld_keep_u16(so + 1, pkeep);
+    if (col) {
+      const unsigned be = reinterpret_cast<const unsigned *>(s_raw + sh.L.col)[s];
+      b = (int)(be & 0xFFFFu);
+      e = (int)(be >> 16);
+    } else {
+      const uint16_t *so = it.seg + (size_t)s * (unsigned)(it.team + 1) + sh.rank;
+      b = ld_keep_u16(so, pkeep);
+      e = ld_keep_u16(so + 1, pkeep);
+    }
   }
 }
 
@@ -933,7 +940,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
   const bool solo = kSolo && it.team == 1;  // the whole network in this CTA: no exchange
   const bool lead = rank == 0 && threadIdx.x == 0;
   if (threadIdx.x == 0) {
-    sh.L = team_layout(it.rc, it.team);
+    sh.L = team_layout(it.rc, it.team, it.col);
     sh.rank = rank;
     sh.nown[0] = sh.nown[1] = 0;
     sh.work[0] = sh.work[1] = 0;
@@ -960,6 +967,14 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
     s_b()[i] = (unsigned)(q & 0xFFFF);
     if (L.vu_sm) s_vu()[i] = v.vu[lo + i];
     if (L.abcd_sm) s_abcd()[i] = v.abcd[lo + i];
+  }
+  if (L.col_sm) {
+    unsigned *col = reinterpret_cast<unsigned *>(s_raw + L.col);
+    const uint16_t *so = it.seg + rank;
+    const int64_t pitch = it.team + 1;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < it.col; i += NT)
+      col[i] = (unsigned)__ldg(so + i * pitch) | (unsigned)__ldg(so + i * pitch + 1) << 16;
   }
   if (L.pay_sm)  // the first step polls one record line per rank
     for (int r = threadIdx.x; r < it.team; r += NT) s_pay()[r * kRankWords] = 0;
@@ -1224,9 +1239,9 @@ __global__ void __launch_bounds__(NT, 1) k_team(const TeamItem *__restrict__ ite
 // Launchers.
 // ---------------------------------------------------------------------------------------
 
-size_t team_smem(int64_t rc, int team) {
+size_t team_smem(int64_t rc, int team, int64_t col) {
   if (rc < 1 || team < 1 || team > kMaxTeam) return 0;
-  const size_t bytes = team_layout(rc, team).bytes;
+  const size_t bytes = team_layout(rc, team, col).bytes;
   return bytes > kTeamSmemLimit ? 0 : (bytes < 16 ? 16 : bytes);
 }
 

@@ -74,6 +74,7 @@ struct TeamItem {
   int last;             // this launch ends the run: record the input current at its last step
   int team;             // CTAs of the team
   int rc;               // neurons per CTA slice
+  int col;              // rows of the segment table's column kept in shared memory (n, or 0: none)
   GridSync *sync;       // error word of the team
   unsigned tag0;        // record tag of step lt: tag0 + lt + 1 (never repeats for the list's words)
 };

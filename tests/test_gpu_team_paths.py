@@ -66,3 +66,11 @@ def test_automatic_team(g4s, oracle, n, nsyn, p):
     with g4s.Network(n, nsyn, seed=54) as net:
         assert net.geometry()[0] == p
     run_both(g4s, oracle, n, nsyn, 54, 2.0, 60, (0, -1), 0)
+
+
+@pytest.mark.parametrize("n,steps,geometry", [(5003, 39, (0, -1)), (5003, 40, (0, -1)), (5003, 40, (16, 1)),
+                                              (5003, 41, (3, 0)), (40_000, 320, (0, -1)), (42_000, 330, (0, -1))])
+def test_segment_columns(g4s, oracle, n, steps, geometry):
+    """Launches on both sides of the number of steps from which the ranks keep their columns of
+    the segment table in shared memory, and sizes on both sides of the largest column."""
+    run_both(g4s, oracle, n, 120, 55, 1.5, 2 * steps, geometry, 768)
