@@ -1226,19 +1226,19 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
 // Estimated device time in us of one step of a network on a team of p CTAs: a chain of round
 // trips, the update and drive of a CTA's neurons, and its share of the step's synapses (by the
 // length of its segments).  Fitted to networks of 1,100 to 10^6 neurons, most within 10%
-// (measured / model: one CTA, 4,189 neurons and 108,000 synapses a step 32 / 40, 1,120 and
-// 24,000 8.9 / 10.8; 8 CTAs, 43,005 and 1.05 million 40 / 39; 152 CTAs, 10^6 and 7.4 million
+// (measured / model: one CTA, 4,189 neurons and 108,000 synapses a step 32 / 33, 1,120 and
+// 24,000 8.9 / 9.1; 8 CTAs, 43,005 and 1.05 million 40 / 39; 152 CTAs, 10^6 and 7.4 million
 // 41 / 41).
 static double team_step_us(const g4s_net *n, double syn, int p) {
   const double neurons = (double)n->v.n / p, seg = std::max(1.0, (double)n->v.nsyn / p);
-  return p == 1 ? 2.2 + 1.6e-3 * neurons + 0.285e-3 * syn : 3.6 + 1.6e-3 * neurons + (0.19e-3 + 2.2e-3 / seg) * syn / p;
+  return p == 1 ? 2.0 + 1.3e-3 * neurons + 0.235e-3 * syn : 3.6 + 1.6e-3 * neurons + (0.19e-3 + 2.2e-3 / seg) * syn / p;
 }
 
 // CTAs of each network of a batch.  At one CTA per kBatchSlice neurons the networks take about
 // their share of a full GPU's time.  Where those teams would leave SMs idle the launch lasts
 // as long as its slowest network, so the CTAs go where the estimated time is: the shortest
 // time for which every network's smallest sufficient team fits one CTA per SM together (64
-// networks of 10^3 to 5 x 10^4 neurons, 16-fold apart in work: 44.3 ms by equal slices, 32.7 so).
+// networks of 10^3 to 5 x 10^4 neurons, 16-fold apart in work: 44.3 ms by equal slices, 32.3 so).
 // Teams of an earlier plan are kept while they are within a fifth of that time (a new team has
 // its segment table to build).
 static void plan_batch(g4s_net *const *nets, const int32_t *steps, int count, std::vector<int> &teams) {
