@@ -664,13 +664,13 @@ static int prepare_team(g4s_net *n, int batch_p = 0) {
   // CTA size: the one asked for; automatically 768 threads when a rank's expected share of
   // a step is small (fewer than 32768 synapses, from the recent firing rate), where the
   // spill-free kernel's shorter chain wins, else 1024 (more reads in flight); a batch takes
-  // 768 (its kernel holds the one-CTA mapping too, which spills at 1024: 64 networks of
-  // 10^3 to 5 x 10^4 neurons in one launch 44.5 ms against 45.4 to 53.7)
+  // 1024, as its CTAs hold large shares of their networks (64 networks of 10^3 to 5 x 10^4
+  // neurons in one launch 29.8 ms against 31.9, 256 of them 326 against 368)
   if (n->team_nt) {
     n->team_nt_eff = n->team_nt;
   } else {
     const double syn = (double)n->v.n * recent_rate(n) / 1000.0 * (double)n->v.nsyn / (double)p;
-    n->team_nt_eff = batch || syn < 32768.0 ? kTeamNTSmall : kTeamNT;
+    n->team_nt_eff = !batch && syn < 32768.0 ? kTeamNTSmall : kTeamNT;
   }
   int rc0 = prepare_rows(n);
   if (rc0) return rc0;
