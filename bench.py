@@ -425,7 +425,7 @@ def timed_leg(g, net, name, cfg, alg, a, pg, local, drive_override):
     elif last_alg == g.ALG_SKL:
         kname = "k_persistent (SKL global-atomic kernel)"
     else:
-        kname = f"k_update + k_deliver ({ALG_LABEL[last_alg]})"
+        kname = f"k_persistent ({ALG_LABEL[last_alg]}, a chunk's steps in one launch)"
     roofline = {"kernel": kname, "bound": "hbm",
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_source": f"{peak_kind} hbm_gbs",

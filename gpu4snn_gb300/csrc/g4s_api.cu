@@ -620,8 +620,8 @@ static bool plan_team(g4s_net *n, int want, int batch_p, int *p_out, int64_t *rc
 
 // The team kernel's buffers that do not depend on the team: the packed rows of its reads
 // (optional: without them, as when the device has no room left for them or a weight is too
-// large to be packed beside its target, the kernel reads the separate arrays) and the tagged spike lists.  Both are ready on return
-// (a batch may launch on another handle's stream).
+// large to be packed beside its target, the kernel reads the separate arrays) and the tagged
+// spike lists.  Both are ready on return (a batch may launch on another handle's stream).
 static int prepare_rows(g4s_net *n) {
   if (!n->v.pair && n->pair_fits) {
     const size_t bytes = (size_t)n->v.n * (size_t)n->v.stride * sizeof(unsigned long long);
@@ -1238,7 +1238,7 @@ static double team_step_us(const g4s_net *n, double syn, int p) {
 // their share of a full GPU's time.  Where those teams would leave SMs idle the launch lasts
 // as long as its slowest network, so the CTAs go where the estimated time is: the shortest
 // time for which every network's smallest sufficient team fits one CTA per SM together (64
-// networks of 10^3 to 5 x 10^4 neurons, 16-fold apart in work: 44.3 ms by equal slices, 32.3 so).
+// networks of 10^3 to 5 x 10^4 neurons, 16-fold apart in work: 44.3 ms by equal slices, 32.3 so, both with 768 threads).
 // Teams of an earlier plan are kept while they are within a fifth of that time (a new team has
 // its segment table to build).
 static void plan_batch(g4s_net *const *nets, const int32_t *steps, int count, std::vector<int> &teams) {

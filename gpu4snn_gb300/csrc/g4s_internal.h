@@ -44,7 +44,7 @@ constexpr int64_t kAbcdSlice = 2048;           // ... keep a, b, c, d in shared 
 constexpr int64_t kBatchMinSlice = 128;        // a network in a batch takes at most one CTA per this
                                                // many neurons
 constexpr int64_t kBatchSlice = 8192;          // neurons per CTA of a network in a batch that fills the
-                                               // GPU (the 256-network ensemble: 364 ms)
+                                               // GPU (256 networks, 3.2e9 synapses: 326 ms)
 constexpr int kStateBlock = 65536;             // neurons of the state read back at a time
 constexpr int kStateThreadBlocks = 3;          // ... in this many blocks or more, a thread per field
 constexpr int kMaxTeam = 176;                  // CTAs of one team (eight source ranks a warp, 22 such warps)

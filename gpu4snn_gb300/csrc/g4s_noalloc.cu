@@ -43,16 +43,16 @@ constexpr size_t kOffRec = 128;                                      // spike re
 constexpr size_t kOffCtl = kOffRec + 2 * kNoAllocMaxTeam * kRecLines * 128;  // int[5]: -, queue head, status, -, next tag
 constexpr size_t kOffSlots = kOffCtl + 128;                          // int2[kNoAllocMaxTeam]
 constexpr size_t kOffItem = kOffSlots + 256;                         // TeamItem
-constexpr size_t kOffList = 16384;                                   // u64[4][kNoAllocMaxNeurons]: overflow, dense ids
-constexpr size_t kOffSeg = kOffList + 4 * kNoAllocMaxNeurons * 8;  // u16[kNoAllocMaxNeurons][kNoAllocMaxTeam + 1]
+constexpr size_t kOffList = 16384;                                   // u64[2][kNoAllocMaxNeurons]: spikes beyond a record
+constexpr size_t kOffSeg = kOffList + 2 * kNoAllocMaxNeurons * 8;  // u16[kNoAllocMaxNeurons][kNoAllocMaxTeam + 1]
 constexpr size_t kScratchBytes = kOffSeg + (size_t)kNoAllocMaxNeurons * (kNoAllocMaxTeam + 1) * 2;
 
 static_assert(sizeof(GridSync) <= kOffRec - kOffSync, "error word");
 static_assert(sizeof(int2) * kNoAllocMaxTeam <= kOffItem - kOffSlots, "slots");
 static_assert(sizeof(TeamItem) <= kOffList - kOffItem, "item");
 static_assert(kNoAllocMaxTeam <= 32, "one setup thread per slot");
-// about 6.5 MB: the documented size of the array in gpu4snn.h
-static_assert(kScratchBytes > 6400000 && kScratchBytes < 6600000, "scratch size as documented");
+// about 4.5 MB: the documented size of the array in gpu4snn.h
+static_assert(kScratchBytes > 4400000 && kScratchBytes < 4600000, "scratch size as documented");
 
 // Everything a call needs before the team kernel, in one launch: the work-queue words, the
 // team's slots and the launch descriptor (which arrives by value as a kernel argument, so the

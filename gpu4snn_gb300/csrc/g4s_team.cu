@@ -49,13 +49,14 @@
 //             step's drive, handed out in chunks of 32 neurons to warps as they finish
 //             delivering.
 //   What bounds a step: with few spikes the chain update -> publish -> poll -> bounds ->
-//   rows; with many, instruction issue and the shared-memory additions together (ncu: issue
-//   50-75%, LSU data pipe 58%; DRAM 18% at N=300,000).  us per step of this kernel and of
-//   the one before it (block-wide scan and staging of the step's ids, a search per synapse,
-//   a conversion per synapse; all mappings in one kernel): N=2,500 x 1000 3.85 / 4.55,
-//   33,333 x 777 at drive 1.5 5.40 / 7.10, 100,000 x 1000 7.32 / 8.77, 10^6 x 1000 40.6 /
-//   43.4 (drive 0.5 14.5 / 17.6, drive 2 106.7 / 112.4), 250,000 x 10,000 40.0 / 54.8; 64
-//   networks in one launch 45.4 / 60.7 ms.
+//   rows, of whose 6,500 cycles (N=2,500) the four trips to L2 are half, the other half the
+//   straight code between them, which all warps issue; with many, the LSU's shared-memory
+//   pipe (ncu: 72% busy at N=250,000, drive 2, by the additions and the row reads; issue 55%,
+//   DRAM 24%).  us per step of this kernel and of the one before it (block-wide scan and
+//   staging of the step's ids, a search per synapse, a conversion per synapse; all mappings in
+//   one kernel): N=2,500 x 1000 3.30 / 4.55, 33,333 x 777 at drive 1.5 5.19 / 7.10, 100,000 x
+//   1000 7.28 / 8.77, 10^6 x 1000 40.1 / 43.4 (drive 0.5 13.0 / 17.6, drive 2 106 / 112),
+//   250,000 x 10,000 39.6 / 54.7; 64 networks in one launch 29.8 / 60.7 ms.
 //   The raster records the spike ids of every step while its buffer has room.
 #include <cuda_runtime.h>
 
@@ -579,8 +580,8 @@ __device__ __forceinline__ bool poll_check(const TeamItem &it, TeamShared &sh, i
 
 // Warps that poll source ranks and deliver their spikes; the others go straight to the next
 // step's drive, beside the first ones' waits.  Of the 768-thread CTA's 24 warps, 22 with
-// segment runs (us per step with 24, 22 and 20: N=33,333 x 777 5.65, 5.40, 5.75, N=100,000
-// 7.45, 7.34, 7.39); all of them for long segments and for 1024 threads, whose steps deliver
+// segment runs (us per step with 24, 23 and 22: N=33,333 x 777 5.37, 5.30, 5.19, N=100,000
+// 7.46, 7.33, 7.28; 20 were slower again); all of them for long segments and for 1024 threads, whose steps deliver
 // most of the time (N=10^6 at drive 2: 107 with 32 warps, 116 with 28).
 __host__ __device__ constexpr int source_warps(int nt, int mode) {
   return nt == kTeamNTSmall && mode == kDeliverRun ? 22 : nt / 32;

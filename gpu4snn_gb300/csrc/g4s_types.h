@@ -68,7 +68,7 @@ struct TeamItem {
   const uint16_t *seg;  // [n][team+1] row segment offsets (team > 1)
   unsigned long long *list;  // [2][n] tagged spike ids beyond a rank's record lines (at its neuron
                              // offset), by step parity
-  unsigned long long *rec;   // [2][team][2 x 16] tagged spike records, by step parity (zero at launch)
+  unsigned long long *rec;   // [2][team][2 x 16] tagged spike records, by step parity
   int64_t t_abs0;       // absolute step of the first step of this launch
   int steps;            // steps of this launch (0: nothing to do)
   int last;             // this launch ends the run: record the input current at its last step

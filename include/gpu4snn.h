@@ -144,9 +144,10 @@ int g4s_net_set_geometry(g4s_net *net, int32_t owner_blocks, int32_t delivery);
 /* Threads per CTA of the SKL team kernel: 1024 (the most table reads in flight, for steps
  * with many synapses per CTA), 768 (80 registers a thread instead of 64, no spills: faster
  * for steps whose work is small) or 0 (the default: 768 when a CTA's expected share of a
- * step, from the recent firing rate, is under 32768 synapses, else 1024; 768 in a batch).
- * Results do not depend on it; the autotuner tries both sizes.  A no-alloc run and a batch
- * of networks that disagree use 1024.  get_block_threads reports the size in use. */
+ * step, from the recent firing rate, is under 32768 synapses, else 1024; 1024 in a batch).
+ * Results do not depend on it; the autotuner tries both sizes.  A batch of networks that
+ * disagree uses 1024, a no-alloc run 768 for slices of at most 2048 neurons, else 1024.
+ * get_block_threads reports the size in use. */
 int g4s_net_set_block_threads(g4s_net *net, int32_t threads);
 int g4s_net_get_block_threads(g4s_net *net, int32_t *threads);
 int g4s_net_get_geometry(g4s_net *net, int32_t *owner_blocks, int64_t *slice);
@@ -299,7 +300,7 @@ typedef struct g4s_dev_net {
  * d_raster int32[raster_cap] spike ids (ids that do not fit are not recorded), d_status
  * (may be NULL) 0 or a device error code; `last` = 1 records i_last at the last step.
  * Stream-ordered on `stream` (NULL: the default stream).  The kernel's scratch is one
- * fixed __device__ array of about 6.5 MB (held by every GPU that loads the library): at
+ * fixed __device__ array of about 4.5 MB (held by every GPU that loads the library): at
  * most 131072 neurons and 16384 neurons per CTA; larger requests are rejected with
  * G4S_ERR_INVALID.  The first call on a device looks the array's address up (once per
  * device, with that device current) and sets the team kernel's shared-memory ceiling.  A
