@@ -218,7 +218,10 @@ __device__ __forceinline__ unsigned update_phase(const NetView &v, int lt, int64
   return mine;
 }
 
-// Groups of `group` consecutive threads take whole spiking rows (N, AP).
+// Groups of `group` consecutive threads take whole spiking rows (N, AP), four vectors a thread
+// in flight: a thread's share of a row is a chain of loads otherwise (us a step with one and
+// with four: N=2,500 x 1000 N 7.3, 6.5, AP 6.1, 5.7; 20,000 x 1000 at drive 1.5 N 12.4, 9.7, AP
+// 10.1, 8.7).
 __device__ __forceinline__ void deliver_groups(const NetView &v, const int *list, int K, int group) {
   const uint32_t rv = (uint32_t)(v.stride >> 2);
   const int gpb = blockDim.x / group;
@@ -227,9 +230,13 @@ __device__ __forceinline__ void deliver_groups(const NetView &v, const int *list
   // (consecutive rows to different blocks: a step's few rows spread over the SMs)
   for (int64_t q = (int64_t)(threadIdx.x / group) * gridDim.x + blockIdx.x; q < K; q += ngroups) {
     const int row = __ldcg(list + q);
-    for (uint32_t j = lig; j < rv; j += group) {
-      const Vec4 x = load_vec(v, row, j);
-      deliver4(v.acc, x.t, x.w);
+    for (uint32_t j = lig; j < rv; j += 4 * group) {
+      Vec4 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = load_vec(v, row, j + u * group < rv ? j + u * group : j);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (j + u * group < rv) deliver4(v.acc, x[u].t, x[u].w);
     }
   }
 }
@@ -427,7 +434,7 @@ int persistent_blocks() { return persistent_occupancy<kPerLarge>() * sm_count();
 
 // Threads per spiking row of a scheme: N a warp for each spiking neuron (one thread, the
 // reference's choice, walks a row as a chain of loads: 88 us a step for N=2,500 x 1000 against
-// 7), AP a group of 64, S and AB flat over all synapses of the step, as the SKL fallback.
+// 6.5), AP a group of 64, S and AB flat over all synapses of the step, as the SKL fallback.
 static int deliver_group(int alg) { return alg == kAlgN ? 32 : alg == kAlgAP ? 64 : 0; }
 
 template <int NT>

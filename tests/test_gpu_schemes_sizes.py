@@ -26,3 +26,18 @@ def test_scheme_sizes(g4s, oracle, n):
             for k in ("v", "u", "I"):
                 assert np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32)), (alg, k)
             assert np.array_equal(got["nospks"], want["nospks"]) and np.array_equal(net.currents(), cur)
+
+
+@pytest.mark.parametrize("nsyn", [125, 129, 511, 512, 513, 1021, 1024, 1025])
+def test_row_lengths(g4s, oracle, nsyn):
+    """Rows around one and four vectors a thread of N's and AP's groups (32 and 64 threads)."""
+    n, seed = 1500, 82
+    d = oracle.make_desc(n, nsyn, seed, drive_scale=3.0)
+    idx, w = oracle.conn_philox(d)
+    sim = oracle.Sim(d, idx, w)
+    sim.run(30, threads=8)
+    for alg in (0, 1):
+        with g4s.Network(n, nsyn, seed=seed, drive_scale=3.0) as net:
+            net.run(30, alg)
+            assert np.array_equal(net.counts(), sim.counts())
+            assert np.array_equal(net.currents(), sim.acc())
