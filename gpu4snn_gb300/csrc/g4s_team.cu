@@ -514,7 +514,7 @@ __device__ __forceinline__ unsigned lanemask_le() { return 0xFFFFFFFFu >> (31u -
 // (by step parity) so that one is cleared while the other is in use.
 struct TeamShared {
   int nown[2];    // spikes of this rank in the step
-  int work[2];    // next chunk of the next step's drive
+  int work[2];    // next chunk of the next step's drive (a warp adds at most two past the last one)
   int off[2];     // spikes of the ranks before this one in the step
   unsigned k[2];  // spikes of the team, plus kPolled for every warp that has added its source
                   // ranks' to off and to this
@@ -559,8 +559,8 @@ __device__ __forceinline__ int tagged_id(const unsigned long long *p, unsigned t
 // The checks of a poll by a warp whose words are not all there yet, every kPollCheck rounds
 // (a round is one trip to L2; t0: the time of the first check, 0 before it): true when the
 // wait is given up.
-constexpr int kPollCheck = 16;
-__device__ __forceinline__ bool poll_check(const TeamItem &it, TeamShared &sh, int iter, unsigned long long &t0,
+constexpr unsigned kPollCheck = 16;
+__device__ __forceinline__ bool poll_check(const TeamItem &it, TeamShared &sh, unsigned iter, unsigned long long &t0,
                                            unsigned long long lim) {
   if (iter % kPollCheck != kPollCheck - 1) return false;
   int f = 0;
@@ -1096,7 +1096,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
           need |= need << 2 & ((more >> src & 1u) << 2 | (more >> (src + 4) & 1u) << 3);
           const unsigned long long *p = recs + (warp + src * kSrc) * kRankWords + 2 * (lane & 7);
           unsigned *to = s_pay() + (warp + src * kSrc) * kRankWords + 2 * (lane & 7);
-          for (int iter = 0;; ++iter) {
+          for (unsigned iter = 0;; ++iter) {
             ulonglong2 a[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k)
@@ -1113,10 +1113,11 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
             if (NT == kTeamNT && kMode == kDeliverRun && !kSolo && L.prez && lt + 1 < steps) {
               // large steps, whose ranks finish some thousand cycles apart: a chunk of the next
               // step's drive instead of waiting (N=10^6 40.7 -> 40.1 us a step; smaller steps wait
-              // for about one trip to L2, and lose by it)
-              int ch = 0;
-              if (lane == 0) ch = atomicAdd(&sh.work[par], 1);
-              ch = __shfl_sync(0xFFFFFFFFu, ch, 0) * 32 + lane;
+              // for about one trip to L2, and lose by it).  Taken only while there is one: a warp
+              // goes past the last chunk once, not in every round of a wait of any length.
+              int ch = cnt;
+              if (lane == 0 && *(volatile int *)&sh.work[par] * 32 < cnt) ch = atomicAdd(&sh.work[par], 1) * 32;
+              ch = __shfl_sync(0xFFFFFFFFu, ch, 0) + lane;
               if (ch < cnt) s_z()[ch] = normal(v.seed, (uint64_t)(lo + ch), (uint64_t)(t_abs + 1));
               __syncwarp();
             }
@@ -1131,7 +1132,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
       } else {
         // few ranks: every warp reads every rank's count and takes its share of the batches
         n_src = it.team;
-        for (int iter = 0;; ++iter) {
+        for (unsigned iter = 0;; ++iter) {
           unsigned long long w = 0;
           if (lane < n_src) w = ld_relaxed_u64(recs + lane * kRankWords);
           if (__all_sync(0xFFFFFFFFu, lane >= n_src || (unsigned)(w >> 32) == tag) && stall == 0) {
