@@ -726,7 +726,9 @@ static int finish_tables(g4s_net *n, bool may_be_sorted) {
   // running, where a server creates networks while its rounds run.
   cudaStream_t st = n->stream;
   int *flag = nullptr, h_unsorted = 1;
-  cudaError_t ef = may_be_sorted ? cudaMallocAsync((void **)&flag, sizeof(int), st) : cudaSuccess;
+  cudaError_t ef = cudaSuccess;
+  if (may_be_sorted)
+    ef = g_fail_next_alloc.exchange(0) ? cudaErrorMemoryAllocation : cudaMallocAsync((void **)&flag, sizeof(int), st);
   if (ef == cudaSuccess && flag) ef = launch_rows_sorted(n->v, flag, st);
   if (ef == cudaSuccess && flag) ef = cudaMemcpyAsync(&h_unsorted, flag, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (flag) cudaFreeAsync(flag, st);
@@ -1577,6 +1579,11 @@ static size_t first_bad_host(const int32_t *idx, size_t cnt, int32_t nn) {
   return *std::min_element(bad.begin(), bad.end());
 }
 
+// Before the tables change: no plan, and no new one until finish_tables has passed the new ones
+// (if it does not get there, runs take the global-atomic kernel, whose additions any table of
+// checked targets keeps in range).
+static void drop_plan(g4s_net *n) { n->team_ready = n->pair_ready = n->tables_fit = false; }
+
 // The same on the device, on the targets' way to it: into memory that holds nothing needed
 // (the packed rows, formed again from the tables; else stream-ordered scratch), checked there
 // and only then moved to v.idx (*moved).  The 400 MB of targets of N=100,000 x 1000 take
@@ -1596,19 +1603,22 @@ static int first_bad_device(g4s_net *n, const int32_t *idx, size_t *bad, bool *m
     return G4S_OK;
   }
   int *stage = scratch ? scratch : reinterpret_cast<int *>(const_cast<unsigned long long *>(v.pair));
-  const bool pair_was_ready = n->pair_ready;
-  if (!scratch) n->pair_ready = false;
+  // (the plan goes with its packed rows: a run after a failure below forms them again)
+  const bool pair_was_ready = n->pair_ready, team_was_ready = n->team_ready;
+  if (!scratch) n->pair_ready = n->team_ready = false;
   cudaError_t e = cudaMemcpyAsync(stage, idx, bytes, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = launch_first_bad(stage, v, d_first, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&first, d_first, 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess && first == ~0ull) {
+    drop_plan(n);
     e = cudaMemcpyAsync(const_cast<int *>(v.idx), stage, bytes, cudaMemcpyDeviceToDevice, s);
     *moved = e == cudaSuccess;
   } else if (e == cudaSuccess && !scratch && pair_was_ready) {
     e = launch_pairs(v, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     n->pair_ready = e == cudaSuccess;
+    n->team_ready = n->pair_ready && team_was_ready;
   }
   cudaFreeAsync(d_first, s);
   if (scratch) cudaFreeAsync(scratch, s);
@@ -1696,6 +1706,7 @@ int g4s_net_load_tables(g4s_net *n, const int32_t *idx, const float *w, int32_t 
   if (bad != SIZE_MAX)
     return set_error(G4S_ERR_INVALID, "table entry " + std::to_string(bad) + " targets neuron " +
                                           std::to_string(idx[bad]) + " >= n");
+  drop_plan(n);
   if (!moved) G4S_CUDA(cudaMemcpyAsync(const_cast<int *>(v.idx), idx, bytes, cudaMemcpyHostToDevice, n->stream));
   G4S_CUDA(cudaMemcpyAsync(const_cast<float *>(v.w), w, bytes, cudaMemcpyHostToDevice, n->stream));
   return finish_tables(n, true);

@@ -92,7 +92,9 @@ int g4s_net_create(const g4s_net_desc *desc, g4s_net **out);
  * tables, gpu4snn.cu:910-911); padding slots carry target -1. */
 int g4s_net_create_from_tables(const g4s_net_desc *desc, const int32_t *idx, const float *w, int32_t stride,
                                g4s_net **out);
-/* Replace the tables of an existing handle from host memory (H2D). */
+/* Replace the tables of an existing handle from host memory (H2D).  Refused tables leave the
+ * handle's own in place; after any other error the handle's tables are undefined until a load
+ * succeeds. */
 int g4s_net_load_tables(g4s_net *net, const int32_t *idx, const float *w, int32_t stride);
 /* Neuron state, currents, statistics and raster back to step 0 (initNeuron, gpu4snn.cu:1094). */
 int g4s_net_reset(g4s_net *net);
@@ -176,8 +178,9 @@ int g4s_net_destroy(g4s_net *net);
  *   G4S_FAULT_BARRIER_STALL  the next SKL launch of `net` waits at its first barrier for
  *                            one block more than it has, so the wait runs out after the
  *                            barrier time limit and the run returns G4S_ERR_TIMEOUT;
- *   G4S_FAULT_ALLOC          the next device allocation of g4s_net_create fails
- *                            (process-wide; `net` may be NULL). */
+ *   G4S_FAULT_ALLOC          the next device allocation of g4s_net_create fails, or of the
+ *                            row-order check of g4s_net_load_tables, or of the optional
+ *                            packed rows (process-wide; `net` may be NULL). */
 #define G4S_FAULT_BARRIER_STALL 1
 #define G4S_FAULT_ALLOC 2
 int g4s_inject_fault(g4s_net *net, int32_t kind);

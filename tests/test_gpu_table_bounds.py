@@ -51,3 +51,35 @@ def test_refused_upload_keeps_the_tables(g4s, oracle, n, nsyn, ran):
         net.run(40)
         assert np.array_equal(np.stack(net.raster()), np.stack(sim.raster()))
         assert all(np.array_equal(a, b) for a, b in zip(own, net.tables()))
+
+
+@pytest.mark.parametrize("ran", [False, True])
+@pytest.mark.parametrize("n,nsyn", [(2001, 9), (20001, 300)])
+def test_upload_that_fails_half_way(g4s, oracle, n, nsyn, ran):
+    """An upload that runs out of memory once the new tables (rows in draw order) have replaced
+    the old ones, checked on the host or on the device, before and after the packed rows exist:
+    no run uses what was planned for the old tables, and the next upload is taken."""
+    from gpu4snn_gb300 import _lib
+    d = oracle.make_desc(n, nsyn, 22, drive_scale=2.0)
+    idx, w = oracle.conn_philox(d)
+    sim = oracle.Sim(d, idx, w)
+    sim.run(40, threads=8)
+    with g4s.Network(n, nsyn, seed=23, drive_scale=2.0) as net:
+        net.run(20 if ran else 0)
+        assert net.geometry()[0] >= 1
+        net.inject_fault(_lib.FAULT_ALLOC)
+        with pytest.raises(g4s.G4SError) as e:
+            net.load_tables(idx, w)
+        assert e.value.code == _lib.ERR_NOMEM
+        assert net.geometry() == (0, 0)
+        net.run(20)
+    with g4s.Network(n, nsyn, seed=22, drive_scale=2.0) as net:
+        net.run(20 if ran else 0)
+        net.inject_fault(_lib.FAULT_ALLOC)
+        with pytest.raises(g4s.G4SError):
+            net.load_tables(idx, w)
+        net.load_tables(idx, w)
+        assert net.geometry()[0] >= 1
+        net.reset()
+        net.run(40)
+        assert np.array_equal(np.stack(net.raster()), np.stack(sim.raster()))
