@@ -182,7 +182,7 @@ struct g4s_net {
   double last_ms = 0, last_wall_ms = 0;
   int64_t last_spikes = 0;
   int last_alg = -1;
-  int barrier_stall = 0;  // injected: extra arrivals the next SKL launch waits for
+  int barrier_stall = 0;  // injected: the waits of the next SKL launch run out
   // SKL team kernel: team size and slice, per-step spike lists, per-row segment table,
   // requested team size (0 = auto), whether the tables satisfy the exactness bound of the
   // split accumulation, and the launch buffers of the handle's own runs
@@ -1097,6 +1097,9 @@ static int team_round(g4s_net *const *nets, const int *steps, const bool *last, 
   return rc ? rc : team_round_finish(L, s, kernel_ms, launches);
 }
 
+// Why the waits of a handle's next SKL launch run out (0: they need not).
+static int stall_of(const g4s_net *n) { return n->barrier_stall ? kStallFault : n->barrier_ns == 0 ? kStallLimit : 0; }
+
 // One chunk of steps by a launch that works on the handle's global arrays.
 static int run_chunk(g4s_net *n, int cs, bool last, bool skl, StepLaunch &launch, int64_t *spikes, double *kernel_ms) {
   NetView &v = n->v;
@@ -1104,7 +1107,7 @@ static int run_chunk(g4s_net *n, int cs, bool last, bool skl, StepLaunch &launch
   G4S_CUDA(cudaMemsetAsync(v.stamps, 0, ((size_t)cs * 2 + 2) * 8, n->stream));
   G4S_CUDA(cudaMemsetAsync(n->gs, 0, sizeof(GridSync), n->stream));
   G4S_CUDA(cudaEventRecord(n->ek0, n->stream));
-  G4S_CUDA(launch(v, n->t_abs, cs, last, n->gs, skl ? n->barrier_ns : kBarrierNs, skl ? n->barrier_stall : 0, n->stream));
+  G4S_CUDA(launch(v, n->t_abs, cs, last, n->gs, skl ? n->barrier_ns : kBarrierNs, skl ? stall_of(n) : 0, n->stream));
   if (skl) n->barrier_stall = 0;
   G4S_CUDA(cudaEventRecord(n->ek1, n->stream));
   int rc = check_status(n, "persistent step kernel");
@@ -1164,7 +1167,7 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
       cs = (int)std::min<int64_t>(remaining, n->chunk_steps);
       const bool last_chunk = remaining == cs;
       g4s_net *one[1] = {n};
-      const int rc = team_round_start(one, &cs, &last_chunk, 1, n->launch, n->stream, n->barrier_ns, n->barrier_stall);
+      const int rc = team_round_start(one, &cs, &last_chunk, 1, n->launch, n->stream, n->barrier_ns, stall_of(n));
       n->barrier_stall = 0;
       remaining -= cs;
       return rc;
@@ -1329,7 +1332,7 @@ static int run_nets(g4s_net *const *nets, const int32_t *steps, int count, doubl
       any = any || cs[i] > 0;
     }
     if (!any) break;
-    int rc = team_round(nets, cs.data(), last.get(), count, L, s, nets[0]->barrier_ns, 0, &kms, &nl);
+    int rc = team_round(nets, cs.data(), last.get(), count, L, s, nets[0]->barrier_ns, nets[0]->barrier_ns == 0 ? kStallLimit : 0, &kms, &nl);
     if (rc) return rc;
     for (int i = 0; i < count; ++i)
       if (cs[i] > 0 && (rc = chunk_copy_raster(nets[i], cs[i], s))) return rc;

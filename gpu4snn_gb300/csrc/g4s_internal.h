@@ -153,7 +153,8 @@ size_t team_smem(int64_t rc, int team, int64_t col = 0);
 const NetView &net_view(const g4s_net *n);
 // `steps` further steps of the handle (at most net_chunk_steps) by a launch of the caller's:
 // it does what the library's own step kernels do with the handle's arrays, and the handle's
-// record takes the results.  `stall`: blocks too many for its grid barrier to wait for.
+// record takes the results.  `stall`: blocks too many for its grid barrier to wait for, so that
+// it runs out.
 struct StepLaunch {
   virtual cudaError_t operator()(const NetView &v, int64_t t_abs0, int steps, bool last, GridSync *gs,
                                  unsigned long long limit_ns, int stall, cudaStream_t s) = 0;

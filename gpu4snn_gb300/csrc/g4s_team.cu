@@ -1037,7 +1037,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
     }
     __syncthreads();
     const int nown = sh.nown[par];
-    if (stall != 0 && solo) {
+    if (stall == kStallFault && solo) {
       // injected fault of a one-CTA team: wait for a member that does not exist
       if (threadIdx.x == 0) {
         const unsigned long long lim = sh.lim, t0 = globaltimer();

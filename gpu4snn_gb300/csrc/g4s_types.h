@@ -16,6 +16,12 @@ constexpr int kErrTimeoutCode = 1;   // a grid barrier waited longer than its li
 constexpr int kErrOverflowCode = 2;  // a spike did not fit the raster buffer
 constexpr int kErrConnCode = 3;      // connectivity generation ran out of draws
 
+// Why a launch's waits run out: a fault is injected (one-CTA teams have a wait then too), or the
+// time limit is 0 (every wait there is; without this, waits shorter than the polls between two
+// looks at the clock would pass).
+constexpr int kStallFault = 1;
+constexpr int kStallLimit = 2;
+
 // Grid barrier state: a monotone counter (arrivals, and a sum in its high half) and an error
 // word (one 128 B line).
 struct alignas(128) GridSync {

@@ -129,8 +129,9 @@ int g4s_net_stats(g4s_net *net, double *rate_hz, double *isi_cv, int64_t *total_
  * neuron and up to 64 MB (8 bytes per neuron if that is more) for the differences. */
 int g4s_net_fp64_check(g4s_net *net, int32_t steps, double *dv_max, double *dv_p99, double *dv_median,
                        int32_t *first_divergent, double *v64_out, double *u64_out);
-/* Grid-barrier time limit of the SKL kernel in ns (default 2 s); 0 makes every barrier
- * give up at once (used to test the timeout path). */
+/* Time limit in ns of the waits between the SKL kernel's CTAs (default 2 s), looked at every
+ * 16 polls of about half a microsecond; 0 makes every wait give up (used to test the timeout
+ * path; a network on one CTA has no waits). */
 int g4s_net_set_barrier_timeout(g4s_net *net, uint64_t ns);
 /* Geometry of the SKL kernel (the reference sizes its persistent grids from occupancy,
  * gpu4snn.cu:1066-1076): `owner_blocks` CTAs, each owning a contiguous slice of target

@@ -45,3 +45,49 @@ def test_team_that_waits_for_another(g4s):
             a, b = alone.state(), net.state()
             assert all(np.array_equal(a[f].view(np.uint32), b[f].view(np.uint32)) for f in ("v", "u", "I", "nospks"))
         net.close()
+
+
+@pytest.mark.parametrize("n,threads,geometry,fits", [(700, 0, (0, -1), True), (2000, 0, (0, -1), True), (2000, 0, (4, 0), True),
+                                                     (2000, 0, (15, 1), True), (9000, 1024, (0, 0), True),
+                                                     (2000, 0, (0, -1), False)])
+def test_limit_of_nothing(g4s, oracle, n, threads, geometry, fits):
+    """A time limit of 0 ends every run that waits, however short the wait would be: alone, in a
+    batch, in the FP64 check, and on the global-atomic kernel (tables beyond the exactness
+    bound of the team kernel)."""
+    from gpu4snn_gb300 import _lib
+    from gpu4snn_gb300.network import run_batch
+    nsyn, seed = 100, 63
+    d = oracle.make_desc(n, nsyn, seed)
+    idx, w = oracle.conn_philox(d)
+    if not fits:
+        w = w.copy()
+        idx[0, :2], w[0, :2] = (5, 6), 30000.0
+        idx[1, :2], w[1, :2] = (5, 6), 30000.0
+    sim = oracle.Sim(d, idx, w)
+    sim.run(30, threads=8)
+
+    def check(call):
+        with pytest.raises(g4s.G4SError) as e:
+            call()
+        assert e.value.code == _lib.ERR_TIMEOUT
+
+    with g4s.Network(n, nsyn, seed=seed, tables=(idx, w)) as net, g4s.Network(300, 50, seed=64) as one:
+        net.set_geometry(*geometry)
+        net.set_block_threads(threads)
+        assert (net.geometry()[0] > 1) == fits
+        net.set_barrier_timeout(0)
+        check(lambda: net.run(20, 4))
+        net.reset()
+        check(lambda: net.fp64_check(5))
+        net.reset()
+        if fits and geometry[0]:
+            check(lambda: run_batch([net, one], 20))
+            net.reset()
+            one.reset()
+        net.set_barrier_timeout(2_000_000_000)
+        net.run(30, 4)
+        assert np.array_equal(np.stack(net.raster()), np.stack(sim.raster()))
+        assert np.array_equal(net.currents(), sim.acc())
+        one.set_barrier_timeout(0)  # (one CTA: no waits)
+        one.run(20, 4)
+        assert one.info().steps_done == 20
