@@ -164,9 +164,11 @@ struct g4s_net {
   // of the neuron state (never both at once)
   unsigned char *h_stage = nullptr;
   size_t stage_bytes = 0;
+  bool stage_pinned = false;
   int *h_raster = nullptr;  // the staged raster (in h_stage)
   void *arena = nullptr;    // device memory of the neuron state and the per-step arrays
   int64_t raster_full = 0;  // raster ids of a full chunk (the buffer holds v.raster_cap, by need)
+  int *raster_step = nullptr;  // the first buffer: one step's ids, in the arena
   // host results since the last reset: the recorded ids, and for each recorded chunk its
   // first step, its steps' place in `counts` and its ids' place in `rid`
   std::vector<int32_t> counts;
@@ -226,6 +228,15 @@ static void net_free(g4s_net *n, const void *p) {
     cudaFree(const_cast<void *>(p));
 }
 
+static void free_stage(g4s_net *n) {
+  if (n->stage_pinned)
+    cudaFreeHost(n->h_stage);
+  else
+    free(n->h_stage);
+  n->h_stage = nullptr;
+  n->stage_bytes = 0;
+}
+
 static void free_net(g4s_net *n) {
   if (!n) return;
   NetView &v = n->v;
@@ -238,10 +249,10 @@ static void free_net(g4s_net *n) {
   net_free(n, n->arena);
   net_free(n, const_cast<int *>(v.idx));
   net_free(n, const_cast<float *>(v.w));
-  net_free(n, v.raster);
+  if (v.raster != n->raster_step) net_free(n, v.raster);
   net_free(n, n->seg);
   net_free(n, n->list);
-  cudaFreeHost(n->h_stage);
+  free_stage(n);
   if (n->ev0) cudaEventDestroy(n->ev0);
   if (n->ev1) cudaEventDestroy(n->ev1);
   if (n->ek0) cudaEventDestroy(n->ek0);
@@ -352,7 +363,8 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
                o_sstat = place(N * sizeof(SpikeStat)), o_counts = place((size_t)cs * sizeof(int)),
                o_base = place((size_t)cs * sizeof(long long)),
                o_stamps = place(((size_t)cs * 2 + 2) * sizeof(unsigned long long)), o_status = place(sizeof(int)),
-               o_gs = place(sizeof(GridSync) * (1 + 2 * (size_t)kMaxTeam * kRecLines)), o_stats = place(2 * sizeof(double));
+               o_gs = place(sizeof(GridSync) * (1 + 2 * (size_t)kMaxTeam * kRecLines)), o_stats = place(2 * sizeof(double)),
+               o_raster = place(pool ? 0 : N * sizeof(int));
   unsigned char *mem = nullptr;
   if ((rc = dalloc(n, &mem, bytes, "neuron state and per-step arrays"))) {
     free_net(n);
@@ -371,6 +383,7 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
   v.status = reinterpret_cast<int *>(mem + o_status);
   n->gs = reinterpret_cast<GridSync *>(mem + o_gs);
   n->d_stats = reinterpret_cast<double *>(mem + o_stats);
+  if (!pool) n->raster_step = v.raster = reinterpret_cast<int *>(mem + o_raster);
   if ((rc = dalloc(n, const_cast<int **>(&v.idx), N * S, "targets")) ||
       (rc = dalloc(n, const_cast<float **>(&v.w), N * S, "weights")) ||
       // (a pool's network gets its whole raster now: a run may use another network's stream)
@@ -378,7 +391,7 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
     free_net(n);
     return rc;
   }
-  v.raster_cap = pool ? n->raster_full : 0;
+  v.raster_cap = pool ? n->raster_full : d->n;
   if ((!n->stream && (e = cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking)) != cudaSuccess) ||
       (e = cudaEventCreate(&n->ev0)) != cudaSuccess || (e = cudaEventCreate(&n->ev1)) != cudaSuccess ||
       (e = cudaEventCreate(&n->ek0)) != cudaSuccess || (e = cudaEventCreate(&n->ek1)) != cudaSuccess) {
@@ -787,42 +800,55 @@ static int chunk_copy_meta(g4s_net *n, int cs, cudaStream_t s) {
 
 static int64_t chunk_total(const g4s_net *n, int cs) { return (int64_t)n->c_base[cs - 1] + n->c_counts[cs - 1]; }
 
-// At least `bytes` of pinned staging (its contents are not kept).
-static int need_stage(g4s_net *n, size_t bytes) {
-  if (bytes <= n->stage_bytes) return G4S_OK;
+// At least `bytes` of staging (its contents are not kept), pinned if that is to be had, else
+// pageable; `pinned`: a failure instead.
+static int need_stage(g4s_net *n, size_t bytes, bool pinned) {
+  if (bytes <= n->stage_bytes && (n->stage_pinned || !pinned)) return G4S_OK;
   bytes = std::max(bytes, (size_t)1 << 18);
-  cudaFreeHost(n->h_stage);
-  n->h_stage = nullptr;
-  n->stage_bytes = 0;
-  G4S_CUDA(cudaMallocHost((void **)&n->h_stage, bytes));
+  free_stage(n);
+  n->stage_pinned = !g_fail_next_alloc.exchange(0) && cudaMallocHost((void **)&n->h_stage, bytes) == cudaSuccess;
+  if (!n->stage_pinned) {
+    (void)cudaGetLastError();
+    n->h_stage = pinned ? nullptr : static_cast<unsigned char *>(malloc(bytes));
+    if (!n->h_stage) return set_error(G4S_ERR_NOMEM, "host staging buffer");
+  }
   n->stage_bytes = bytes;
   return G4S_OK;
 }
 
 // The raster buffer for chunks of up to `steps` steps (every neuron firing at every step).  A
-// full chunk's buffer is up to 1 GiB, of which a short run uses little: allocated by need.
-static int need_raster(g4s_net *n, int64_t steps) {
+// full chunk's buffer is up to 1 GiB, of which a short run uses little: allocated by need, and
+// where the device has no room for that much, by halves down to the one step's ids that the
+// handle holds from its creation.  Chunks are then as long as the buffer allows.
+static void need_raster(g4s_net *n, int64_t steps) {
   const int64_t want = std::min(n->raster_full, std::max<int64_t>(1, steps) * n->v.n);
-  if (want <= n->v.raster_cap) return G4S_OK;
-  const int64_t ids = std::min(n->raster_full, std::max(want, (int64_t)1 << 20));
-  net_free(n, n->v.raster);
-  n->v.raster = nullptr;
-  n->device_bytes -= (size_t)n->v.raster_cap * 4;
-  n->v.raster_cap = 0;
-  const cudaError_t e = net_malloc(n, (void **)&n->v.raster, (size_t)ids * 4);
-  if (e != cudaSuccess) {
-    n->v.raster = nullptr;
-    return cuda_error(e, "raster buffer");
+  if (want <= n->v.raster_cap) return;
+  if (n->v.raster != n->raster_step) {
+    net_free(n, n->v.raster);
+    n->device_bytes -= (size_t)n->v.raster_cap * 4;
   }
-  n->v.raster_cap = ids;
-  n->device_bytes += (size_t)ids * 4;
-  return G4S_OK;
+  n->v.raster = n->raster_step;
+  n->v.raster_cap = n->v.n;
+  for (int64_t ids = std::min(n->raster_full, std::max(want, (int64_t)1 << 20)); ids > n->v.n; ids /= 2) {
+    int *p = nullptr;
+    if (!g_fail_next_alloc.exchange(0) && net_malloc(n, (void **)&p, (size_t)ids * 4) == cudaSuccess) {
+      n->v.raster = p;
+      n->v.raster_cap = ids;
+      n->device_bytes += (size_t)ids * 4;
+      return;
+    }
+    (void)cudaGetLastError();
+  }
 }
+
+// Steps of a chunk at most, where the raster buffer is written (recorded runs, and the schemes
+// whose spike list it is).
+static int64_t raster_steps(const g4s_net *n) { return std::max<int64_t>(1, n->v.raster_cap / n->v.n); }
 
 static int chunk_copy_raster(g4s_net *n, int cs, cudaStream_t s) {
   const int64_t total = chunk_total(n, cs);
   if (n->desc.record_raster && total > 0) {
-    const int rc = need_stage(n, (size_t)total * 4);
+    const int rc = need_stage(n, (size_t)total * 4, false);
     if (rc) return rc;
     n->h_raster = reinterpret_cast<int *>(n->h_stage);
     G4S_CUDA(cudaMemcpyAsync(n->h_raster, n->v.raster, (size_t)total * 4, cudaMemcpyDeviceToHost, s));
@@ -1119,13 +1145,16 @@ static int run_chunk(g4s_net *n, int cs, bool last, bool skl, StepLaunch &launch
 }
 
 namespace g4s {
-int64_t net_chunk_steps(const g4s_net *n) { return n->chunk_legacy; }
+int64_t net_chunk_steps(g4s_net *n, int64_t steps) {
+  steps = std::min(steps, n->chunk_legacy);
+  need_raster(n, steps);
+  return std::min(steps, raster_steps(n));
+}
 
 int net_run_by(g4s_net *n, int steps, bool last, StepLaunch &launch) {
-  int rc = need_raster(n, steps);
   int64_t spikes = 0;
   double ms = 0.0;
-  if (!rc) rc = run_chunk(n, steps, last, true, launch, &spikes, &ms);
+  const int rc = run_chunk(n, steps, last, true, launch, &spikes, &ms);
   if (rc) return rc;
   n->last_ms = n->last_wall_ms = n->last_kernel_ms = ms;
   n->last_launches = 1;
@@ -1149,10 +1178,10 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
   const bool team = alg == kAlgSKL && n->team_ok && n->team_ready;
   // (the team kernel writes a raster only where it is recorded; the other schemes' spike lists
   // are the raster)
+  int64_t longest = team ? n->chunk_steps : n->chunk_legacy;
   if (!team || n->desc.record_raster) {
-    const int64_t longest = team ? n->chunk_steps : n->chunk_legacy;
-    const int rcr = need_raster(n, std::min<int64_t>(steps, longest));
-    if (rcr) return rcr;
+    need_raster(n, std::min<int64_t>(steps, longest));
+    longest = std::min(longest, raster_steps(n));
   }
   const auto w0 = std::chrono::steady_clock::now();
   G4S_CUDA(cudaEventRecord(n->ev0, n->stream));
@@ -1164,7 +1193,7 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
     // while the GPU runs the next one.
     int cs = 0;
     auto start = [&]() -> int {
-      cs = (int)std::min<int64_t>(remaining, n->chunk_steps);
+      cs = (int)std::min<int64_t>(remaining, longest);
       const bool last_chunk = remaining == cs;
       g4s_net *one[1] = {n};
       const int rc = team_round_start(one, &cs, &last_chunk, 1, n->launch, n->stream, n->barrier_ns, stall_of(n));
@@ -1207,7 +1236,7 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
   schemes.alg = alg;
   schemes.launches = &launches;
   while (!team && remaining > 0) {
-    const int cs = (int)std::min<int64_t>(remaining, n->chunk_legacy);
+    const int cs = (int)std::min<int64_t>(remaining, longest);
     int64_t chunk_spikes = 0;
     const int rc = run_chunk(n, cs, remaining == cs, alg == kAlgSKL, schemes, &chunk_spikes, &kernel_ms);
     if (rc) return rc;
@@ -1303,7 +1332,7 @@ static int run_nets(g4s_net *const *nets, const int32_t *steps, int count, doubl
     if (!nets[i]) return set_error(G4S_ERR_INVALID, "null handle in batch");
   std::vector<int> teams;
   if (count > 1) plan_batch(nets, steps, count, teams);
-  std::vector<int64_t> remaining(count);
+  std::vector<int64_t> remaining(count), longest(count);
   for (int i = 0; i < count; ++i) {
     if (steps[i] < 0 || nets[i]->t_abs + steps[i] > (int64_t)INT32_MAX)
       return set_error(G4S_ERR_INVALID, "bad step count in batch");
@@ -1313,7 +1342,11 @@ static int run_nets(g4s_net *const *nets, const int32_t *steps, int count, doubl
     if (rc) return rc;
     if (!nets[i]->team_ok)
       return set_error(G4S_ERR_INVALID, "a network of the batch does not fit the team kernel");
-    if (nets[i]->desc.record_raster && (rc = need_raster(nets[i], std::min<int64_t>(steps[i], nets[i]->chunk_steps)))) return rc;
+    longest[i] = nets[i]->chunk_steps;
+    if (nets[i]->desc.record_raster) {
+      need_raster(nets[i], std::min<int64_t>(steps[i], longest[i]));
+      longest[i] = std::min(longest[i], raster_steps(nets[i]));
+    }
     remaining[i] = steps[i];
     nets[i]->last_spikes = 0;
   }
@@ -1327,7 +1360,7 @@ static int run_nets(g4s_net *const *nets, const int32_t *steps, int count, doubl
   for (;;) {
     bool any = false;
     for (int i = 0; i < count; ++i) {
-      cs[i] = (int)std::min<int64_t>(remaining[i], nets[i]->chunk_steps);
+      cs[i] = (int)std::min<int64_t>(remaining[i], longest[i]);
       last[i] = cs[i] > 0 && cs[i] == remaining[i];
       any = any || cs[i] > 0;
     }
@@ -1873,8 +1906,20 @@ int g4s_net_state(g4s_net *n, float *v, float *u, float *i_last, float *a, float
   const int64_t N = n->v.n;
   const int nb = (int)((N + kStateBlock - 1) / kStateBlock);
   const int64_t blk = std::min<int64_t>(N, kStateBlock);
-  const int rcs = need_stage(n, (size_t)blk * 32 * (nb > 1 ? 2 : 1));
-  if (rcs) return rcs;
+  if (need_stage(n, (size_t)blk * 32 * (nb > 1 ? 2 : 1), true) != G4S_OK) {
+    // (no pinned memory: field by field out of the device's records, slowly)
+    const NetView &w = n->v;
+    const struct {
+      const void *at;
+      size_t pitch;
+    } src[8] = {{w.vu, 8},    {&w.vu->y, 8},    {w.ilast, 4},    {w.abcd, 16}, {&w.abcd->y, 16}, {&w.abcd->z, 16},
+                {&w.abcd->w, 16}, {w.sstat, sizeof(SpikeStat)}};
+    for (int k = 0; k < 8; ++k)
+      if (dst[k])
+        G4S_CUDA(cudaMemcpy2DAsync(dst[k], 4, src[k].at, src[k].pitch, 4, (size_t)N, cudaMemcpyDeviceToHost, n->stream));
+    G4S_CUDA(cudaStreamSynchronize(n->stream));
+    return G4S_OK;
+  }
   float *const h_state = reinterpret_cast<float *>(n->h_stage);
   float *const half[2] = {h_state, h_state + (nb > 1 ? blk * 8 : 0)};
   auto count = [&](int b) { return (int)std::min<int64_t>(kStateBlock, N - (int64_t)b * kStateBlock); };

@@ -350,21 +350,29 @@ extern "C" int g4s_net_fp64_check(g4s_net *net, int32_t steps, double *dv_max, d
   // steps of a chunk: differences of up to kTwinBytes at a time (so that the selection reads
   // them from L2), the handle's own chunk, a few thousand steps
   constexpr int64_t kTwinBytes = (int64_t)64 << 20;
-  const int64_t chunk = std::max<int64_t>(
-      1, std::min({kTwinBytes / (n * 8), net_chunk_steps(net), (int64_t)4096, (int64_t)std::max(steps, 1)}));
-  size_t bytes = 0;
+  int64_t chunk = net_chunk_steps(net, std::max<int64_t>(1, std::min({kTwinBytes / (n * 8), (int64_t)4096, (int64_t)steps})));
+  size_t bytes, o_vu, o_acc, o_list, o_cnt, o_dv, o_out, o_words;
   auto place = [&](size_t b) {
     const size_t at = bytes;
     bytes = (bytes + b + 255) / 256 * 256;
     return at;
   };
-  const size_t o_vu = place((size_t)n * sizeof(double2)), o_acc = place((size_t)n * sizeof(Q128)),
-               o_list = place((size_t)n * sizeof(int)), o_cnt = place((size_t)chunk * sizeof(int)),
-               o_dv = place((size_t)chunk * (size_t)n * sizeof(double)), o_out = place((size_t)chunk * 3 * sizeof(double)),
-               o_words = place(2 * sizeof(int));
   DevBuf buf;
-  cudaError_t e = cudaMalloc((void **)&buf.p, bytes);
-  if (e != cudaSuccess) return cuda_error(e, "g4s_net_fp64_check: allocation");
+  cudaError_t e;
+  for (;; chunk /= 2) {  // (shorter chunks where the device has no room for the differences of these)
+    bytes = 0;
+    o_vu = place((size_t)n * sizeof(double2));
+    o_acc = place((size_t)n * sizeof(Q128));
+    o_list = place((size_t)n * sizeof(int));
+    o_cnt = place((size_t)chunk * sizeof(int));
+    o_dv = place((size_t)chunk * (size_t)n * sizeof(double));
+    o_out = place((size_t)chunk * 3 * sizeof(double));
+    o_words = place(2 * sizeof(int));
+    if ((e = cudaMalloc((void **)&buf.p, bytes)) == cudaSuccess) break;
+    (void)cudaGetLastError();
+    buf.p = nullptr;
+    if (chunk == 1) return cuda_error(e, "g4s_net_fp64_check: allocation");
+  }
   LockstepLaunch run;
   run.w = Twin{reinterpret_cast<double2 *>(buf.p + o_vu), reinterpret_cast<Q128 *>(buf.p + o_acc),
                reinterpret_cast<int *>(buf.p + o_list),   reinterpret_cast<int *>(buf.p + o_cnt),

@@ -151,7 +151,7 @@ size_t team_smem(int64_t rc, int team, int64_t col = 0);
 // A handle's arrays, stream and absolute step, for the library's other translation units
 // (the on-device FP64 check, g4s_fp64check.cu).
 const NetView &net_view(const g4s_net *n);
-// `steps` further steps of the handle (at most net_chunk_steps) by a launch of the caller's:
+// `steps` further steps of the handle (at most net_chunk_steps' last answer) by a launch of the caller's:
 // it does what the library's own step kernels do with the handle's arrays, and the handle's
 // record takes the results.  `stall`: blocks too many for its grid barrier to wait for, so that
 // it runs out.
@@ -160,7 +160,8 @@ struct StepLaunch {
                                  unsigned long long limit_ns, int stall, cudaStream_t s) = 0;
 };
 int net_run_by(g4s_net *n, int steps, bool last, StepLaunch &launch);
-int64_t net_chunk_steps(const g4s_net *n);
+// steps that one such launch may take, of the `steps` asked for (by the raster buffer to be had)
+int64_t net_chunk_steps(g4s_net *n, int64_t steps);
 cudaStream_t net_stream(const g4s_net *n);
 int64_t net_steps_done(const g4s_net *n);
 // CTAs of the team the handle's last planned geometry uses (solo or batched), without

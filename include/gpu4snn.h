@@ -57,7 +57,9 @@ typedef struct g4s_net_desc {
   uint64_t seed;               /* network seed (tables, parameters, drive)                  */
   float drive_scale;           /* thalamic gains (5, 2) x scale; modes 0/1/2 = 0.5/1.0/1.5  */
   int32_t record_raster;       /* 1: keep the spike raster on the host                      */
-  int64_t raster_budget_bytes; /* device raster buffer per chunk (0 = default 1 GiB)        */
+  int64_t raster_budget_bytes; /* device raster buffer per chunk at most (0 = default 1 GiB);
+                                  allocated as runs need it, and chunks are shorter where the
+                                  device has less                                           */
 } g4s_net_desc;
 
 typedef struct g4s_net g4s_net;
