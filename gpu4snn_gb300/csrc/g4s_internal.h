@@ -56,9 +56,18 @@ constexpr int kRecWords = 16;
 
 // Ranks of a team from which every warp polls source ranks of its own; in smaller teams, where
 // that would leave most warps idle, every warp reads every rank's count and takes its share
-// of the step's spikes (from 6 ranks on instead: 64 networks in one launch, teams of up to 7
-// CTAs, 118 ms against 45).
+// of the step's spikes.  Small steps (768 threads, segment runs) gain by it from 12 ranks on,
+// as each warp waits for less (us a step: N=800 x 50 with 12 CTAs 2.88, with 7 and shares 3.57;
+// N=5,000 x 1000 with 11 and shares 5.42, with 12 4.84).  Large steps, and those of the group
+// mapping, are bound by the delivery, for which idle warps count: shares up to the sixteen
+// ranks that fetch_spike's search takes (shares / own sources with 12 and with 16 CTAs of 1024
+// threads: groups N=50,000 x 1000 18.7 / 28.7, 15.7 / 20.3, N=40,000 x 4000 35.6 / 62.5, 28.1 / 40.4;
+// runs N=50,000 x 1000 19.8 / 28.9, 16.3 / 20.2, but N=5,000 x 1000 5.8 / 5.7, 5.6 / 5.1).
 constexpr int kOwnSources = 12;
+constexpr int kOwnSourcesLarge = 17;
+__host__ __device__ constexpr bool own_sources(int team, bool small_steps) {
+  return team >= (small_steps ? kOwnSources : kOwnSourcesLarge);
+}
 
 // Shared-memory layout of one team rank (byte offsets; the optional arrays are present
 // when their flag is set).
@@ -66,14 +75,15 @@ struct TeamLayout {
   unsigned abcd, vu, a, b, own, z, pay, col, bytes;
   bool abcd_sm, vu_sm, prez, pay_sm, col_sm;
 };
-// (col: rows of the rank's column of the segment table, 0 if it stays in global memory)
+// (col: rows of the rank's column of the segment table, 0 if it stays in global memory; own:
+// every warp polls source ranks of its own)
 __host__ __device__ inline unsigned team_align16(size_t x) { return (unsigned)((x + 15) & ~(size_t)15); }
-__host__ __device__ inline TeamLayout team_layout(int64_t rc, int team, int64_t col) {
+__host__ __device__ inline TeamLayout team_layout(int64_t rc, int team, int64_t col, bool own) {
   TeamLayout L{};
   L.abcd_sm = rc <= kAbcdSlice;
   L.vu_sm = rc <= kVuSlice;
   L.prez = rc <= kPrezSlice;
-  L.pay_sm = team >= kOwnSources;
+  L.pay_sm = own;
   size_t o = 0;
   L.abcd = (unsigned)o;
   if (L.abcd_sm) o += (size_t)rc * 16;

@@ -603,7 +603,7 @@ struct Source {
   int lt;       // step of the launch
 };
 
-static_assert(kOwnSources <= 16, "fetch_spike searches sixteen sources");
+static_assert(kOwnSources <= 17 && kOwnSourcesLarge <= 17, "fetch_spike searches sixteen sources");
 // This lane's spike of the batch at position q0 (whole warps call it): its row and the
 // bounds of this rank's segment in it; an empty segment past the end.
 template <int NT, int kMode>
@@ -612,7 +612,7 @@ __device__ __forceinline__ void fetch_spike(const TeamItem &it, TeamShared &sh, 
   const int q = q0 + (threadIdx.x & 31);
   s = b = e = 0;
   if (q0 >= c.total) return;
-  // the source holding position q: the last one that starts at or before it (at most eleven
+  // the source holding position q: the last one that starts at or before it (at most sixteen
   // sources, or eight of the warp's own; its offset and count in one word, as the shuffles
   // share the shared-memory pipe that bounds large steps, busy 72% of one: N=10^6 41.1 -> 40.7 us)
   int k = 0;
@@ -941,7 +941,7 @@ __device__ void team_run(const TeamItem &it, int rank, unsigned char *s_raw, Tea
   const bool solo = kSolo && it.team == 1;  // the whole network in this CTA: no exchange
   const bool lead = rank == 0 && threadIdx.x == 0;
   if (threadIdx.x == 0) {
-    sh.L = team_layout(it.rc, it.team, it.col);
+    sh.L = team_layout(it.rc, it.team, it.col, own_sources(it.team, NT == kTeamNTSmall && kMode == kDeliverRun));
     sh.rank = rank;
     sh.nown[0] = sh.nown[1] = 0;
     sh.work[0] = sh.work[1] = 0;
@@ -1253,7 +1253,7 @@ __global__ void __launch_bounds__(NT, 1) k_team(const TeamItem *__restrict__ ite
 
 size_t team_smem(int64_t rc, int team, int64_t col) {
   if (rc < 1 || team < 1 || team > kMaxTeam) return 0;
-  const size_t bytes = team_layout(rc, team, col).bytes;
+  const size_t bytes = team_layout(rc, team, col, own_sources(team, true)).bytes;  // (the kernel that takes most)
   return bytes > kTeamSmemLimit ? 0 : (bytes < 16 ? 16 : bytes);
 }
 

@@ -43,6 +43,15 @@ def test_source_ranks(g4s, oracle, p, threads):
     assert counts.max() > 31 * 2
 
 
+@pytest.mark.parametrize("threads,delivery", [(768, 1), (1024, 0), (1024, 1)])
+@pytest.mark.parametrize("p", [14, 15, 16, 17, 18, 24])
+def test_shared_sources(g4s, oracle, p, threads, delivery):
+    """Teams around sixteen ranks, up to which the warps of large steps and of the group mapping
+    share all ranks' spikes."""
+    counts = run_both(g4s, oracle, 3001, 203, 56, 2.0, 60, (p, delivery), threads)
+    assert counts.max() > 31 * 2
+
+
 @pytest.mark.parametrize("delivery", [0, 1])
 def test_single_spikes_and_bursts(g4s, oracle, delivery):
     """Steps without any spike, and a burst with more than 64 spikes a rank."""
