@@ -83,3 +83,20 @@ def test_segment_columns(g4s, oracle, n, steps, geometry):
     """Launches on both sides of the number of steps from which the ranks keep their columns of
     the segment table in shared memory, and sizes on both sides of the largest column."""
     run_both(g4s, oracle, n, 120, 55, 1.5, 2 * steps, geometry, 768)
+
+
+@pytest.mark.parametrize("n,p", [(152 * 14896, 152), (152 * 14896 + 1, 0)])
+def test_largest_automatic_slices(g4s, n, p):
+    """The largest network that a team takes by itself, and the first that the global-atomic
+    kernel does (also with a team, if one is asked for): the same results as scheme S."""
+    with g4s.Network(n, 12, seed=57, drive_scale=1.5) as a, g4s.Network(n, 12, seed=57, drive_scale=1.5) as b:
+        assert a.geometry()[0] == p
+        a.run(12, 4)
+        b.run(20, 2)
+        a.set_geometry(152, 0)
+        assert a.geometry()[0] == 152
+        a.run(8, 4)
+        assert np.array_equal(np.stack(a.raster()), np.stack(b.raster()))
+        assert np.array_equal(a.currents(), b.currents())
+        x, y = a.state(), b.state()
+        assert all(np.array_equal(x[k].view(np.uint32), y[k].view(np.uint32)) for k in x)
