@@ -156,7 +156,9 @@ struct g4s_net {
   uint32_t tag_next = 0;  // record tags of the team kernel: never repeated for this handle's lists
   unsigned long long barrier_ns = kBarrierNs;
   size_t device_bytes = 0;
-  // per-step arrays of the last finished chunk
+  // per-step arrays of the last finished chunk, and where a chunk of k_persistent is packed
+  unsigned char *d_pack = nullptr;  // (in the arena)
+  std::vector<unsigned char> c_pack;
   std::vector<int> c_counts;
   std::vector<long long> c_base;
   std::vector<unsigned long long> c_stamps;
@@ -364,7 +366,7 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
                o_base = place((size_t)cs * sizeof(long long)),
                o_stamps = place(((size_t)cs * 2 + 2) * sizeof(unsigned long long)), o_status = place(sizeof(int)),
                o_gs = place(sizeof(GridSync) * (1 + 2 * (size_t)kMaxTeam * kRecLines)), o_stats = place(2 * sizeof(double)),
-               o_raster = place(pool ? 0 : N * sizeof(int));
+               o_raster = place(pool ? 0 : N * sizeof(int)), o_pack = place(round_pack_bytes((int)cs));
   unsigned char *mem = nullptr;
   if ((rc = dalloc(n, &mem, bytes, "neuron state and per-step arrays"))) {
     free_net(n);
@@ -383,6 +385,7 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
   v.status = reinterpret_cast<int *>(mem + o_status);
   n->gs = reinterpret_cast<GridSync *>(mem + o_gs);
   n->d_stats = reinterpret_cast<double *>(mem + o_stats);
+  n->d_pack = mem + o_pack;
   if (!pool) n->raster_step = v.raster = reinterpret_cast<int *>(mem + o_raster);
   if ((rc = dalloc(n, const_cast<int **>(&v.idx), N * S, "targets")) ||
       (rc = dalloc(n, const_cast<float **>(&v.w), N * S, "weights")) ||
@@ -789,20 +792,14 @@ static int finish_tables(g4s_net *n, bool may_be_sorted) {
   return check_status(n, "row sort");
 }
 
-// Results of one chunk of `cs` steps: per-step counts, raster offsets and stamps, and the
-// raster itself when recorded; each step's ids sorted (the device order is by CTA).
-// The three steps of absorbing a chunk, so that a batch can enqueue every network's
-// copies on one stream and synchronise once: per-step metadata, then the raster of the
-// networks that record it, then the host-side bookkeeping.
-static int chunk_copy_meta(g4s_net *n, int cs, cudaStream_t s) {
-  NetView &v = n->v;
-  n->c_counts.resize((size_t)cs);
-  n->c_base.resize((size_t)cs);
-  n->c_stamps.resize((size_t)cs * 2);
-  G4S_CUDA(cudaMemcpyAsync(n->c_counts.data(), v.counts, (size_t)cs * 4, cudaMemcpyDeviceToHost, s));
-  G4S_CUDA(cudaMemcpyAsync(n->c_base.data(), v.base, (size_t)cs * 8, cudaMemcpyDeviceToHost, s));
-  G4S_CUDA(cudaMemcpyAsync(n->c_stamps.data(), v.stamps, (size_t)cs * 16, cudaMemcpyDeviceToHost, s));
-  return G4S_OK;
+// A chunk's per-step arrays out of its pack (round_pack_bytes), status words first.
+static void chunk_unpack(g4s_net *n, const unsigned char *p, size_t cs) {
+  const int *counts = reinterpret_cast<const int *>(p + 8);
+  const long long *base = reinterpret_cast<const long long *>(p + 8 + ((cs * 4 + 7) & ~(size_t)7));
+  const unsigned long long *stamps = reinterpret_cast<const unsigned long long *>(base + cs);
+  n->c_counts.assign(counts, counts + cs);
+  n->c_base.assign(base, base + cs);
+  n->c_stamps.assign(stamps, stamps + 2 * cs);
 }
 
 static int64_t chunk_total(const g4s_net *n, int cs) { return (int64_t)n->c_base[cs - 1] + n->c_counts[cs - 1]; }
@@ -934,17 +931,6 @@ static int chunk_finish(g4s_net *n, int cs, int64_t *spikes) {
   const int rc = chunk_finish_from(n, cs, n->t_abs, spikes);
   n->t_abs += cs;
   return rc;
-}
-
-// Results of one chunk of `cs` steps of one network: per-step counts, raster offsets and
-// stamps, and the raster itself when recorded, each step's ids in order.
-static int absorb_chunk(g4s_net *n, int cs, int64_t *spikes) {
-  int rc = chunk_copy_meta(n, cs, n->stream);
-  if (rc) return rc;
-  G4S_CUDA(cudaStreamSynchronize(n->stream));
-  if ((rc = chunk_copy_raster(n, cs, n->stream))) return rc;
-  G4S_CUDA(cudaStreamSynchronize(n->stream));
-  return chunk_finish(n, cs, spikes);
 }
 
 // The recorded raster's first m spikes: the step of each (t) and its id.  Large rasters on
@@ -1105,16 +1091,8 @@ static int team_round_finish(TeamLaunch &L, cudaStream_t s, double *kernel_ms, i
   *kernel_ms += ms;
   *launches += 1;
   for (int i : L.order) {
-    // each network's share of the pack: status words, counts, raster offsets, stamps
-    g4s_net *n = L.nets[(size_t)i];
-    const size_t st = (size_t)L.steps[(size_t)i];
-    const unsigned char *p = L.h_mem + L.o_pack + L.at[(size_t)i];
-    const int *status = reinterpret_cast<const int *>(p), *counts = status + 2;
-    const long long *base = reinterpret_cast<const long long *>(p + 8 + ((st * 4 + 7) & ~(size_t)7));
-    const unsigned long long *stamps = reinterpret_cast<const unsigned long long *>(base + st);
-    n->c_counts.assign(counts, counts + st);
-    n->c_base.assign(base, base + st);
-    n->c_stamps.assign(stamps, stamps + 2 * st);
+    // (each network's share of the pack)
+    chunk_unpack(L.nets[(size_t)i], L.h_mem + L.o_pack + L.at[(size_t)i], (size_t)L.steps[(size_t)i]);
   }
   for (int i : L.order) {
     const int *status = reinterpret_cast<const int *>(L.h_mem + L.o_pack + L.at[(size_t)i]);
@@ -1143,12 +1121,24 @@ static int run_chunk(g4s_net *n, int cs, bool last, bool skl, StepLaunch &launch
   G4S_CUDA(launch(v, n->t_abs, cs, last, n->gs, skl ? n->barrier_ns : kBarrierNs, skl ? stall_of(n) : 0, n->stream));
   if (skl) n->barrier_stall = 0;
   G4S_CUDA(cudaEventRecord(n->ek1, n->stream));
-  int rc = check_status(n, "persistent step kernel");
+  // (packed on the device and brought back by one copy: as five pageable ones, and two waits, a
+  // run of one step of N=2,500 took 75 us, 43 so)
+  G4S_CUDA(launch_chunk_gather(v, n->gs, cs, n->d_pack, n->stream));
+  n->c_pack.resize(round_pack_bytes(cs));
+  G4S_CUDA(cudaMemcpyAsync(n->c_pack.data(), n->d_pack, n->c_pack.size(), cudaMemcpyDeviceToHost, n->stream));
+  G4S_CUDA(cudaStreamSynchronize(n->stream));
+  const int *status = reinterpret_cast<const int *>(n->c_pack.data());
+  int rc = status_rc(status[0], status[1], "persistent step kernel");
   if (rc) return rc;
   float kms = 0.0f;
   G4S_CUDA(cudaEventElapsedTime(&kms, n->ek0, n->ek1));
   *kernel_ms += kms;
-  return absorb_chunk(n, cs, spikes);
+  chunk_unpack(n, n->c_pack.data(), (size_t)cs);
+  if (n->desc.record_raster && chunk_total(n, cs) > 0) {
+    if ((rc = chunk_copy_raster(n, cs, n->stream))) return rc;
+    G4S_CUDA(cudaStreamSynchronize(n->stream));
+  }
+  return chunk_finish(n, cs, spikes);
 }
 
 namespace g4s {

@@ -1439,23 +1439,29 @@ __global__ void k_round_clear(const TeamItem *items) {
   for (int64_t i = threadIdx.x; i < words; i += blockDim.x) g[i] = 0ull;
 }
 
-__global__ void k_round_gather(const TeamItem *items, const int64_t *off, unsigned char *pack) {
-  const TeamItem &it = items[blockIdx.x];
-  const int s = it.steps;
-  if (s <= 0) return;
-  unsigned char *p = pack + off[blockIdx.x];
+__device__ __forceinline__ void gather_steps(const NetView &v, const GridSync *gs, int s, unsigned char *p) {
   if (threadIdx.x == 0) {
-    reinterpret_cast<int *>(p)[0] = *it.v.status;
-    reinterpret_cast<int *>(p)[1] = it.sync->error;
+    reinterpret_cast<int *>(p)[0] = *v.status;
+    reinterpret_cast<int *>(p)[1] = gs->error;
   }
   int *c = reinterpret_cast<int *>(p + 8);
   long long *b = reinterpret_cast<long long *>(p + 8 + (((size_t)s * 4 + 7) & ~(size_t)7));
   unsigned long long *t = reinterpret_cast<unsigned long long *>(b + s);
   for (int i = threadIdx.x; i < s; i += blockDim.x) {
-    c[i] = it.v.counts[i];
-    b[i] = it.v.base[i];
+    c[i] = v.counts[i];
+    b[i] = v.base[i];
   }
-  for (int i = threadIdx.x; i < 2 * s; i += blockDim.x) t[i] = it.v.stamps[i];
+  for (int i = threadIdx.x; i < 2 * s; i += blockDim.x) t[i] = v.stamps[i];
+}
+
+__global__ void k_round_gather(const TeamItem *items, const int64_t *off, unsigned char *pack) {
+  const TeamItem &it = items[blockIdx.x];
+  if (it.steps > 0) gather_steps(it.v, it.sync, it.steps, pack + off[blockIdx.x]);
+}
+
+// The same for one network's chunk by another kernel.
+__global__ void k_chunk_gather(NetView v, const GridSync *gs, int steps, unsigned char *pack) {
+  gather_steps(v, gs, steps, pack);
 }
 
 cudaError_t launch_round_clear(const TeamItem *items, int count, cudaStream_t s) {
@@ -1466,6 +1472,11 @@ cudaError_t launch_round_clear(const TeamItem *items, int count, cudaStream_t s)
 cudaError_t launch_round_gather(const TeamItem *items, const int64_t *off, int count, unsigned char *pack,
                                 cudaStream_t s) {
   k_round_gather<<<(unsigned)count, 512, 0, s>>>(items, off, pack);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_chunk_gather(const NetView &v, const GridSync *gs, int steps, unsigned char *pack, cudaStream_t s) {
+  k_chunk_gather<<<1, 512, 0, s>>>(v, gs, steps, pack);
   return cudaGetLastError();
 }
 
