@@ -156,8 +156,7 @@ struct g4s_net {
   uint32_t tag_next = 0;  // record tags of the team kernel: never repeated for this handle's lists
   unsigned long long barrier_ns = kBarrierNs;
   size_t device_bytes = 0;
-  // per-step arrays of the last finished chunk, and where a chunk of k_persistent is packed
-  unsigned char *d_pack = nullptr;  // (in the arena)
+  // per-step arrays of the last finished chunk, and the packs they came in from k_persistent
   std::vector<unsigned char> c_pack;
   std::vector<int> c_counts;
   std::vector<long long> c_base;
@@ -366,7 +365,7 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
                o_base = place((size_t)cs * sizeof(long long)),
                o_stamps = place(((size_t)cs * 2 + 2) * sizeof(unsigned long long)), o_status = place(sizeof(int)),
                o_gs = place(sizeof(GridSync) * (1 + 2 * (size_t)kMaxTeam * kRecLines)), o_stats = place(2 * sizeof(double)),
-               o_raster = place(pool ? 0 : N * sizeof(int)), o_pack = place(round_pack_bytes((int)cs));
+               o_raster = place(pool ? 0 : N * sizeof(int));
   unsigned char *mem = nullptr;
   if ((rc = dalloc(n, &mem, bytes, "neuron state and per-step arrays"))) {
     free_net(n);
@@ -385,7 +384,6 @@ static int alloc_net(const g4s_net_desc *d, g4s_net **out, cudaMemPool_t pool = 
   v.status = reinterpret_cast<int *>(mem + o_status);
   n->gs = reinterpret_cast<GridSync *>(mem + o_gs);
   n->d_stats = reinterpret_cast<double *>(mem + o_stats);
-  n->d_pack = mem + o_pack;
   if (!pool) n->raster_step = v.raster = reinterpret_cast<int *>(mem + o_raster);
   if ((rc = dalloc(n, const_cast<int **>(&v.idx), N * S, "targets")) ||
       (rc = dalloc(n, const_cast<float **>(&v.w), N * S, "weights")) ||
@@ -792,14 +790,18 @@ static int finish_tables(g4s_net *n, bool may_be_sorted) {
   return check_status(n, "row sort");
 }
 
-// A chunk's per-step arrays out of its pack (round_pack_bytes), status words first.
-static void chunk_unpack(g4s_net *n, const unsigned char *p, size_t cs) {
+// The per-step arrays of `cs` steps out of their pack (round_pack_bytes, status words first), as
+// the steps from `at` of the chunk.
+static void chunk_unpack(g4s_net *n, const unsigned char *p, size_t cs, size_t at = 0) {
   const int *counts = reinterpret_cast<const int *>(p + 8);
   const long long *base = reinterpret_cast<const long long *>(p + 8 + ((cs * 4 + 7) & ~(size_t)7));
   const unsigned long long *stamps = reinterpret_cast<const unsigned long long *>(base + cs);
-  n->c_counts.assign(counts, counts + cs);
-  n->c_base.assign(base, base + cs);
-  n->c_stamps.assign(stamps, stamps + 2 * cs);
+  n->c_counts.resize(at);
+  n->c_base.resize(at);
+  n->c_stamps.resize(2 * at);
+  n->c_counts.insert(n->c_counts.end(), counts, counts + cs);
+  n->c_base.insert(n->c_base.end(), base, base + cs);
+  n->c_stamps.insert(n->c_stamps.end(), stamps, stamps + 2 * cs);
 }
 
 static int64_t chunk_total(const g4s_net *n, int cs) { return (int64_t)n->c_base[cs - 1] + n->c_counts[cs - 1]; }
@@ -1108,6 +1110,9 @@ static int team_round(g4s_net *const *nets, const int *steps, const bool *last, 
   return rc ? rc : team_round_finish(L, s, kernel_ms, launches);
 }
 
+// Steps that one pack holds in the memory of the spike records.
+constexpr int kPackSteps = (int)((sizeof(GridSync) * 2 * kMaxTeam * kRecLines - 16) / 28);
+
 // Why the waits of a handle's next SKL launch run out (0: they need not).
 static int stall_of(const g4s_net *n) { return n->barrier_stall ? kStallFault : n->barrier_ns == 0 ? kStallLimit : 0; }
 
@@ -1121,19 +1126,29 @@ static int run_chunk(g4s_net *n, int cs, bool last, bool skl, StepLaunch &launch
   G4S_CUDA(launch(v, n->t_abs, cs, last, n->gs, skl ? n->barrier_ns : kBarrierNs, skl ? stall_of(n) : 0, n->stream));
   if (skl) n->barrier_stall = 0;
   G4S_CUDA(cudaEventRecord(n->ek1, n->stream));
-  // (packed on the device and brought back by one copy: as five pageable ones, and two waits, a
-  // run of one step of N=2,500 took 75 us, 43 so)
-  G4S_CUDA(launch_chunk_gather(v, n->gs, cs, n->d_pack, n->stream));
-  n->c_pack.resize(round_pack_bytes(cs));
-  G4S_CUDA(cudaMemcpyAsync(n->c_pack.data(), n->d_pack, n->c_pack.size(), cudaMemcpyDeviceToHost, n->stream));
+  // (packed on the device, where the team kernel has its records, and brought back by one copy for
+  // some 3,200 steps: as five pageable ones, and two waits, a run of one step of N=2,500 took 75
+  // us, 43 so)
+  unsigned char *d_pack = reinterpret_cast<unsigned char *>(n->gs + 1);
+  n->c_pack.resize((size_t)((cs - 1) / kPackSteps + 1) * round_pack_bytes(kPackSteps));
+  auto piece = [&](int s0) { return n->c_pack.data() + (size_t)(s0 / kPackSteps) * round_pack_bytes(kPackSteps); };
+  for (int s0 = 0; s0 < cs; s0 += kPackSteps) {
+    const int k = std::min(kPackSteps, cs - s0);
+    NetView part = v;
+    part.counts += s0;
+    part.base += s0;
+    part.stamps += 2 * s0;
+    G4S_CUDA(launch_chunk_gather(part, n->gs, k, d_pack, n->stream));
+    G4S_CUDA(cudaMemcpyAsync(piece(s0), d_pack, round_pack_bytes(k), cudaMemcpyDeviceToHost, n->stream));
+  }
   G4S_CUDA(cudaStreamSynchronize(n->stream));
-  const int *status = reinterpret_cast<const int *>(n->c_pack.data());
+  const int *status = reinterpret_cast<const int *>(piece(0));
   int rc = status_rc(status[0], status[1], "persistent step kernel");
   if (rc) return rc;
   float kms = 0.0f;
   G4S_CUDA(cudaEventElapsedTime(&kms, n->ek0, n->ek1));
   *kernel_ms += kms;
-  chunk_unpack(n, n->c_pack.data(), (size_t)cs);
+  for (int s0 = 0; s0 < cs; s0 += kPackSteps) chunk_unpack(n, piece(s0), (size_t)std::min(kPackSteps, cs - s0), (size_t)s0);
   if (n->desc.record_raster && chunk_total(n, cs) > 0) {
     if ((rc = chunk_copy_raster(n, cs, n->stream))) return rc;
     G4S_CUDA(cudaStreamSynchronize(n->stream));
