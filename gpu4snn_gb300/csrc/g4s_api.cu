@@ -1269,15 +1269,15 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
   return G4S_OK;
 }
 
-// Estimated device time in us of one step of a network on a team of p CTAs: a chain of round
-// trips, the update and drive of a CTA's neurons, and its share of the step's synapses (by the
-// length of its segments).  Fitted to networks of 1,100 to 10^6 neurons, most within 10%
-// (measured / model: one CTA, 4,189 neurons and 108,000 synapses a step 32 / 33, 1,120 and
-// 24,000 8.9 / 9.1; 8 CTAs, 43,005 and 1.05 million 40 / 39; 152 CTAs, 10^6 and 7.4 million
-// 41 / 41).
+// Estimated device time in us of one step of a network on a team of p CTAs of 1024 threads: a chain
+// of round trips, the update and drive of a CTA's neurons, and its share of the step's synapses.
+// One CTA walks rows in pieces of 128 synapses.  A larger team's share depends on the length of
+// its segments; where a step has few spikes the time is that of walking the longest one, eight
+// lanes a spike.
 static double team_step_us(const g4s_net *n, double syn, int p) {
   const double neurons = (double)n->v.n / p, seg = std::max(1.0, (double)n->v.nsyn / p);
-  return p == 1 ? 2.0 + 1.3e-3 * neurons + 0.235e-3 * syn : 3.6 + 1.6e-3 * neurons + (0.19e-3 + 2.2e-3 / seg) * syn / p;
+  if (p == 1) return 2.0 + 1.35e-3 * neurons + 0.185e-3 * syn * (double)((n->v.nsyn + 127) / 128 * 128) / n->v.nsyn;
+  return std::max(3.6 + 1.6e-3 * neurons + (0.19e-3 + 2.2e-3 / seg) * syn / p, 2.8 + 1.6e-3 * neurons + 5.8e-3 * seg);
 }
 
 // CTAs of each network of a batch.  At one CTA per kBatchSlice neurons the networks take about
