@@ -1236,11 +1236,12 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
   }
   struct Schemes : StepLaunch {  // (the time limit and injected faults are the SKL scheme's)
     int alg;
+    double synapses;
     int64_t *launches;
     cudaError_t operator()(const NetView &v, int64_t t_abs0, int cs, bool last, GridSync *gs, unsigned long long limit_ns,
                            int stall, cudaStream_t s) override {
       int made = 0;
-      const cudaError_t e = launch_steps(v, t_abs0, cs, last, gs, limit_ns, alg, stall, s, &made);
+      const cudaError_t e = launch_steps(v, t_abs0, cs, last, gs, limit_ns, alg, synapses, stall, s, &made);
       *launches += made;
       return e;
     }
@@ -1250,6 +1251,7 @@ static int run_net(g4s_net *n, int32_t steps, int32_t alg_in) {
   while (!team && remaining > 0) {
     const int cs = (int)std::min<int64_t>(remaining, longest);
     int64_t chunk_spikes = 0;
+    schemes.synapses = (double)v.n * recent_rate(n) * 1e-3 * (double)v.nsyn;
     const int rc = run_chunk(n, cs, remaining == cs, alg == kAlgSKL, schemes, &chunk_spikes, &kernel_ms);
     if (rc) return rc;
     spikes += chunk_spikes;

@@ -24,9 +24,9 @@ constexpr int kAlgAuto = 5;
 cudaError_t launch_init(const NetView &v, cudaStream_t s);
 cudaError_t launch_conngen(const NetView &v, int self_loops, cudaStream_t s);
 // nsteps steps of a scheme (kAlgSKL: the fallback of the team kernel) with the currents in
-// global memory; *launches: kernel launches made
+// global memory; synapses: those expected of a step; *launches: kernel launches made
 cudaError_t launch_steps(const NetView &v, int64_t t_abs0, int nsteps, bool last_chunk, GridSync *gs,
-                         unsigned long long limit_ns, int alg, int stall, cudaStream_t s, int *launches);
+                         unsigned long long limit_ns, int alg, double synapses, int stall, cudaStream_t s, int *launches);
 cudaError_t launch_stats(const NetView &v, double *out, cudaStream_t s);
 // fields of neurons [i0, i0 + cnt) as separate arrays: bits 0..7 of `fields` are v, u, I, a, b,
 // c, d and the spike count; `out` is device-accessible, cnt values per field asked for

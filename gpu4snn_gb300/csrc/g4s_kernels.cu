@@ -5,7 +5,7 @@
 //   k_persistent   the steps of a chunk of the N, S, AP and AB schemes (and of SKL where the team
 //                  kernel does not fit): update (stateupdate, gpu4snn.cu:334-417) and delivery in
 //                  one cooperative launch with timed grid barriers (k_update and k_deliver, two
-//                  launches a step, for S on large networks):
+//                  launches a step, for S where steps have many synapses):
 //                    N  a warp per spiking neuron              (deliverspks1, gpu4snn.cu:420-443)
 //                    S  flat over the step's synapses          (deliverspks2, gpu4snn.cu:446-467)
 //                    AP thread group per spiking row           (propagatespikes, gpu4snn.cu:323-331)
@@ -455,12 +455,16 @@ static cudaError_t persistent_nt(const NetView &v, int64_t t_abs0, int nsteps, b
 }
 
 cudaError_t launch_steps(const NetView &v, int64_t t_abs0, int nsteps, bool last_chunk, GridSync *gs,
-                         unsigned long long limit_ns, int alg, int stall, cudaStream_t s, int *launches) {
+                         unsigned long long limit_ns, int alg, double synapses, int stall, cudaStream_t s, int *launches) {
   const int group = deliver_group(alg);
   *launches = 1;
-  // S on large networks with long rows: two launches a step, the delivery's grid oversubscribed
-  // (N=250,000 x 10,000 238 us a step against 266 persistent; N=10^6 x 1000 83 against 80)
-  if (!(alg == kAlgS && v.n >= 200000 && v.nsyn >= 4096))
+  // S where steps are expected to have many synapses: two launches a step, the delivery's grid
+  // oversubscribed, which costs 10 to 20 us a step and then delivers 7 to 12% faster (us a step
+  // persistent / two, with the synapses: N=100,000 x 1000 15.2 / 24.2 at 1.7 million, 250,000 x 10,000
+  // 33.0 / 42.9 at 4.3, 100,000 x 10,000 100 / 97 at 15.8, 300,000 x 1000 127 / 131 at 21, 100,000 x
+  // 10,000 179 / 166 at 29, 10^6 x 3000 288 / 265 at 48, 250,000 x 10,000 435 / 388 at 73)
+  constexpr double kTwoLaunches = 16e6;
+  if (!(alg == kAlgS && synapses >= kTwoLaunches))
     return v.n <= (int64_t)sm_count() * kPerSmall
                ? persistent_nt<kPerSmall>(v, t_abs0, nsteps, last_chunk, gs, limit_ns, group, stall, s)
                : persistent_nt<kPerLarge>(v, t_abs0, nsteps, last_chunk, gs, limit_ns, group, stall, s);

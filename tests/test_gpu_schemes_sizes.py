@@ -41,3 +41,21 @@ def test_row_lengths(g4s, oracle, nsyn):
             net.run(30, alg)
             assert np.array_equal(net.counts(), sim.counts())
             assert np.array_equal(net.currents(), sim.acc())
+
+
+@pytest.mark.parametrize("nsyn,two", [(7000, False), (7600, True)])
+def test_steps_with_many_synapses(g4s, nsyn, two):
+    """Scheme S at sizes on both sides of 16 million expected synapses a step (22 Hz at drive 3
+    before there is a measured rate), from which it takes two launches a step: the results of
+    the SKL scheme."""
+    n = 100_000
+    with g4s.Network(n, nsyn, seed=83, drive_scale=3.0) as net:
+        net.run(24, 4)
+        want, cur, raster = net.state(), net.currents(), np.stack(net.raster())
+        net.reset()
+        net.run(10, 2)
+        assert net.info().last_run_launches == (20 if two else 1)
+        net.run(14, 2)
+        assert np.array_equal(np.stack(net.raster()), raster) and np.array_equal(net.currents(), cur)
+        got = net.state()
+        assert all(np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32)) for k in want)
