@@ -677,6 +677,7 @@ static int prepare_team(g4s_net *n, int batch_p = 0) {
   int p = 0;
   int64_t rc = 0;
   const bool batch = batch_p > 0;
+  n->team_ready = false;  // (until everything below is in place)
   n->team_batch = batch_p;
   if (!plan_team(n, n->want_p, batch_p, &p, &rc)) {
     n->team_ok = false;
@@ -702,8 +703,12 @@ static int prepare_team(g4s_net *n, int batch_p = 0) {
       n->seg = nullptr;
       n->device_bytes -= n->seg_bytes;
       n->seg_bytes = 0;
-      cudaError_t e = net_malloc(n, (void **)&n->seg, bytes);
-      if (e != cudaSuccess) return cuda_error(e, "segment table");
+      cudaError_t e = g_fail_next_alloc.exchange(0) ? cudaErrorMemoryAllocation : net_malloc(n, (void **)&n->seg, bytes);
+      if (e != cudaSuccess) {
+        n->seg = nullptr;
+        (void)cudaGetLastError();
+        return cuda_error(e, "segment table");
+      }
       n->seg_bytes = bytes;
       n->device_bytes += bytes;
     }

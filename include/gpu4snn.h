@@ -181,9 +181,10 @@ int g4s_net_destroy(g4s_net *net);
  *   G4S_FAULT_BARRIER_STALL  the next SKL launch of `net` waits at its first barrier for
  *                            one block more than it has, so the wait runs out after the
  *                            barrier time limit and the run returns G4S_ERR_TIMEOUT;
- *   G4S_FAULT_ALLOC          the next device allocation of g4s_net_create fails, or of the
- *                            row-order check of g4s_net_load_tables, or of the optional
- *                            packed rows (process-wide; `net` may be NULL). */
+ *   G4S_FAULT_ALLOC          the next device allocation of g4s_net_create fails, or the next of
+ *                            these, whichever comes first: the row-order check's of
+ *                            g4s_net_load_tables, the packed rows, the segment table, the
+ *                            raster buffer, pinned staging (process-wide; `net` may be NULL). */
 #define G4S_FAULT_BARRIER_STALL 1
 #define G4S_FAULT_ALLOC 2
 int g4s_inject_fault(g4s_net *net, int32_t kind);

@@ -93,3 +93,23 @@ def test_state_without_staging(g4s):
         net.inject_fault(_lib.FAULT_ALLOC)
         a = state(net)
         assert same(a, state(net))
+
+
+def test_segment_table_of_another_team(g4s):
+    """No room for the segment table of a larger team, in a batch and then alone: the call reports
+    it, and the next one plans anew instead of running the former team without a table."""
+    from gpu4snn_gb300 import _lib
+    from gpu4snn_gb300.network import run_batch
+    with g4s.Network(3001, 100, seed=74, drive_scale=1.5) as a, g4s.Network(3001, 100, seed=74, drive_scale=1.5) as b, \
+            g4s.Network(64, 8, seed=75) as c:
+        a.set_geometry(2, -1)
+        a.run(30, 4)
+        a.set_geometry(0, -1)
+        for call in (lambda: run_batch([a, c], 10), lambda: a.run(10, 4)):
+            a.inject_fault(_lib.FAULT_ALLOC)
+            with pytest.raises(g4s.G4SError) as e:
+                call()
+            assert e.value.code == _lib.ERR_NOMEM
+            call()
+        b.run(50, 4)
+        assert same(a.raster(), b.raster()) and same(state(a), state(b))
