@@ -589,9 +589,8 @@ static int resolve_alg(g4s_net *n, int alg) {
 // polls source ranks of its own (N=800 x 50 with 7 CTAs 3.57, 12 2.88), and as many as it takes,
 // where that is possible, for segments short enough to be walked as runs (N=2,500 x 2000 with
 // 77 CTAs 3.92, 88 3.72; 11,000 x 2000 5.15, 4.48).
-// Slices of more than kTeamSlice neurons (beyond N=2,264,192 on 152 SMs), which leave no room to
-// draw the next step's drive ahead, take the global-atomic kernel: never more than 5% slower, and
-// far faster where a rank reads many spikes for few synapses (team / global-atomic, N=2,340,000: x
+// Slices of more than kTeamSlice neurons (beyond N=2,264,192 on 152 SMs; the largest that fit hold
+// 15,445) take the global-atomic kernel: never more than 5% slower, and far faster where a rank reads many spikes for few synapses (team / global-atomic, N=2,340,000: x
 // 10 at drive 1 35.0 / 33.8, at drive 2 67.3 / 35.6, at drive 8 695 / 61; x 400 39.9 / 37.7, 35.8 / 35.3,
 // 973 / 470; the worst x 400 at drive 1.5 30.4 / 32.0).
 constexpr int64_t kTeamSlice = 14896;
@@ -629,11 +628,6 @@ static bool plan_team(g4s_net *n, int want, int batch_p, int *p_out, int64_t *rc
     if (team_smem(rc, (int)p) == 0) return false;
   }
   if (want <= 0 && batch_p <= 0 && rc > kTeamSlice) return false;
-  int pfit = 0;
-  if (team_max_blocks(team_smem(rc, (int)p), &pfit) != cudaSuccess || pfit < p) {
-    (void)cudaGetLastError();
-    return false;
-  }
   *p_out = (int)p;
   *rc_out = rc;
   return true;
@@ -722,10 +716,6 @@ static int prepare_team(g4s_net *n, int batch_p = 0) {
   return G4S_OK;
 }
 
-// Tables are kept with every row sorted by target (the pairs stay together); the
-// segment table of the team kernel is rebuilt on the next SKL run.  The exactness bound
-// of the split shared-memory accumulation is measured here: fewer than 65536 synapses
-// into any neuron and sum(|q| >> 16) + 1 over them below 2^31 - 2^20.
 // Largest in-degree (h[0]) of the tables and, with with_mag, the largest sum(|q| >> 16) + 1
 // over a neuron's inputs (h[1]), else the largest (|q| >> 16) + 1 of any synapse (h[2]); on
 // the network's stream (stream-ordered scratch).
@@ -745,6 +735,10 @@ static int bound_pass(g4s_net *n, bool with_mag, unsigned long long h[3]) {
   return e == cudaSuccess ? G4S_OK : cuda_error(e, "table bound pass");
 }
 
+// Tables are kept with every row sorted by target (the pairs stay together); the
+// segment table of the team kernel is rebuilt on the next SKL run.  The exactness bound
+// of the split shared-memory accumulation is measured here: fewer than 65536 synapses
+// into any neuron and sum(|q| >> 16) + 1 over them below 2^31 - 2^20.
 static int finish_tables(g4s_net *n, bool may_be_sorted) {
   // (rows that arrive sorted, as tables read back from a network do, skip the sort)
   // Scratch is stream-ordered (cudaMallocAsync / cudaFreeAsync on the network's stream):

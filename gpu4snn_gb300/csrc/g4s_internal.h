@@ -128,7 +128,8 @@ cudaError_t launch_inbound(const NetView &v, unsigned *cnt, unsigned long long *
 // team_max_blocks also raises the kernel's shared-memory ceiling: call it once before the
 // first launch_team (which may then be captured in a CUDA graph)
 // Threads per CTA of the team kernel: 1024 (the default; the most reads in flight) or 768
-// (80 registers a thread instead of 64: no spills, faster when a step's work is small).
+// (80 registers a thread instead of 64: no spills, or 48 bytes in launches with one-CTA teams;
+// faster when a step's work is small).
 constexpr int kTeamNT = 1024;
 constexpr int kTeamNTSmall = 768;
 // pair: the tables are read from v.pair (packed words) instead of v.idx and v.w;

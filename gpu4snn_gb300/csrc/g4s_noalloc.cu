@@ -39,7 +39,7 @@ constexpr int64_t kNoAllocMaxSlice = 16384;
 
 // Layout of the scratch array.
 constexpr size_t kOffSync = 0;                                       // GridSync (128 B): error word
-constexpr size_t kOffRec = 128;                                      // spike records: [2][team][4 x 16] u64
+constexpr size_t kOffRec = 128;                                      // spike records: [2][team][2 x 16] u64
 constexpr size_t kOffCtl = kOffRec + 2 * kNoAllocMaxTeam * kRecLines * 128;  // int[5]: -, queue head, status, -, next tag
 constexpr size_t kOffSlots = kOffCtl + 128;                          // int2[kNoAllocMaxTeam]
 constexpr size_t kOffItem = kOffSlots + 256;                         // TeamItem
@@ -135,15 +135,17 @@ __global__ void __launch_bounds__(kSetupNT) k_noalloc_setup(TeamItem item, int *
 
 }  // namespace
 
-// The scratch of g4s_run_noalloc (about 6.5 MB per GPU, held until exit).
+// The scratch of g4s_run_noalloc (about 4.5 MB per GPU, held until exit).
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 // In host code g_noalloc_scratch names a host-side stand-in, not device memory: its
-// device address is looked up once per device, with that device current, and cached.
+// device address is looked up once per device, with that device current, and cached, and
+// with it the device's SMs.
 static std::mutex g_scratch_mu;
 static void *g_scratch_dev[256];
+static int g_scratch_sms[256];
 
-static int scratch_address(unsigned char **out) {
+static int scratch_address(unsigned char **out, int *sms) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_error(e, "cudaGetDevice");
@@ -155,8 +157,11 @@ static int scratch_address(unsigned char **out) {
     if (e != cudaSuccess || !p) return cuda_error(e, "cudaGetSymbolAddress of the no-alloc scratch");
     // once per device, outside any stream capture of the caller's launches
     if ((e = team_smem_ceiling()) != cudaSuccess) return cuda_error(e, "team kernel shared-memory ceiling");
+    e = cudaDeviceGetAttribute(&g_scratch_sms[dev], cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return cuda_error(e, "cudaDeviceGetAttribute");
     g_scratch_dev[dev] = p;
   }
+  *sms = g_scratch_sms[dev];
   *out = static_cast<unsigned char *>(g_scratch_dev[dev]);
   return G4S_OK;
 }
@@ -188,7 +193,8 @@ extern "C" int g4s_run_noalloc(const g4s_dev_net *d, int64_t t_abs0, int32_t ste
   if (steps == 0) return G4S_OK;
 
   unsigned char *scr = nullptr;
-  int rc0 = scratch_address(&scr);
+  int sms = 1;
+  int rc0 = scratch_address(&scr, &sms);
   if (rc0) return rc0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   GridSync *sync = reinterpret_cast<GridSync *>(scr + kOffSync);
@@ -230,7 +236,7 @@ extern "C" int g4s_run_noalloc(const g4s_dev_net *d, int64_t t_abs0, int32_t ste
   h.rc = (int)rc;
   h.sync = sync;
   const int64_t rows = team > 1 ? (d->n + kSetupNT / 32 - 1) / (kSetupNT / 32) : 1;
-  k_noalloc_setup<<<(unsigned)std::min<int64_t>(rows, 152 * 16), kSetupNT, 0, s>>>(h, ctl, slots, item, seg,
+  k_noalloc_setup<<<(unsigned)std::min<int64_t>(rows, 16 * sms), kSetupNT, 0, s>>>(h, ctl, slots, item, seg,
                                                                                     2 * kNoAllocMaxNeurons);
   cudaError_t e = cudaGetLastError();
   // (768 threads for slices whose state lives in shared memory, as for small steps elsewhere)

@@ -147,8 +147,8 @@ int g4s_net_set_barrier_timeout(g4s_net *net, uint64_t ns);
  * mapping in use (0 or 1; -1 without a multi-CTA team).  Results do not depend on either. */
 int g4s_net_set_geometry(g4s_net *net, int32_t owner_blocks, int32_t delivery);
 /* Threads per CTA of the SKL team kernel: 1024 (the most table reads in flight, for steps
- * with many synapses per CTA), 768 (80 registers a thread instead of 64, no spills: faster
- * for steps whose work is small) or 0 (the default: 768 when a CTA's expected share of a
+ * with many synapses per CTA), 768 (80 registers a thread instead of 64: faster for steps
+ * whose work is small) or 0 (the default: 768 when a CTA's expected share of a
  * step, from the recent firing rate, is under 32768 synapses, else 1024; 1024 in a batch).
  * Results do not depend on it; the autotuner tries both sizes.  A batch of networks that
  * disagree uses 1024, a no-alloc run 768 for slices of at most 2048 neurons, else 1024.
