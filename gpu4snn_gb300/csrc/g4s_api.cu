@@ -590,9 +590,10 @@ static int resolve_alg(g4s_net *n, int alg) {
 // where that is possible, for segments short enough to be walked as runs (N=2,500 x 2000 with
 // 77 CTAs 3.92, 88 3.72; 11,000 x 2000 5.15, 4.48).
 // Slices of more than kTeamSlice neurons (beyond N=2,264,192 on 152 SMs; the largest that fit hold
-// 15,445) take the global-atomic kernel: never more than 5% slower, and far faster where a rank reads many spikes for few synapses (team / global-atomic, N=2,340,000: x
-// 10 at drive 1 35.0 / 33.8, at drive 2 67.3 / 35.6, at drive 8 695 / 61; x 400 39.9 / 37.7, 35.8 / 35.3,
-// 973 / 470; the worst x 400 at drive 1.5 30.4 / 32.0).
+// 15,445) take the global-atomic kernel: never more than 5% slower, and far faster where a rank
+// reads many spikes for few synapses (team / global-atomic, N=2,340,000: x 10 at drive 1 35.0 /
+// 33.8, at drive 2 67.3 / 35.6, at drive 8 695 / 61; x 400 39.9 / 37.7, 35.8 / 35.3, 973 / 470; the
+// worst x 400 at drive 1.5 30.4 / 32.0).
 constexpr int64_t kTeamSlice = 14896;
 constexpr int64_t kLoneNeurons = 640, kLoneSlice = 52;
 static int64_t lone_team(int64_t n, int64_t nsyn, int64_t pmax) {
