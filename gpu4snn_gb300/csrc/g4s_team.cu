@@ -28,7 +28,8 @@
 //             with a step number that never repeats for the network's buffers, so a
 //             reader that sees the tag it expects needs no fence to trust the payload:
 //             two 128-byte record lines (count and 31 ids), further ids in a per-rank
-//             overflow list.  In teams of kOwnSources CTAs and more every warp polls the
+//             overflow list.  In teams of kOwnSources CTAs and more (kOwnSourcesLarge where
+//             steps are large) every warp polls the
 //             records of a few source ranks of its own (line 0, and line 1 of the ranks that
 //             had more than kLine1After spikes in the previous step, with a time limit) and
 //             goes on to deliver those ranks' spikes at once: no warp waits for another
@@ -51,8 +52,8 @@
 //   What bounds a step: with few spikes the chain update -> publish -> poll -> bounds ->
 //   rows, of whose 6,500 cycles (N=2,500) the four trips to L2 are half, the other half the
 //   straight code between them, which all warps issue; with many, the LSU's shared-memory
-//   pipe (ncu: 72% busy at N=250,000, drive 2, by the additions and the row reads; issue 55%,
-//   DRAM 24%).  us per step of this kernel and of the one before it (block-wide scan and
+//   pipe, by the additions and the row reads (ncu: busy 66% of N=10^6 x 1000, 75% at drive 2, 77%
+//   and 82% of N=250,000 x 10,000; issue 56, 53, 43 and 42%).  us per step of this kernel and of the one before it (block-wide scan and
 //   staging of the step's ids, a search per synapse, a conversion per synapse; all mappings in
 //   one kernel): N=2,500 x 1000 3.30 / 4.55, 33,333 x 777 at drive 1.5 5.19 / 7.10, 100,000 x
 //   1000 7.28 / 8.77, 10^6 x 1000 40.1 / 43.4 (drive 0.5 13.0 / 17.6, drive 2 106 / 112),
@@ -614,7 +615,7 @@ __device__ __forceinline__ void fetch_spike(const TeamItem &it, TeamShared &sh, 
   if (q0 >= c.total) return;
   // the source holding position q: the last one that starts at or before it (at most sixteen
   // sources, or eight of the warp's own; its offset and count in one word, as the shuffles
-  // share the shared-memory pipe that bounds large steps, busy 72% of one: N=10^6 41.1 -> 40.7 us)
+  // share the shared-memory pipe that bounds large steps: N=10^6 41.1 -> 40.7 us)
   int k = 0;
 #pragma unroll
   for (int step = 8; step; step >>= 1)
