@@ -39,3 +39,18 @@ def test_recorded_and_streamed_stretches(g4s, oracle, tmp_path, alg, budget):
             assert (a[cap:] == -9).all() and (b[cap:] == -9).all()
         r = formats.read_raster(str(tmp_path / "r.bin"))
         assert r.t0 == 30 and np.array_equal(r.ids, oi[~keep]) and np.array_equal(r.counts, sim.counts()[30:50])
+
+
+@pytest.mark.parametrize("alg", [3, 4])
+@pytest.mark.parametrize("n", [2000, 300_000, 2_500_000, 4_300_000])
+def test_large_steps_in_order(g4s, n, alg):
+    """Steps with a burst of a third of the neurons, whose ids the host sorts (by two or three
+    digits of 11 bits): ascending, each as often as the neuron's own count of its spikes."""
+    with g4s.Network(n, 4, seed=58, drive_scale=3.0) as net:
+        net.run(30, alg)
+        t, i = net.raster()
+        c = net.counts()
+        assert c.max() > n // 8
+        assert np.array_equal(np.bincount(t, minlength=30), c)
+        assert (np.diff(i.astype(np.int64) + t.astype(np.int64) * n) > 0).all()
+        assert np.array_equal(np.bincount(i, minlength=n), net.state()["nospks"])
